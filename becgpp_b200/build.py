@@ -33,35 +33,11 @@ MAX_N_WITH_KERNEL = 384
 # two-size kernels for batches that mix grids (sweeps over 128^2 and 256^2)
 COMBOS = ((128, 0, 256, 0),)
 
-# stream-pass candidates of the autotuner: radix orders of the line FFT and lines
-# per tile (a strided tile groups that many neighbours, so N must be a multiple;
-# the tile must fit in shared memory)
-RADIX_ORDERS = (0, 1, 2)   # Stockham stage orders; 3 = the register-resident transform (N = 32 R)
-CONV_LINES = (1, 2, 4, 8, 16)
-
-
-def radix_orders(n):
-    """Transforms of the stream H psi passes: 0-2 Stockham orders, 3 the register
-    transform (N = 32 R); each again at doubled occupancy (+4: half the registers)."""
-    base = RADIX_ORDERS + ((3,) if n % 32 == 0 else ())
-    return base + tuple(v + 4 for v in base)
-
-
-def stream_lines(n):
-    def smem(L, ln):
-        pitch = ((L + L // 8 + 1) | 1) if ln >= 8 else (((L + L // 8 + 1 + 5) // 8) * 8 + 2)
-        return ln * pitch * 16
-    return [ln for ln in (1, 2, 4, 8, 16) if n % ln == 0 and ln <= n and smem(n, ln) <= 160 * 1024]
-
-
-def conv_lines(m):
-    """Lines per tile of the stream convolution passes over the padded length m:
-    the line buffers and the tile's kernel slab must fit in shared memory."""
-    def smem(L, ln):
-        pitch = ((L + L // 8 + 1) | 1) if ln >= 8 else (((L + L // 8 + 1 + 5) // 8) * 8 + 2)
-        slab = ((ln * ((L // 2 + 1) | 1) * 8 + 15) // 16) * 16
-        return ln * pitch * 16 + slab
-    return [ln for ln in CONV_LINES if smem(m, ln) <= 200 * 1024]
+# stream-pass candidates of the autotuner: lines per tile and factorization variants
+# of the line transform (csrc/bgp_lfft.cuh)
+STREAM_LINES = (2, 4, 8)
+PAD_LINES = (4, 8)        # the padded, strided passes
+VARIANTS = (0, 1)
 
 
 NVCC = os.environ.get("NVCC", "nvcc")
@@ -88,7 +64,8 @@ def _write_if_changed(path, text):
 def generate():
     os.makedirs(GEN, exist_ok=True)
     units = []
-    hdr = ["// generated by becgpp_b200/build.py: compiled grid sizes", "#pragma once"]
+    hdr = ["// generated by becgpp_b200/build.py: compiled grid sizes", "#pragma once",
+           "namespace bgp { struct SKernel; }"]
     hdr.append("#define BGP_FOR_SIZES(X) " + " ".join(f"X({n}, {m})" for n, m in pairs()))
     hdr.append("#define BGP_FOR_COMBOS(X) " + " ".join(f"X({a}, {b}, {c}, {d})" for a, b, c, d in COMBOS))
     hdr.append("#define BGP_FOR_TABLE_LENGTHS(X) "
@@ -119,37 +96,48 @@ def generate():
                 path = os.path.join(GEN, f"k2_{name}.cu")
                 _write_if_changed(path, src)
                 units.append(path)
-    # stream passes (standalone and batched H psi): one unit per line length N with
-    # every (lines per tile, radix order) candidate of the autotuner, and the
-    # convolution passes of the padded length M = 2N
+    # stream passes (standalone and batched H psi): per line length N the axis passes,
+    # and per padded length M = 2N the convolution's, in every (lines per tile,
+    # factorization) candidate of the autotuner, for one instance and for a batch
+    def stream_unit(path, include, groups):
+        lines = [f'#include "{include}"']
+        for fn, kern, length, widths, kinds in groups:
+            cases = []
+            for ln in widths:
+                for v in VARIANTS:
+                    for k in kinds:
+                        for nb in ("1", "bgp::kStreamBatch"):
+                            if k is None and nb != "1":
+                                continue
+                            inst = f"bgp::{kern}<{length}, {ln}, {v}, {k}, {nb}>"
+                            if k is None:          # the energy sums: all axes, one instance
+                                inst = f"bgp::{kern}<{length}, {ln}, {v}>"
+                            lines.append(f"template __global__ void {inst}(const __grid_constant__ bgp::SLaunchT<{nb}>);")
+                            cases.append(f"  if (c == {ln} && v == {v} && k == {k or 0} && batch == {int(nb != '1')}) {{\n"
+                                         f"    constexpr int th = bgp::s_threads({length}, {ln}, {v});\n"
+                                         f"    constexpr size_t sm = bgp::s_smem({length}, {ln}, {v});\n"
+                                         f"    static const bgp::SKernel e{{(void*)&{inst}, th, sm}};\n"
+                                         f"    return &e;\n  }}")
+            lines.append(f'extern "C" const bgp::SKernel* {fn}(int c, int v, int k, int batch) {{')
+            lines += cases
+            lines.append("  return nullptr;\n}")
+            hdr.append(f'extern "C" const bgp::SKernel* {fn}(int c, int v, int k, int batch);')
+        _write_if_changed(path, "\n".join(lines) + "\n")
+        units.append(path)
+
+        hdr.append("#define BGP_FOR_LINE_LENGTHS(X) "
+               + " ".join(f"X({n})" for n in sorted({n for n, _ in pairs()} | {m for _, m in pairs() if m})))
     hdr.append("#define BGP_FOR_STREAM_N(X) " + " ".join(f"X({n})" for n in SIZES_N))
     hdr.append("#define BGP_FOR_STREAM_M(X) " + " ".join(f"X({2 * n})" for n in SIZES_N if n <= MAX_N_WITH_KERNEL))
     for n in SIZES_N:
-        lns = stream_lines(n)
-        hdr.append(f'extern "C" void* bgp_sptr_{n}(int ln, int v);')
-        lines = ['#include "bgp_stream.cuh"']
-        cases = []
-        for ln in lns:
-            for v in radix_orders(n):
-                lines.append(f"template __global__ void bgp::k_stream_h<{n}, {ln}, {v}>(bgp::SLaunch, int, int);")
-                cases.append(f"  if (ln == {ln} && v == {v}) return (void*)&bgp::k_stream_h<{n}, {ln}, {v}>;")
-        lines.append(f'extern "C" void* bgp_sptr_{n}(int ln, int v) {{')
-        lines += cases
-        lines.append("  return nullptr;\n}")
+        stream_unit(os.path.join(GEN, f"s_{n}.cu"), "bgp_stream.cuh",
+                    [(f"bgp_sptr_{n}", "k_stream_h", n, STREAM_LINES, (0, 1, 2)),
+                     (f"bgp_septr_{n}", "k_stream_energy", n, PAD_LINES, (None,))])
         if n <= MAX_N_WITH_KERNEL:
             m = 2 * n
-            hdr.append(f'extern "C" void* bgp_scptr_{m}(int ln, int v);')
-            ccases = []
-            for ln in conv_lines(m):
-                for v in (0, 3) if m % 32 == 0 else (0,):
-                    lines.append(f"template __global__ void bgp::k_stream_conv<{m}, {ln}, {v}>(bgp::SLaunch, int);")
-                    ccases.append(f"  if (ln == {ln} && v == {v}) return (void*)&bgp::k_stream_conv<{m}, {ln}, {v}>;")
-            lines.append(f'extern "C" void* bgp_scptr_{m}(int ln, int v) {{')
-            lines += ccases
-            lines.append("  return nullptr;\n}")
-        path = os.path.join(GEN, f"s_{n}.cu")
-        _write_if_changed(path, "\n".join(lines) + "\n")
-        units.append(path)
+            stream_unit(os.path.join(GEN, f"s_conv_{m}.cu"), "bgp_stream.cuh",
+                        [(f"bgp_srptr_{m}", "k_stream_real", n, STREAM_LINES, (0, 1)),
+                         (f"bgp_spptr_{m}", "k_stream_pad", m, PAD_LINES, (0, 1, 2))])
     _write_if_changed(os.path.join(GEN, "bgp_sizes_gen.h"), "\n".join(hdr) + "\n")
     return units
 
@@ -165,7 +153,8 @@ def _deps(src):
     if os.path.basename(src).startswith(("k_", "k2_")):
         return [os.path.join(CSRC, f) for f in KERNEL_HEADERS]
     if os.path.basename(src).startswith("s_"):
-        return [os.path.join(CSRC, f) for f in KERNEL_HEADERS + ("bgp_stream.cuh", "bgp_regfft.cuh")]
+        return [os.path.join(CSRC, f) for f in ("bgp_stream.cuh", "bgp_lfft.cuh", "bgp_device.cuh", "bgp_fft.cuh",
+                                                "bgp_common.cuh")]
     return [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".cu", ".h"))] + [
         os.path.join(os.path.dirname(HERE), "include", "bgp.h"), os.path.abspath(__file__)]
 

@@ -121,6 +121,7 @@ struct DevCtx {
   size_t max_smem_optin = 0;
   std::map<int, double2*> tw;   // twiddle tables by length
   std::map<int, float2*> tw32;  // the same rounded to FP32
+  std::map<int, double2*> lf[kLVariants];   // line-transform tables of the stream passes
 };
 std::mutex g_mu;
 std::map<int, DevCtx> g_dev;
@@ -170,6 +171,32 @@ int twiddles(DevCtx* d, int L, const double2** out) {
   d->tw32[L] = fp;
   *out = dp;
   return BGP_OK;
+}
+
+// stage twiddles of the stream passes' line transform of length L, variant V
+template <int L, int V>
+int lf_table(DevCtx* d) {
+  if (d->lf[V].count(L)) return BGP_OK;
+  constexpr int len = lf_tab_len(L, V);
+  std::vector<double2> w(L), tab(len);
+  const double2* dw = nullptr;
+  int rc = twiddles(d, L, &dw);
+  if (rc) return rc;
+  CK(cudaMemcpy(w.data(), dw, sizeof(double2) * L, cudaMemcpyDeviceToHost));
+  lf_fill_table<L, V>(w.data(), tab.data());
+  double2* dp = nullptr;
+  CK(cudaMalloc(&dp, sizeof(double2) * len));
+  CK(cudaMemcpy(dp, tab.data(), sizeof(double2) * len, cudaMemcpyHostToDevice));
+  d->lf[V][L] = dp;
+  return BGP_OK;
+}
+int lf_tables(DevCtx* d, int L) {
+  switch (L) {
+#define X(l) case l: { int rc = lf_table<l, 0>(d); return rc ? rc : lf_table<l, 1>(d); }
+    BGP_FOR_LINE_LENGTHS(X)
+#undef X
+    default: return fail(BGP_ERR_UNSUPPORTED, "line length not compiled in");
+  }
 }
 
 int twiddles32(DevCtx* d, int L, const float2** out) {
@@ -529,6 +556,8 @@ int bgp_plan_create(const bgp_instance_desc* desc, int n_inst, bgp_plan** plan) 
     if ((rc = twiddles32(dev, I.N, &I.twN32))) return bail(rc);
     if (I.M && (rc = twiddles(dev, I.M, &I.twM))) return bail(rc);
     if (I.M && (rc = twiddles32(dev, I.M, &I.twM32))) return bail(rc);
+    if ((rc = lf_tables(dev, I.N))) return bail(rc);
+    if (I.M && (rc = lf_tables(dev, I.M))) return bail(rc);
     if ((rc = palloc_t(p, (size_t)kNB * n, &I.pool))) return bail(rc);
     // potentials: current and trial; 3D with a kernel also the potentials of the
     // density's linear and quadratic parts in the step (the line search's quartic)
@@ -544,9 +573,12 @@ int bgp_plan_create(const bgp_instance_desc* desc, int n_inst, bgp_plan** plan) 
     if ((rc = palloc_t(p, (size_t)1, &I.bar))) return bail(rc);
     if ((rc = palloc(p, sizeof(Ctl), &I.save))) return bail(rc);
     if (I.M) {
-      const size_t c1 = I.ndim == 2 ? (size_t)I.N * I.Mh : (size_t)I.N * I.N * I.Mh;
+      // rows of conv_pitch(N) >= Mh columns (the stream passes' pitch; the persistent
+      // programs pack theirs Mh apart)
+      const size_t pitch = (size_t)conv_pitch(I.N);
+      const size_t c1 = I.ndim == 2 ? I.N * pitch : (size_t)I.N * I.N * pitch;
       if ((rc = palloc_t(p, c1, &I.cb1))) return bail(rc);
-      if (I.ndim == 3 && (rc = palloc_t(p, (size_t)I.N * I.M * I.Mh, &I.cb2))) return bail(rc);
+      if (I.ndim == 3 && (rc = palloc_t(p, (size_t)I.N * I.M * pitch, &I.cb2))) return bail(rc);
       double* Kq = nullptr;
       if ((rc = build_table(p, d, I, 0, &Kq))) return bail(rc);
       I.Kq = Kq;
@@ -797,27 +829,53 @@ int bgp_precondition(bgp_plan* p, int i, const void* grad, const void* psi, cons
   return BGP_OK;
 }
 
+}  // extern "C"
+
 namespace {
 // ------------------------------------------------------------ stream passes
-void* stream_h_kernel(int N, int ln, int v) {
+// compiled passes by tile width C, factorization V, kind and parameter block (one
+// instance or a batch); null where not compiled
+const SKernel* stream_h_kernel(int N, int C, int V, int stage, bool batch) {
   switch (N) {
-#define X(n) case n: return bgp_sptr_##n(ln, v);
+#define X(n) case n: return bgp_sptr_##n(C, V, stage, batch);
     BGP_FOR_STREAM_N(X)
 #undef X
     default: return nullptr;
   }
 }
-void* stream_conv_kernel(int M, int ln, int v) {
+const SKernel* stream_real_kernel(int N, int C, int V, int inv, bool batch) {
+  switch (2 * N) {
+#define X(m) case m: return bgp_srptr_##m(C, V, inv, batch);
+    BGP_FOR_STREAM_M(X)
+#undef X
+    default: return nullptr;
+  }
+}
+const SKernel* stream_pad_kernel(int M, int C, int V, int mode, bool batch) {
   switch (M) {
-#define X(m) case m: return bgp_scptr_##m(ln, v);
+#define X(m) case m: return bgp_spptr_##m(C, V, mode, batch);
     BGP_FOR_STREAM_M(X)
 #undef X
     default: return nullptr;
   }
 }
 
+// A pass schedule in compiled terms: tile widths and factorization variants.
+struct Sched {
+  int c, v;          // H psi passes
+  int cr, cs, cv;    // convolution: real (contiguous) and padded (strided) passes, variant
+};
+// The public codes name 1 to 16 lines and radix orders 0 to 7 (0 and 3 for the
+// convolution); tiles of 2, 4 and 8 lines in two factorizations are compiled, and a
+// code runs as the nearest of them.
+Sched sched_of(const bgp_plan::StreamSched& sc) {
+  auto w = [](int ln, int lo) { return ln < lo ? lo : (ln > 8 ? 8 : ln); };
+  return Sched{w(sc.ln, 2), sc.v & 1, w(sc.cln, 2), w(sc.csln, 4), sc.cv ? 1 : 0};
+}
+
 // per-instance total of the tiles' partial sums, in tile order: mu = sum dV
-__global__ void k_stream_mu(SLaunch SL, int tiles, double* mu, int offset) {
+template <int NB>
+__global__ void k_stream_mu(const __grid_constant__ SLaunchT<NB> SL, int tiles, double* mu, int offset) {
   const int a = blockIdx.x;
   if (a >= SL.ninst) return;
   const SInst& I = SL.insts[a];
@@ -835,29 +893,60 @@ __global__ void k_stream_mu(SLaunch SL, int tiles, double* mu, int offset) {
   }
 }
 
-int stream_launch(void* kern, int tiles, int threads, size_t smem, SLaunch& SL, cudaStream_t st, void** args) {
+// One pass; chained: it may start while the launch before it on the stream still runs
+// (the pass itself waits, griddepcontrol, before it reads what that one writes).
+template <int NB>
+int stream_launch(const SKernel* kern, int tiles, SLaunchT<NB>& SL, cudaStream_t st, bool chained) {
+  if (!kern) return fail(BGP_ERR_UNSUPPORTED, "stream pass not compiled for this size / schedule");
   SL.tiles = tiles;
-  CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  CK(cudaLaunchKernel(kern, dim3(tiles * SL.ninst), dim3(threads), args, smem, st));
+  if (kern->smem > 48 * 1024)
+    CK(cudaFuncSetAttribute(kern->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kern->smem));
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(tiles * SL.ninst);
+  cfg.blockDim = dim3(kern->threads);
+  cfg.dynamicSmemBytes = kern->smem;
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = chained ? 1 : 0;
+  void* args[] = {&SL};
+  CK(cudaLaunchKernelExC(&cfg, kern->fn, args));
   return BGP_OK;
+}
+
+// The convolution passes of a group: phi from |psi|^2. The first is a plain launch
+// (it reads psi and writes the scratch, so it waits for all earlier work).
+template <int NB>
+int stream_conv(SLaunchT<NB>& SL, const Sched& S, cudaStream_t st) {
+  const SInst& I0 = SL.insts[0];
+  const int N = I0.N, ndim = I0.ndim, M = I0.M, tpl = (N + 1 + S.cs - 1) / S.cs;
+  const int lines = ndim == 2 ? N : N * N;
+  int rc = stream_launch(stream_real_kernel(N, S.cr, S.cv, 0, NB > 1), lines / S.cr, SL, st, false);
+  if (!rc && ndim == 3)
+    rc = stream_launch(stream_pad_kernel(M, S.cs, S.cv, 0, NB > 1), N * tpl, SL, st, true);
+  if (!rc)
+    rc = stream_launch(stream_pad_kernel(M, S.cs, S.cv, 1, NB > 1), (ndim == 2 ? 1 : M) * tpl, SL, st, true);
+  if (!rc && ndim == 3)
+    rc = stream_launch(stream_pad_kernel(M, S.cs, S.cv, 2, NB > 1), N * tpl, SL, st, true);
+  if (!rc) rc = stream_launch(stream_real_kernel(N, S.cr, S.cv, 1, NB > 1), lines / S.cr, SL, st, true);
+  return rc;
 }
 
 // The passes of one group (same N, ndim, kernel): optional convolution (phi from
 // |psi|^2), then the H psi axis passes, then mu.
-int stream_run(SLaunch& SL, int ln, int v, int cln, int csln, int cv, bool conv, double* mu_dev, int mu_off,
-               cudaStream_t st, cudaStream_t side = nullptr, cudaEvent_t ev_fork = nullptr,
-               cudaEvent_t ev_join = nullptr) {
+template <int NB>
+int stream_run(SLaunchT<NB>& SL, const Sched& S, bool conv, double* mu_dev, int mu_off, cudaStream_t st,
+               cudaStream_t side = nullptr, cudaEvent_t ev_fork = nullptr, cudaEvent_t ev_join = nullptr) {
   const SInst& I0 = SL.insts[0];
   const int N = I0.N, ndim = I0.ndim, n = I0.n;
-  void* k = stream_h_kernel(N, ln, v);
-  if (!k) return fail(BGP_ERR_UNSUPPORTED, "stream H psi pass not compiled for this size / schedule");
-  const size_t smem = s_smem(N, ln);
-  const int tiles = n / (N * ln);
-  auto hstage = [&](int st_, cudaStream_t q) -> int {
-    int ax = ndim - 1 - st_;
-    int stage = (st_ == 0) ? 0 : (ax == 0 ? 2 : 1);
-    void* args[] = {&SL, &ax, &stage};
-    return stream_launch(k, tiles, ln * 32, smem, SL, q, args);
+  const int tiles = n / (N * S.c);
+  // the first axis pass is a plain launch, the later ones are chained to it; the last
+  // one is plain where another stream's work comes in between
+  auto hstage = [&](int st_, cudaStream_t q, bool chained) -> int {
+    const int stage = (st_ == 0) ? 0 : (st_ == ndim - 1 ? 2 : 1);
+    return stream_launch(stream_h_kernel(N, S.c, S.v, stage, NB > 1), tiles, SL, q, chained);
   };
   // with the potential computed and a side stream given, the H psi passes before the
   // last (which reads phi) run on the side stream beside the convolution: they write
@@ -867,62 +956,42 @@ int stream_run(SLaunch& SL, int ln, int v, int cln, int csln, int cv, bool conv,
     CK(cudaEventRecord(ev_fork, st));
     CK(cudaStreamWaitEvent(side, ev_fork, 0));
     for (int st_ = 0; st_ < ndim - 1; ++st_) {
-      int rc = hstage(st_, side);
+      int rc = hstage(st_, side, st_ > 0);
       if (rc) return rc;
     }
     CK(cudaEventRecord(ev_join, side));
   }
   if (conv) {
-    const int M = I0.M, Mh = I0.Mh;
-    // contiguous passes (ops 0, 5) in tiles of cln lines, strided passes in tiles
-    // of csln lines (wider rows of the strided loads and stores)
-    void* kc = stream_conv_kernel(M, cln, cv);
-    void* ks = stream_conv_kernel(M, csln, cv);
-    if (!kc || !ks) return fail(BGP_ERR_UNSUPPORTED, "stream convolution not compiled for this size");
-    const int lines = ndim == 2 ? N : N * N, tpl = (Mh + csln - 1) / csln;
-    const int ops2[3] = {0, 1, 5}, ops3[5] = {0, 2, 3, 4, 5};
-    const int* ops = ndim == 2 ? ops2 : ops3;
-    const int nops = ndim == 2 ? 3 : 5;
-    for (int q = 0; q < nops; ++q) {
-      int op = ops[q];
-      const bool contig = (op == 0 || op == 5);
-      const int lw = contig ? cln : csln;
-      int ctiles;
-      if (contig) ctiles = (lines + cln - 1) / cln;
-      else if (op == 1) ctiles = tpl;
-      else if (op == 3) ctiles = M * tpl;
-      else ctiles = N * tpl;
-      void* args[] = {&SL, &op};
-      int rc = stream_launch(contig ? kc : ks, ctiles, lw * 32, s_conv_smem(M, lw), SL, st, args);
-      if (rc) return rc;
-    }
+    int rc = stream_conv(SL, S, st);
+    if (rc) return rc;
   }
   if (overlap) CK(cudaStreamWaitEvent(st, ev_join, 0));
   for (int st_ = overlap ? ndim - 1 : 0; st_ < ndim; ++st_) {
-    int rc = hstage(st_, st);
+    int rc = hstage(st_, st, !overlap && st_ > 0);
     if (rc) return rc;
   }
   if (mu_dev) {
-    k_stream_mu<<<SL.ninst, 256, 0, st>>>(SL, tiles, mu_dev, mu_off);
+    k_stream_mu<NB><<<SL.ninst, 256, 0, st>>>(SL, tiles, mu_dev, mu_off);
   }
   CK(cudaGetLastError());
   return BGP_OK;
 }
 
-// Time every compiled (lines, radix order) candidate of line length N on this
-// group, then the convolution's lines per tile; keep the fastest (median of 3).
-int stream_autotune(bgp_plan* p, bgp_plan::StreamSched& sc, SLaunch& SL, bool conv, cudaStream_t st) {
+// Time every compiled (lines, factorization) candidate of line length N on this
+// group, then the convolution's; keep the fastest (median of 3).
+template <int NB>
+int stream_autotune(bgp_plan::StreamSched& sc, SLaunchT<NB>& SL, bool conv, cudaStream_t st) {
   const int N = SL.insts[0].N;
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
-  auto timed = [&](int ln, int v, int cln, int csln, int cv, bool with_conv, float* ms) -> int {
+  auto timed = [&](const bgp_plan::StreamSched& s, bool with_conv, float* ms) -> int {
     float t[3];
-    int rc = stream_run(SL, ln, v, cln, csln, cv, with_conv, nullptr, 0, st);   // warm-up
+    int rc = stream_run(SL, sched_of(s), with_conv, nullptr, 0, st);   // warm-up
     if (rc) return rc;
     for (int r = 0; r < 3; ++r) {
       CK(cudaEventRecord(e0, st));
-      if ((rc = stream_run(SL, ln, v, cln, csln, cv, with_conv, nullptr, 0, st))) return rc;
+      if ((rc = stream_run(SL, sched_of(s), with_conv, nullptr, 0, st))) return rc;
       CK(cudaEventRecord(e1, st));
       CK(cudaEventSynchronize(e1));
       CK(cudaEventElapsedTime(&t[r], e0, e1));
@@ -931,27 +1000,29 @@ int stream_autotune(bgp_plan* p, bgp_plan::StreamSched& sc, SLaunch& SL, bool co
     *ms = t[1];
     return BGP_OK;
   };
+  int rc = BGP_OK;
   float best = 1e30f;
   sc.cand.clear();
-  for (int ln : {1, 2, 4, 8, 16}) {
-    for (int v = 0; v < 8; ++v) {
-      if (!stream_h_kernel(N, ln, v)) continue;
+  bgp_plan::StreamSched s = sc;
+  for (int ln : {2, 4, 8}) {
+    for (int v = 0; v < kLVariants && !rc; ++v) {
       float ms = 0.f;
-      int rc = timed(ln, v, 8, 8, 0, false, &ms);
-      if (rc) { cudaEventDestroy(e0); cudaEventDestroy(e1); return rc; }
+      s.ln = ln; s.v = v;
+      if ((rc = timed(s, false, &ms))) break;
       sc.cand.push_back({(float)ln, (float)v, 0.f, ms});
       if (ms < best) { best = ms; sc.ln = ln; sc.v = v; }
     }
   }
-  if (conv) {
+  if (conv && !rc) {
     float bc = 1e30f;
-    for (int cln : {1, 2, 4, 8}) {
-      for (int csln : {1, 2, 4, 8, 16}) {
+    s.ln = sc.ln; s.v = sc.v;
+    for (int cln : {2, 4, 8}) {
+      for (int csln : {4, 8}) {
         for (int cv : {0, 3}) {
-          if (!stream_conv_kernel(SL.insts[0].M, cln, cv) || !stream_conv_kernel(SL.insts[0].M, csln, cv)) continue;
           float ms = 0.f;
-          int rc = timed(sc.ln, sc.v, cln, csln, cv, true, &ms);
-          if (rc) { cudaEventDestroy(e0); cudaEventDestroy(e1); return rc; }
+          s.cln = cln; s.csln = csln; s.cv = cv;
+          if (cv == 3 && (2 * N) % 32 != 0) continue;
+          if (rc || (rc = timed(s, true, &ms))) break;
           // negative lines: a convolution candidate
           sc.cand.push_back({(float)(-cln), (float)cv, (float)csln, ms});
           if (ms < bc) { bc = ms; sc.cln = cln; sc.csln = csln; sc.cv = cv; }
@@ -961,11 +1032,29 @@ int stream_autotune(bgp_plan* p, bgp_plan::StreamSched& sc, SLaunch& SL, bool co
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  sc.tuned = 1;
-  (void)p;
-  return BGP_OK;
+  if (!rc) sc.tuned = 1;
+  return rc;
+}
+
+// stream descriptor of an instance (the caller sets psi, H and phi)
+void stream_inst(const bgp_plan* p, const Inst& I, SInst& S) {
+  S.ndim = I.ndim; S.N = I.N; S.n = I.n; S.M = I.M; S.Mh = I.Mh; S.i0 = I.i0;
+  S.dx = I.dx; S.kfac = I.kfac; S.s = I.s; S.tc = I.tc; S.beta2 = I.beta2; S.beta3 = I.beta3;
+  S.Omega = I.Omega; S.dv = I.dv;
+  S.A = I.pool;                 // pool field 0 of the instance as the accumulator
+  S.part = I.part;
+  S.cb1 = I.cb1; S.cb2 = I.cb2; S.Kq = I.Kq; S.conv_scale = I.conv_scale;
+  S.phi_out = I.phi2;           // computed potential: the instance's first potential field
+  S.hscale = 1.0;
+  S.twM = I.twM;
+  for (int V = 0; V < kLVariants; ++V) {
+    S.tabN[V] = p->dev->lf[V][I.N];
+    S.tabM[V] = I.M ? p->dev->lf[V][I.M] : nullptr;
+  }
 }
 }  // namespace
+
+extern "C" {
 
 // H psi of several instances of a plan, enqueued without host synchronisation
 int bgp_apply_H_batch(bgp_plan* p, int n, const int* idx, const void* const* psi, void* const* hpsi,
@@ -1008,31 +1097,6 @@ int bgp_apply_H_batch(bgp_plan* p, int n, const int* idx, const void* const* psi
         done[b] = 1;
       }
     }
-    SLaunch SL;
-    memset(&SL, 0, sizeof(SL));
-    SL.ninst = (int)grp.size();
-    for (int g = 0; g < SL.ninst; ++g) {
-      const int b = grp[g];
-      const Inst& I = p->inst[idx[b]];
-      SInst& S = SL.insts[g];
-      S.ndim = I.ndim; S.N = I.N; S.n = I.n; S.M = I.M; S.Mh = I.Mh; S.i0 = I.i0;
-      S.dx = I.dx; S.kfac = I.kfac; S.s = I.s; S.tc = I.tc; S.beta2 = I.beta2; S.beta3 = I.beta3;
-      S.Omega = I.Omega; S.dv = I.dv;
-      S.psi = (const double2*)psi[b];
-      S.H = (double2*)hpsi[b];
-      S.A = I.pool;                 // pool field 0 of the instance as the accumulator
-      S.part = I.part;
-      S.cb1 = I.cb1; S.cb2 = I.cb2; S.Kq = I.Kq; S.conv_scale = I.conv_scale;
-      S.phi_out = I.phi2;           // computed potential: the instance's first potential field
-      S.phi = conv ? I.phi2 : (phi_mode == 1 ? phi[b] : nullptr);
-      if (I.kind == kNone || I.M == 0) S.phi = (phi_mode == 1) ? phi[b] : nullptr;
-      S.twN = I.twN; S.twM = I.twM;
-    }
-    bgp_plan::StreamSched& sc = p->ssched[A0.N];
-    if (sc.tuned == 0) {
-      int rc = stream_autotune(p, sc, SL, conv, st);
-      if (rc) return rc;
-    }
     cudaStream_t gs = st;
     if (gi > 0) {
       while ((int)p->side_st.size() < gi) {
@@ -1061,24 +1125,44 @@ int bgp_apply_H_batch(bgp_plan* p, int n, const int* idx, const void* const* psi
       }
       os = p->ovl_st[gi]; oe0 = p->ovl_ev[2 * gi]; oe1 = p->ovl_ev[2 * gi + 1];
     }
-    // mu of the group, written in call order
-    int rc = BGP_OK;
-    if (mu_dev) {
+    auto group = [&](auto& SL) -> int {
+      SL.ninst = (int)grp.size();
+      for (int g = 0; g < SL.ninst; ++g) {
+        const int b = grp[g];
+        const Inst& I = p->inst[idx[b]];
+        SInst& S = SL.insts[g];
+        stream_inst(p, I, S);
+        S.psi = (const double2*)psi[b];
+        S.H = (double2*)hpsi[b];
+        S.phi = conv ? I.phi2 : (phi_mode == 1 ? phi[b] : nullptr);
+      }
+      bgp_plan::StreamSched& sc = p->ssched[A0.N];
+      if (sc.tuned == 0) {
+        int rc = stream_autotune(sc, SL, conv, gs);
+        if (rc) return rc;
+      }
+      const Sched S = sched_of(sc);
+      if (!mu_dev) return stream_run(SL, S, conv, nullptr, 0, gs, os, oe0, oe1);
       // the mu kernel writes SL order; the group's members are consecutive in the
       // output only when the caller passed them so: write each one at its own index
       double* tmp = nullptr;
-      if (!(grp.back() - grp.front() == (int)grp.size() - 1)) {
+      if (!(grp.back() - grp.front() == (int)grp.size() - 1))
         CK(cudaMallocAsync((void**)&tmp, sizeof(double) * grp.size(), gs));
-      }
-      rc = stream_run(SL, sc.ln, sc.v, sc.cln, sc.csln, sc.cv, conv, tmp ? tmp : mu_dev, tmp ? 0 : grp.front(), gs,
-                      os, oe0, oe1);
+      int rc = stream_run(SL, S, conv, tmp ? tmp : mu_dev, tmp ? 0 : grp.front(), gs, os, oe0, oe1);
       if (!rc && tmp) {
         for (int g = 0; g < SL.ninst; ++g)
           CK(cudaMemcpyAsync(mu_dev + grp[g], tmp + g, sizeof(double), cudaMemcpyDeviceToDevice, gs));
       }
       if (tmp) cudaFreeAsync(tmp, gs);
+      return rc;
+    };
+    int rc;
+    if (grp.size() == 1) {
+      SLaunchT<1> SL{};
+      rc = group(SL);
     } else {
-      rc = stream_run(SL, sc.ln, sc.v, sc.cln, sc.csln, sc.cv, conv, nullptr, 0, gs, os, oe0, oe1);
+      SLaunch SL;
+      rc = group(SL);
     }
     if (rc) return rc;
     if (gi > 0) CK(cudaEventRecord(p->side_ev[gi], gs));
@@ -1116,18 +1200,19 @@ int bgp_plan_stream_set(bgp_plan* p, int N, int lines, int radix_order, int conv
   if (!p) return fail(BGP_ERR_ARG, "null plan");
   bgp_plan::StreamSched& sc = p->ssched[N];
   if (lines == 0) { sc.tuned = 0; sc.cand.clear(); return BGP_OK; }   // tune again on next use
-  if (!stream_h_kernel(N, lines, radix_order)) return fail(BGP_ERR_UNSUPPORTED, "schedule not compiled for this N");
+  const bool known = stream_h_kernel(N, 8, 0, 0, false) != nullptr;
+  if (!known || (lines != 1 && lines != 2 && lines != 4 && lines != 8 && lines != 16) || N % lines != 0 ||
+      radix_order < 0 || radix_order > 7 || ((radix_order & 3) == 3 && N % 32 != 0))
+    return fail(BGP_ERR_UNSUPPORTED, "schedule not available for this N");
   if (conv_lines != 1 && conv_lines != 2 && conv_lines != 4 && conv_lines != 8)
     return fail(BGP_ERR_ARG, "contiguous convolution lines per tile: 1, 2, 4 or 8");
   if (conv_strided_lines != 1 && conv_strided_lines != 2 && conv_strided_lines != 4 && conv_strided_lines != 8 &&
       conv_strided_lines != 16)
     return fail(BGP_ERR_ARG, "strided convolution lines per tile: 1, 2, 4, 8 or 16");
   if (conv_order != 0 && conv_order != 3) return fail(BGP_ERR_ARG, "convolution radix order: 0 or 3");
-  if (conv_order == 3 && (2 * N) % 32 != 0) return fail(BGP_ERR_UNSUPPORTED, "register transform needs 2N = 32 R");
-  // where the convolution is compiled for this N, both of its tile widths must be
-  if (stream_conv_kernel(2 * N, 4, 0) &&
-      (!stream_conv_kernel(2 * N, conv_lines, conv_order) || !stream_conv_kernel(2 * N, conv_strided_lines, conv_order)))
-    return fail(BGP_ERR_UNSUPPORTED, "convolution tile width not compiled for this N");
+  if (conv_order == 3 && (2 * N) % 32 != 0) return fail(BGP_ERR_UNSUPPORTED, "convolution order 3 needs 2N = 32 R");
+  if (conv_strided_lines == 16 && 2 * N == 768)
+    return fail(BGP_ERR_UNSUPPORTED, "convolution tile width not available for this N");
   sc.ln = lines; sc.v = radix_order; sc.cln = conv_lines; sc.csln = conv_strided_lines; sc.cv = conv_order;
   sc.tuned = 2;
   return BGP_OK;

@@ -1,18 +1,20 @@
-// Stream passes: the Hamiltonian apply and the zero-padded convolution as plain
-// (non-persistent) launches, one launch per axis pass over every tile of every
-// instance of a batch, for the standalone and batched H psi entry points.
+// Stream passes: the Hamiltonian apply, the zero-padded convolution, the energy sums
+// and the residual as plain (non-persistent) launches, one launch per axis pass over
+// every tile of every instance of a batch, for every entry point but the solver's.
 //
 // Unlike the solver's persistent team kernel, a stream pass needs no team
 // barrier: the launch boundary orders the passes, so all SMs work on one pass at
 // a time and nothing waits on the host. Each pass is templated on
-//   L   the line length,
-//   LN  the lines per tile (one warp per line; a CTA is LN warps). On a strided
-//       axis a tile groups LN neighbours along the contiguous axis, so each of its
-//       rows is LN x 16 contiguous bytes (LN = 8: one 128-byte line),
-//   V   the radix order of the line FFT (0: largest radix first, 1: reversed,
-//       2: radix 4 first),
-// and the host's autotuner times the compiled (LN, V) candidates of a plan's grid
+//   L   the line length (N, or M = 2 N for the padded axes),
+//   C   the lines per tile. On a strided axis a tile groups C neighbours along the
+//       contiguous axis, so each of its rows is 16 C contiguous bytes,
+//   V   the line's factorization (bgp_lfft.cuh),
+//   NB  the instances the launch parameters hold (1, or a batch),
+// and the host's autotuner times the compiled (C, V) candidates of a plan's grid
 // size on its own data and keeps the fastest.
+//
+// A line lives in the registers of T = L / E threads from its load to its store
+// (bgp_lfft.cuh); shared memory only carries the exchanges between radix stages.
 //
 // H psi of an instance (operators.py:36-45 of the reference) is a sum of
 // per-axis terms: along a y-line the multiplier (k_y^2/2 - Omega x k_y), along an
@@ -20,114 +22,17 @@
 // an inverse line FFT. The passes accumulate them in a scratch field A; the last
 // pass adds (V + b2 rho + b3 rho^2 + phi) psi, writes H psi and each CTA's part
 // of Re<psi, H psi>.
+//
+// The passes of one apply are a chain of programmatic dependent launches: a pass
+// lets its successor start as soon as all its CTAs run, and waits for its
+// predecessor only where it first reads what that wrote. The later H psi passes
+// transform psi, which no pass writes, before that point, so on a grid too small to
+// fill the GPU the passes of an apply overlap.
 #pragma once
 #include "bgp_device.cuh"
-#include "bgp_regfft.cuh"
+#include "bgp_lfft.cuh"
 
 BGP_NS_BEGIN
-
-// ---------------------------------------------------------------- radix orders
-template <int V>
-BGP_HD constexpr RPlan make_rplan_v(int N) {
-  if constexpr (V == 0) {
-    return make_rplan(N);
-  } else if constexpr (V == 1) {
-    RPlan p = make_rplan(N);
-    for (int a = 0, b = p.n - 1; a < b; ++a, --b) { const int t = p.r[a]; p.r[a] = p.r[b]; p.r[b] = t; }
-    return p;
-  } else {
-    RPlan p{};
-    int m = N;
-    const int cand[5] = {4, 8, 5, 3, 2};
-    while (m > 1 && p.n < 16) {
-      int pick = 0;
-      for (int q = 0; q < 5 && !pick; ++q)
-        if (m % cand[q] == 0 && (N / cand[q]) % 32 == 0) pick = cand[q];
-      for (int q = 0; q < 5 && !pick; ++q)
-        if (m % cand[q] == 0) pick = cand[q];
-      if (!pick) { p.n = -1; return p; }
-      p.r[p.n++] = pick;
-      m /= pick;
-    }
-    return p;
-  }
-}
-
-// Host emulation of a line transform in radix order V (CPU tests of the orders).
-template <int N, int V, int S, int P, bool INV>
-inline void host_stages_v(double2* a, double2* b, const double2* tw) {
-  constexpr RPlan pl = make_rplan_v<V>(N);
-  if constexpr (S < pl.n) {
-    constexpr int R = pl.r[S];
-    constexpr int B = N / R;
-    for (int bi = 0; bi < B; ++bi) {
-      double2 v[R];
-      for (int q = 0; q < R; ++q) v[q] = a[bi + q * B];
-      const int j = butterfly_at<N, R, P, INV>(v, tw, bi);
-      for (int q = 0; q < R; ++q) b[j + q * P] = v[q];
-    }
-    for (int i = 0; i < N; ++i) a[i] = b[i];
-    host_stages_v<N, V, S + 1, P * R, INV>(a, b, tw);
-  }
-}
-
-#if defined(__CUDACC__)
-
-template <int N, int V, int S, int P, bool INV>
-BGP_D void warp_stages_v(double2* buf, const double2* __restrict__ tw, int lane) {
-  constexpr RPlan pl = make_rplan_v<V>(N);
-  if constexpr (S < pl.n) {
-    constexpr int R = pl.r[S];
-    constexpr int B = N / R;
-    constexpr int U = (B + 31) / 32;
-    double2 v[U][R];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int b = lane + 32 * u;
-      if (B % 32 == 0 || b < B) {
-#pragma unroll
-        for (int q = 0; q < R; ++q) v[u][q] = buf[swz(b + q * B)];
-      }
-    }
-    __syncwarp();
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int b = lane + 32 * u;
-      if (B % 32 == 0 || b < B) {
-        const int j = butterfly_at<N, R, P, INV>(v[u], tw, b);
-#pragma unroll
-        for (int q = 0; q < R; ++q) buf[swz(j + q * P)] = v[u][q];
-      }
-    }
-    __syncwarp();
-    warp_stages_v<N, V, S + 1, P * R, INV>(buf, tw, lane);
-  }
-}
-
-template <int N, bool INV, int V>
-BGP_D void warp_fft_v(double2* buf, const double2* __restrict__ tw, int lane) {
-  static_assert(make_rplan_v<V>(N).n > 0, "FFT length must be 2^a 3^b 5^c");
-  warp_stages_v<N, V, 0, 1, INV>(buf, tw, lane);
-}
-
-#endif  // __CUDACC__
-
-// ------------------------------------------------ register-resident line FFT
-// -------------------------------------------------------------- tile geometry
-// Shared-memory line pitch for LN lines of length L: element i of a line at
-// swz(i); the pitch keeps the LN-lane row accesses of a strided tile on distinct
-// banks (odd pitch for LN >= 8, 2 mod 8 for LN = 4).
-BGP_HD constexpr int s_pitch(int L, int LN) {
-  return (LN >= 8) ? ((L + L / 8 + 1) | 1) : (((L + L / 8 + 1 + 5) / 8) * 8 + 2);
-}
-BGP_HD constexpr size_t s_smem(int L, int LN) { return (size_t)LN * s_pitch(L, LN) * 16; }
-// Convolution passes: the line buffers, then the tile's slab of the kernel
-// quadrant, (M/2 + 1) values per line (doubles; the pitch is odd, so that the
-// lanes of a line read distinct banks).
-BGP_HD constexpr int s_kpitch(int M) { return (M / 2 + 1) | 1; }
-BGP_HD constexpr size_t s_conv_smem(int M, int LN) {
-  return s_smem(M, LN) + (((size_t)LN * s_kpitch(M) * 8 + 15) / 16) * 16;
-}
 
 // One instance of a stream batch (device copy).
 struct SInst {
@@ -139,410 +44,503 @@ struct SInst {
   const double* phi;      // long-range potential (n) or null
   double* part;           // per-tile partial sums of Re<psi, H psi> (last pass)
   // zero-padded convolution (phi from |psi|^2): scratch and kernel quadrant
-  double2* cb1;           // 2D: N x Mh; 3D: N x N x Mh
-  double2* cb2;           // 3D: N x M x Mh
+  double2* cb1;           // 2D: N x Mp; 3D: N x N x Mp    (Mp = conv_pitch(N))
+  double2* cb2;           // 3D: N x M x Mp
   const double* Kq;       // real even quadrant of the kernel transform, (Mh)^d
-  double* phi_out;        // computed potential (n)
+  double* phi_out;        // computed potential (n), or null (only its sum is wanted)
   double conv_scale;      // -G_C dV / M^d
-  const double2* twN;
-  const double2* twM;
+  const double* rho;      // the convolution's density, or null: |psi|^2
+  double* gpart;          // per-tile partial sums of phi rho (last convolution pass), or null
+  double hscale;          // H psi is written times this
+  const double2* twM;     // w_M^t, t < M
+  const double2* tabN[kLVariants];   // line-transform tables (lf_fill_table)
+  const double2* tabM[kLVariants];
 };
 
-// A launch of one pass over up to kStreamBatch instances of one size, passed by
-// value (kernel parameter space), so nothing is staged in device memory per call.
+// A launch of one pass over up to NB instances of one size, passed by value (kernel
+// parameter space), so nothing is staged in device memory per call. A single
+// instance has its own, small parameter block: the 64-instance block is 17 KB that
+// every launch would copy.
 constexpr int kStreamBatch = 64;
-struct SLaunch {
-  SInst insts[kStreamBatch];
+template <int NB>
+struct SLaunchT {
+  SInst insts[NB];
   int ninst;
   int tiles;              // tiles of one instance in this pass
 };
+using SLaunch = SLaunchT<kStreamBatch>;
 
-// lines of the last (contiguous) axis of an instance
-BGP_HD int ndim_lines(const SInst& I) { return I.ndim == 2 ? I.N : I.N * I.N; }
+// Row pitch of the convolution scratch: N + 1 spectral columns, rows of whole
+// 128-byte lines (N is a multiple of 8), so a tile's rows are aligned.
+BGP_HD constexpr int conv_pitch(int N) { return N + 8; }
 
-// flat index of element r of line c of tile t along axis ax (N-lines)
-template <int LN>
-BGP_D int s_elem(int ndim, int N, int ax, int t, int r, int c, int& i, int& j, int& k) {
-  if (ndim == 2) {
-    k = 0;
-    if (ax == 1) { i = t * LN + c; j = r; } else { j = t * LN + c; i = r; }
-    return i * N + j;
-  }
-  const int tpl = N / LN;
-  if (ax == 2) { const int line = t * LN + c; i = line / N; j = line - i * N; k = r; }
-  else if (ax == 1) { i = t / tpl; k = (t - i * tpl) * LN + c; j = r; }
-  else { j = t / tpl; k = (t - j * tpl) * LN + c; i = r; }
-  return (i * N + j) * N + k;
+// lines per tile with the CTA filled up to a warp (the lines beyond C idle)
+BGP_HD constexpr int s_cp(int L, int C, int V) { return C * lf_threads(L, V) >= 32 ? C : 32 / lf_threads(L, V); }
+BGP_HD constexpr int s_threads(int L, int C, int V) { return s_cp(L, C, V) * lf_threads(L, V); }
+BGP_HD constexpr size_t s_smem(int L, int C, int V) { return (size_t)s_cp(L, C, V) * lf_slots(L, V) * 16; }
+// resident threads per SM the registers are budgeted for: 24 values a thread need
+// about 170 registers, 16 or 12 fit in 128, 8 in 80
+BGP_HD constexpr int s_min_blocks(int L, int C, int V) {
+  const int E = lplan(L, V).E, want = E > 16 ? 384 : (E > 8 ? 512 : 768);
+  const int b = want / s_threads(L, C, V);
+  return b < 1 ? 1 : (b > 16 ? 16 : b);
 }
+
+// A compiled pass: its entry and launch geometry (evaluated at compile time).
+struct SKernel {
+  void* fn;
+  int threads;
+  size_t smem;
+};
 
 #if defined(__CUDACC__)
 
-template <int L, int LN, bool CONTIG>
-BGP_D void s_map(int e, int& r, int& c) {
-  if (CONTIG) { c = e / L; r = e - c * L; } else { r = e / LN; c = e - r * LN; }
+// programmatic dependent launch: let the next pass start; wait for the previous one
+BGP_D void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;"); }
+BGP_D void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Thread and buffer layout of a tile: on the contiguous axis the T threads of a line
+// are neighbours (and, for T <= 32, in one warp); on a strided axis the lines are.
+template <int L, int C, int V, bool CONTIG>
+struct Tile {
+  static constexpr int T = lf_threads(L, V), CP = s_cp(L, C, V), E = lplan(L, V).E;
+  static constexpr bool WARP = CONTIG && T <= 32;
+  using Fft = LineFft<L, V, CONTIG ? 1 : CP, WARP>;
+  int c, t;
+  BGP_D Tile() {
+    const int tid = threadIdx.x;
+    c = CONTIG ? tid / T : tid % CP;
+    t = CONTIG ? tid % T : tid / CP;
+  }
+  BGP_D double2* line(double2* sm) const { return sm + (CONTIG ? c * lf_slots(L, V) : c); }
+};
+
+// Sums of NV values over the CTA (W warps) in a fixed order; thread 0 holds the totals.
+template <int W, int NV>
+BGP_D void block_sums(double (&v)[NV]) {
+  __shared__ double red[NV * W];
+#pragma unroll
+  for (int q = 0; q < NV; ++q) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
+  }
+  if constexpr (W > 1) {
+    if ((threadIdx.x & 31) == 0) {
+#pragma unroll
+      for (int q = 0; q < NV; ++q) red[q * W + (threadIdx.x >> 5)] = v[q];
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll
+      for (int q = 0; q < NV; ++q) {
+        double s = 0.0;
+        for (int w = 0; w < W; ++w) s += red[q * W + w];
+        v[q] = s;
+      }
+    }
+  }
 }
 
 // --------------------------------------------------------------- H psi pass
-// stage 0: A = T(psi) on the first (contiguous) axis; 1: A += T(psi) (3D middle);
+// STAGE 0: A = T(psi) on the contiguous axis; 1: A += T(psi) (3D, middle axis);
 // 2: H = A + T(psi) + (V + b2 rho + b3 rho^2 + phi) psi and the CTA's part of
 // Re<psi, H> (axis 0). T = inverse FFT o multiplier o forward FFT along the axis.
-// Transform of one warp's line b (shared memory, natural order) by radix order
-// V (0-2: Stockham stages in shared memory, 3: the register-resident transform).
-// mode 0: forward only; 1: inverse only; 2: forward, v <- mult(k, v), inverse.
-// The result is left in b in natural order.
-template <int L, int V, class F>
-BGP_D void line_xform(double2* b, const double2* __restrict__ tw, int lane, int mode, F mult) {
-  if constexpr (V == 3) {
-    constexpr int R = L / 32;
-    const int kb = R * rev5(lane);
-    double2 v[R];
-    if (mode == 1) {
-#pragma unroll
-      for (int k1 = 0; k1 < R; ++k1) v[k1] = b[swz(k1 + kb)];
-    } else {
-#pragma unroll
-      for (int q = 0; q < R; ++q) v[q] = b[swz(lane + 32 * q)];
-    }
-    __syncwarp();
-    if (mode != 1) reg_fft_fwd<L>(v, tw, lane);
-    if (mode == 2) {
-#pragma unroll
-      for (int k1 = 0; k1 < R; ++k1) v[k1] = mult(k1 + kb, v[k1]);
-    }
-    if (mode != 0) reg_fft_inv<L>(v, tw, lane);
-    if (mode == 0) {
-#pragma unroll
-      for (int k1 = 0; k1 < R; ++k1) b[swz(k1 + kb)] = v[k1];
-    } else {
-#pragma unroll
-      for (int q = 0; q < R; ++q) b[swz(lane + 32 * q)] = v[q];
-    }
-    __syncwarp();
-  } else {
-    if (mode != 1) warp_fft_v<L, false, V>(b, tw, lane);
-    if (mode == 2) {
-      constexpr int PL = (L + 31) / 32;
-#pragma unroll
-      for (int q = 0; q < PL; ++q) {
-        const int r = lane + 32 * q;
-        if (L % 32 == 0 || r < L) b[swz(r)] = mult(r, b[swz(r)]);
-      }
-      __syncwarp();
-    }
-    if (mode != 0) warp_fft_v<L, true, V>(b, tw, lane);
-  }
-}
-
-// Occupancy floor of the stream passes: 16 warps per SM (at most 128 registers).
-template <int LN>
-constexpr int s_min_blocks() { return (LN >= 16) ? 1 : 16 / LN; }
-
-// V: 0-3 the line transform (see line_xform) at 16 warps per SM; 4-7 the same
-// transform (V - 4) with the register budget halved for 32 warps per SM.
-template <int N, int LN, int V>
-__global__ void __launch_bounds__(LN * 32, (V >= 4 ? 2 : 1) * s_min_blocks<LN>()) k_stream_h(SLaunch SL, int ax,
-                                                                                            int stage) {
-  constexpr int VT = V & 3;   // the line transform
+//
+// Bound: 256^3 moves 268 MB per field and pass and is bound by HBM; a single plane
+// grid is a few microseconds of latency (one tile per CTA).
+template <int N, int C, int V, int STAGE, int NB>
+__global__ void __launch_bounds__(s_threads(N, C, V), s_min_blocks(N, C, V))
+    k_stream_h(const __grid_constant__ SLaunchT<NB> SL) {
+  constexpr bool CONTIG = STAGE == 0;
+  using TL = Tile<N, C, V, CONTIG>;
+  constexpr int E = TL::E, T = TL::T;
   extern __shared__ double2 sm[];
-  constexpr int NT = LN * 32, TOT = LN * N, PER = (TOT + NT - 1) / NT, LS = s_pitch(N, LN);
-  constexpr int CH = PER < 4 ? PER : 4;    // elements per thread in flight on the way out
-  const int inst = blockIdx.x / SL.tiles, t = blockIdx.x - inst * SL.tiles;
+  const int inst = NB == 1 ? 0 : blockIdx.x / SL.tiles, tile = blockIdx.x - inst * SL.tiles;
   const SInst& I = SL.insts[inst];
-  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  const int ndim = I.ndim;
-  const bool contig = (ax == ndim - 1);
+  const TL tl;
+  const int c = tl.c, t = tl.t, ndim = I.ndim;
+  const bool valid = c < C;
+  pdl_trigger();
+  // line (i, j[, k]) of this thread: element r at base + r * str; its coordinate across
+  // the rotation plane (xo) and, for the trap, the squared radius of the fixed axes
+  int base, str, ci = 0, cj = 0, ck = 0;
+  if (STAGE == 0) {
+    const int line = tile * C + c;
+    base = line * N; str = 1;
+    ci = line;                                   // 2D: i = line
+  } else if (ndim == 2) {
+    cj = tile * C + c;
+    base = cj; str = N;
+  } else {
+    constexpr int tpl = N / C;
+    const int a = tile / tpl;
+    ck = (tile - a * tpl) * C + c;
+    if (STAGE == 1) { ci = a; base = a * N * N + ck; str = N; }
+    else { cj = a; base = a * N + ck; str = N * N; }
+  }
   const double2* __restrict__ psi = I.psi;
-  auto where = [&](int e, int& r, int& c) {
-    if (contig) s_map<N, LN, true>(e, r, c); else s_map<N, LN, false>(e, r, c);
-  };
-  if constexpr (VT == 3) {
-    if (contig && stage == 0) {
-      // contiguous lines straight from and to global memory: warp w owns line
-      // t LN + w, lane l slot q element l + 32 q (coalesced in every q)
-      constexpr int R = N / 32;
-      const int line = t * LN + w;
-      const size_t base = (size_t)line * N;
-      double2 v[R];
+  double2 v[E];
 #pragma unroll
-      for (int q = 0; q < R; ++q) v[q] = __ldg(psi + base + lane + 32 * q);
-      reg_fft_fwd<N>(v, I.twN, lane);
-      // 2D y-line: wx = -Omega x(i), i = line; 3D z-line: no rotation term
-      const double wx = (ndim == 2) ? -I.Omega * ((double)(line - N / 2) * I.dx) : 0.0;
-      const double inv = 1.0 / (double)N, kf = I.kfac;
-      const int kb = R * rev5(lane);
-#pragma unroll
-      for (int k1 = 0; k1 < R; ++k1) {
-        const int kk_i = k1 + kb;
-        const int mm = (kk_i < (N + 1) / 2) ? kk_i : kk_i - N;
-        const double kk = kTwoPi * ((double)mm * kf);
-        v[k1] = cscale(v[k1], (0.5 * kk * kk + wx * kk) * inv);
-      }
-      reg_fft_inv<N>(v, I.twN, lane);
-#pragma unroll
-      for (int q = 0; q < R; ++q) I.A[base + lane + 32 * q] = v[q];
-      return;
-    }
-  }
-  // load the tile: every load of the thread first, then into shared memory
+  for (int q = 0; q < E; ++q) v[q] = valid ? __ldg(psi + base + (t + T * q) * str) : cmk(0.0, 0.0);
+  const typename TL::Fft fft{tl.line(sm), I.tabN[V], t};
+  fft.template forward<false>(v);
   {
-    double2 va[PER];
+    const double dx = I.dx, Om = I.Omega, kf = I.kfac, inv = 1.0 / (double)N;
+    double wx = 0.0;                             // y-line: -Omega x(i); x-line: +Omega y(j)
+    if (STAGE == 2) wx = Om * ((double)(cj - N / 2) * dx);
+    else if (STAGE == 1 || ndim == 2) wx = -Om * ((double)(ci - N / 2) * dx);
 #pragma unroll
-    for (int q = 0; q < PER; ++q) {
-      const int e = tid + q * NT;
-      if (TOT % NT == 0 || e < TOT) {
-        int r, c, i, j, k;
-        where(e, r, c);
-        va[q] = __ldg(psi + s_elem<LN>(ndim, N, ax, t, r, c, i, j, k));
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < PER; ++q) {
-      const int e = tid + q * NT;
-      if (TOT % NT == 0 || e < TOT) {
-        int r, c;
-        where(e, r, c);
-        sm[c * LS + swz(r)] = va[q];
-      }
-    }
-  }
-  __syncthreads();
-  {
-    double2* b = sm + w * LS;
-    int i, j, k;
-    s_elem<LN>(ndim, N, ax, t, 0, w, i, j, k);
-    const double dx = I.dx, Om = I.Omega;
-    const double wx = (ax == 1) ? -Om * ((double)(i - N / 2) * dx)
-                                : ((ax == 0) ? Om * ((double)(j - N / 2) * dx) : 0.0);
-    const double inv = 1.0 / (double)N, kf = I.kfac;
-    line_xform<N, VT>(b, I.twN, lane, 2, [&](int r, double2 x) {
-      const int mm = (r < (N + 1) / 2) ? r : r - N;
+    for (int q = 0; q < E; ++q) {
+      const int r = t + T * q, mm = (r < (N + 1) / 2) ? r : r - N;
       const double kk = kTwoPi * ((double)mm * kf);
-      return cscale(x, (0.5 * kk * kk + wx * kk) * inv);
-    });
+      v[q] = cscale(v[q], (0.5 * kk * kk + wx * kk) * inv);
+    }
   }
-  __syncthreads();
+  fft.template inverse<false>(v);
+  if (STAGE > 0) pdl_wait();                     // A, and phi, come from the passes before
   double acc = 0.0;
-#pragma unroll 1
-  for (int q0 = 0; q0 < PER; q0 += CH) {
-    // issue the chunk's loads (A, and psi and phi on the last axis), then use them
+  constexpr int CH = E % 4 == 0 ? 4 : 3;         // elements in flight on the way out
+#pragma unroll
+  for (int q0 = 0; q0 < E; q0 += CH) {
     double2 pa[CH], pv[CH];
     double pp[CH];
-    int f[CH];
 #pragma unroll
     for (int u = 0; u < CH; ++u) {
-      const int e = tid + (q0 + u) * NT;
-      f[u] = -1;
-      if (q0 + u < PER && (TOT % NT == 0 || e < TOT)) {
-        int r, c, i, j, k;
-        where(e, r, c);
-        f[u] = s_elem<LN>(ndim, N, ax, t, r, c, i, j, k);
-        if (stage > 0) pa[u] = I.A[f[u]];
-        if (stage == 2) {
-          pv[u] = __ldg(psi + f[u]);
-          pp[u] = I.phi ? __ldg(I.phi + f[u]) : 0.0;
-        }
+      const int f = base + (t + T * (q0 + u)) * str;
+      if (STAGE > 0) pa[u] = valid ? I.A[f] : cmk(0.0, 0.0);
+      if (STAGE == 2) {
+        pv[u] = valid ? __ldg(psi + f) : cmk(0.0, 0.0);
+        pp[u] = (valid && I.phi) ? I.phi[f] : 0.0;
       }
     }
 #pragma unroll
     for (int u = 0; u < CH; ++u) {
-      if (f[u] < 0) continue;
-      const int e = tid + (q0 + u) * NT;
-      int r, c, i, j, k;
-      where(e, r, c);
-      const double2 v = sm[c * LS + swz(r)];
-      if (stage == 0) { I.A[f[u]] = v; continue; }
-      const double2 a2 = cadd(pa[u], v);
-      if (stage == 1) { I.A[f[u]] = a2; continue; }
-      s_elem<LN>(ndim, N, ax, t, r, c, i, j, k);
+      const int r = t + T * (q0 + u), f = base + r * str;
+      if (STAGE == 0) { if (valid) I.A[f] = v[q0 + u]; continue; }
+      const double2 a2 = cadd(pa[u], v[q0 + u]);
+      if (STAGE == 1) { if (valid) I.A[f] = a2; continue; }
       const double2 p = pv[u];
       const double rho = cabs2(p);
       // trap tc r^s from the indices (becgpp/grid.py:90-91)
-      const double x = (double)(i - N / 2) * I.dx, y = (double)(j - N / 2) * I.dx;
+      const double x = (double)(r - N / 2) * I.dx, y = (double)(cj - N / 2) * I.dx;
       double r2 = x * x + y * y;
-      if (ndim == 3) { const double z = (double)(k - N / 2) * I.dx; r2 = r2 + z * z; }
+      if (ndim == 3) { const double z = (double)(ck - N / 2) * I.dx; r2 = r2 + z * z; }
       const double Vt = (I.s <= 0.0) ? 0.0 : ((I.s == 2.0) ? I.tc * r2 : I.tc * pow(r2, 0.5 * I.s));
       const double pot = Vt + I.beta2 * rho + I.beta3 * rho * rho + pp[u];
       const double2 h = cadd(a2, cscale(p, pot));
-      I.H[f[u]] = h;
+      if (valid) I.H[f] = cscale(h, I.hscale);
       acc += p.x * h.x + p.y * h.y;
     }
   }
-  if (stage == 2 && I.part) {
-    __shared__ double red[LN];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (lane == 0) red[w] = acc;
-    __syncthreads();
-    if (tid == 0) {
-      double s = 0.0;
-#pragma unroll
-      for (int q = 0; q < LN; ++q) s += red[q];
-      I.part[t] = s;
-    }
+  if (STAGE == 2 && I.part) {
+    double g[1] = {acc};
+    block_sums<s_threads(N, C, V) / 32, 1>(g);
+    if (threadIdx.x == 0) I.part[tile] = g[0];
   }
 }
 
 // ------------------------------------------------- zero-padded convolution
-// The padded density of an instance lives in the M^d box with the N^d grid at
-// offset i0 = (M - N)/2; only M/2+1 spectral columns of the last axis are kept
-// (the input is real), only the N^d central outputs are written, and K^ is read
-// from its real even quadrant Kq.
-//   step a  (2D/3D): lines of the last axis, padded: FFT, keep kj <= M/2 -> cb1
-//   step b  (2D): columns kj along i: FFT, times K^, inverse FFT, central i -> cb1
-//   3D: step b fwd (j-lines) cb1 -> cb2, step c (i-lines: FFT, K^, IFFT) in cb2,
-//       step b inv (j-lines) cb2 -> cb1 (central j)
-//   last   : lines of the last axis: Hermitian rebuild, inverse FFT, central part:
-//            phi = conv_scale * Re
-// op: 0 step a, 1 2D step b, 2 3D step b fwd, 3 3D step c, 4 3D step b inv, 5 last.
-template <int M, int LN, int V>
-__global__ void __launch_bounds__(LN * 32, s_min_blocks<LN>()) k_stream_conv(SLaunch SL, int op) {
+// phi = conv_scale (K * rho) on the N^d grid, cyclic in the M^d box (M = 2 N). The
+// grid sits at the box's origin (a cyclic convolution commutes with the shift), so the
+// upper half of every padded line is zero on the way in and unused on the way out.
+//   step a  lines of the last axis: real transform, columns kk <= N kept   -> cb1
+//   2D: columns along i: forward, times K^, inverse, rows i < N            -> cb1
+//   3D: step b (along j) cb1 -> cb2, step c (along i: forward, K^, inverse) in cb2,
+//       step d (inverse along j) cb2 -> cb1
+//   last    lines of the last axis: inverse real transform, phi
+// A real line of M points is one complex transform of N: z_n = x_2n + i x_(2n+1), and
+//   X_k = E_k + w_M^k O_k,  E_k = (Z_k + conj Z_(N-k)) / 2,  O_k = (Z_k - conj Z_(N-k)) / 2i.
+
+// step a (INV = 0) and the last step (INV = 1)
+template <int N, int C, int V, int INV, int NB>
+__global__ void __launch_bounds__(s_threads(N, C, V), s_min_blocks(N, C, V))
+    k_stream_real(const __grid_constant__ SLaunchT<NB> SL) {
+  using TL = Tile<N, C, V, true>;
+  constexpr int E = TL::E, T = TL::T, Mp = conv_pitch(N);
   extern __shared__ double2 sm[];
-  constexpr int NT = LN * 32, TOT = LN * M, PER = (TOT + NT - 1) / NT, LS = s_pitch(M, LN);
-  const int inst = blockIdx.x / SL.tiles, t = blockIdx.x - inst * SL.tiles;
+  const int inst = NB == 1 ? 0 : blockIdx.x / SL.tiles, tile = blockIdx.x - inst * SL.tiles;
   const SInst& I = SL.insts[inst];
-  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  const int N = I.N, Mh = I.Mh, i0 = I.i0;
-  const bool contig = (op == 0 || op == 5);
-  const int tpl = (Mh + LN - 1) / LN;
-  // decode (a, b) of the tile's line c for the strided ops
-  auto line_ab = [&](int c, int& a, int& b2) {
-    if (op == 1) { a = t * LN + c; b2 = 0; }                  // 2D column kj
-    else { a = t / tpl; b2 = (t - a * tpl) * LN + c; }       // 3D: (i or jj, kk)
-  };
-  // kernel multiply (ops 1, 3): K^ is real and even, so line c needs the
-  // M/2 + 1 values K^[a, ...] of its quadrant; the LN lines of a tile are
-  // consecutive in the quadrant's contiguous index, so the slab is read as runs
-  // of LN doubles, issued with the tile's own loads
-  constexpr int KH = M / 2 + 1, KP = s_kpitch(M), KTOT = KH * LN, KPER = (KTOT + NT - 1) / NT;
-  double* ks = reinterpret_cast<double*>(sm + LN * LS);
-  const bool kmul = (op == 1 || op == 3);
-  const size_t mh = (size_t)Mh;
-  double kv[KPER];
-  if (kmul) {
-    int a1 = 0, a2 = 0;
-    line_ab(0, a1, a2);
-    const int bj = (a1 <= M / 2) ? a1 : M - a1;
+  const TL tl;
+  const int t = tl.t, line = tile * C + tl.c;
+  const bool valid = tl.c < C;
+  double2* b = tl.line(sm);
+  const typename TL::Fft fft{b, I.tabN[V], t};
+  const double2* __restrict__ tw = I.twM;
+  double2 v[E];
+  pdl_trigger();
+  if (INV == 0) {
+    const double2* __restrict__ psi = I.psi + (size_t)line * N;
+    const double2* __restrict__ rho = reinterpret_cast<const double2*>(I.rho + (size_t)line * N);
+    const bool given = I.rho != nullptr;
 #pragma unroll
-    for (int q = 0; q < KPER; ++q) {
-      const int e = tid + q * NT;
-      kv[q] = 0.0;
-      if (KTOT % NT == 0 || e < KTOT) {
-        const int a = e / LN, c = e - a * LN;
-        // op 1: column kj = a1 + c of row a; op 3: (a, bj, kk = a2 + c)
-        const int col = (op == 1 ? a1 : a2) + c;
-        if (col < Mh) kv[q] = __ldg(I.Kq + ((op == 1) ? (size_t)a * mh : ((size_t)a * mh + bj) * mh) + col);
+    for (int q = 0; q < E / 2; ++q) {
+      const int n = t + T * q;
+      v[q] = cmk(0.0, 0.0);
+      if (valid) {
+        if (given) v[q] = __ldg(rho + n);
+        else v[q] = cmk(cabs2(__ldg(psi + 2 * n)), cabs2(__ldg(psi + 2 * n + 1)));
       }
     }
-  }
-  double2 va[PER];
+    fft.template forward<true>(v);
+    TL::Fft::sync();
 #pragma unroll
-  for (int q = 0; q < PER; ++q) {
-    const int e = tid + q * NT;
-    va[q] = cmk(0.0, 0.0);
-    if (!(TOT % NT == 0 || e < TOT)) continue;
-    int r, c;
-    if (contig) s_map<M, LN, true>(e, r, c); else s_map<M, LN, false>(e, r, c);
-    if (op == 0) {
-      const int line = t * LN + c, j = r - i0;
-      if (j >= 0 && j < N && line < (ndim_lines(I))) {
-        const double2 p = __ldg(I.psi + (size_t)line * N + j);
-        va[q] = cmk(cabs2(p), 0.0);
+    for (int q = 0; q < E; ++q) b[t + T * q] = v[q];
+    TL::Fft::sync();
+    double2* out = I.cb1 + (size_t)line * Mp;
+#pragma unroll
+    for (int q = 0; q < E; ++q) {
+      const int k = t + T * q;
+      const double2 z = v[q], p = b[k ? N - k : 0];     // p: Z_(N-k), conjugated below
+      const double2 e = cmk(0.5 * (z.x + p.x), 0.5 * (z.y - p.y));
+      const double2 o = cmk(0.5 * (z.y + p.y), 0.5 * (p.x - z.x));
+      if (valid) out[k] = cadd(e, cmul(o, __ldg(tw + k)));
+    }
+    if (t == 0 && valid) out[N] = cmk(v[0].x - v[0].y, 0.0);
+  } else {
+    pdl_wait();
+    const double2* in = I.cb1 + (size_t)line * Mp;
+#pragma unroll
+    for (int q = 0; q < E; ++q) v[q] = valid ? in[t + T * q] : cmk(0.0, 0.0);
+#pragma unroll
+    for (int q = 0; q < E; ++q) b[t + T * q] = v[q];
+    if (t == 0) b[N] = valid ? in[N] : cmk(0.0, 0.0);
+    TL::Fft::sync();
+#pragma unroll
+    for (int q = 0; q < E; ++q) {
+      const int k = t + T * q;
+      const double2 x = v[q], p = b[N - k];
+      const double2 e = cmk(x.x + p.x, x.y - p.y);       // X_k + conj X_(N-k)
+      const double2 d = cmk(x.x - p.x, x.y + p.y);       // X_k - conj X_(N-k)
+      const double2 o = cconjmul(__ldg(tw + k), d);      // times conj w_M^k
+      v[q] = cmk(e.x - o.y, e.y + o.x);                  // e + i o
+    }
+    fft.template inverse<true>(v);
+    double2* out = reinterpret_cast<double2*>(I.phi_out + (size_t)line * N);
+    const bool store = valid && I.phi_out != nullptr;
+    const double sc = I.conv_scale;
+#pragma unroll
+    for (int q = 0; q < E / 2; ++q) {
+      v[q] = cscale(v[q], sc);
+      if (store) out[t + T * q] = v[q];
+    }
+    if (I.gpart) {
+      // the tile's part of sum phi |psi|^2
+      const double2* __restrict__ psi = I.psi + (size_t)line * N;
+      double g[1] = {0.0};
+#pragma unroll
+      for (int q = 0; q < E / 2; ++q) {
+        const int n = t + T * q;
+        if (valid) g[0] += v[q].x * cabs2(__ldg(psi + 2 * n)) + v[q].y * cabs2(__ldg(psi + 2 * n + 1));
       }
-    } else if (op == 5) {
-      const int line = t * LN + c;
-      if (line < ndim_lines(I)) {
-        const double2* row = I.cb1 + (size_t)line * Mh;
-        if (r < Mh) va[q] = row[r];
-        else { const double2 v = row[M - r]; va[q] = cmk(v.x, -v.y); }
-      }
-    } else if (op == 1) {
-      int kj, u;
-      line_ab(c, kj, u);
-      const int i = r - i0;
-      if (kj < Mh && i >= 0 && i < N) va[q] = I.cb1[(size_t)i * Mh + kj];
-    } else if (op == 2) {
-      int i, kk;
-      line_ab(c, i, kk);
-      const int j = r - i0;
-      if (kk < Mh && j >= 0 && j < N) va[q] = I.cb1[((size_t)i * N + j) * Mh + kk];
-    } else if (op == 3) {
-      int jj, kk;
-      line_ab(c, jj, kk);
-      const int i = r - i0;
-      if (kk < Mh && i >= 0 && i < N) va[q] = I.cb2[((size_t)i * M + jj) * Mh + kk];
-    } else {  // op 4
-      int i, kk;
-      line_ab(c, i, kk);
-      if (kk < Mh) va[q] = I.cb2[((size_t)i * M + r) * Mh + kk];
+      block_sums<s_threads(N, C, V) / 32, 1>(g);
+      if (threadIdx.x == 0) I.gpart[tile] = g[0];
     }
   }
+}
+
+// strided steps: MODE 0: step b (forward); 1: 2D columns and 3D step c (forward, K^,
+// inverse); 2: step d (inverse)
+template <int M, int C, int V, int MODE, int NB>
+__global__ void __launch_bounds__(s_threads(M, C, V), s_min_blocks(M, C, V))
+    k_stream_pad(const __grid_constant__ SLaunchT<NB> SL) {
+  using TL = Tile<M, C, V, false>;
+  constexpr int E = TL::E, T = TL::T, N = M / 2, Mh = N + 1, Mp = conv_pitch(N), tpl = (Mh + C - 1) / C;
+  extern __shared__ double2 sm[];
+  const int inst = NB == 1 ? 0 : blockIdx.x / SL.tiles, tile = blockIdx.x - inst * SL.tiles;
+  const SInst& I = SL.insts[inst];
+  const TL tl;
+  const int t = tl.t;
+  const int a = tile / tpl, kk = (tile - a * tpl) * C + tl.c;   // a: i (b, d) or jj (c); 0 in 2D
+  const bool valid = tl.c < C && kk < Mh;
+  const typename TL::Fft fft{tl.line(sm), I.tabM[V], t};
+  pdl_trigger();
+  const double2* in;
+  double2* out;
+  size_t si, so;
+  if (MODE == 1) {
+    out = I.ndim == 2 ? I.cb1 + kk : I.cb2 + (size_t)a * Mp + kk;
+    in = out;
+    si = so = I.ndim == 2 ? (size_t)Mp : (size_t)M * Mp;
+  } else {
+    double2* x1 = I.cb1 + (size_t)a * N * Mp + kk;
+    double2* x2 = I.cb2 + (size_t)a * M * Mp + kk;
+    in = MODE == 0 ? x1 : x2;
+    out = MODE == 0 ? x2 : x1;
+    si = so = Mp;
+  }
+  pdl_wait();
+  double2 v[E];
 #pragma unroll
-  for (int q = 0; q < PER; ++q) {
-    const int e = tid + q * NT;
-    if (TOT % NT == 0 || e < TOT) {
-      int r, c;
-      if (contig) s_map<M, LN, true>(e, r, c); else s_map<M, LN, false>(e, r, c);
-      sm[c * LS + swz(r)] = va[q];
+  for (int q = 0; q < (MODE == 2 ? E : E / 2); ++q)
+    v[q] = valid ? in[(size_t)(t + T * q) * si] : cmk(0.0, 0.0);
+  if (MODE != 2) fft.template forward<true>(v);
+  if (MODE == 1) {
+    // K^ is real and even: K^[min(k, M - k)] of the quadrant's column
+    const int bj = a <= N ? a : M - a;
+    const double* __restrict__ K = I.Kq + (I.ndim == 2 ? (size_t)0 : (size_t)bj * Mh) + kk;
+    const size_t sk = I.ndim == 2 ? (size_t)Mh : (size_t)Mh * Mh;
+#pragma unroll
+    for (int q = 0; q < E; ++q) {
+      const int k = t + T * q;
+      const double kv = valid ? __ldg(K + (size_t)(k <= N ? k : M - k) * sk) : 0.0;
+      v[q] = cscale(v[q], kv);
     }
   }
-  if (kmul) {
+  if (MODE != 0) fft.template inverse<true>(v);
 #pragma unroll
-    for (int q = 0; q < KPER; ++q) {
-      const int e = tid + q * NT;
-      if (KTOT % NT == 0 || e < KTOT) {
-        const int a = e / LN, c = e - a * LN;
-        ks[c * KP + a] = kv[q];
+  for (int q = 0; q < (MODE == 0 ? E : E / 2); ++q)
+    if (valid) out[(size_t)(t + T * q) * so] = v[q];
+}
+
+// ------------------------------------------------------------------ energy sums
+// The sums of energy_components (operators.py:10-29 of the reference) over a state as
+// given: on the contiguous axis the local sums of rho = |psi|^2, on every axis the
+// spectral sums  sum k^2 |psi^|^2  and, for L_z,  X sum k_y |psi^|^2  and
+// Y sum k_x |psi^|^2  (Parseval along one axis). All axes' tiles are one launch: block
+// b of axis slot a = b / tiles; slot 0 is the contiguous axis. Each block leaves
+// kESums sums and one maximum in I.part, value q of block b at q * gridDim.x + b.
+enum : int { E_N0, E_V, E_2, E_3, E_R2, E_PERP, E_Z2, E_K, E_L, kESums };
+template <int N, int C, int V>
+__global__ void __launch_bounds__(s_threads(N, C, V), s_min_blocks(N, C, V))
+    k_stream_energy(const __grid_constant__ SLaunchT<1> SL) {
+  constexpr int T = lf_threads(N, V), E = lplan(N, V).E, W = s_threads(N, C, V) / 32;
+  extern __shared__ double2 sm[];
+  const SInst& I = SL.insts[0];
+  const int slot = blockIdx.x / SL.tiles, tile = blockIdx.x - slot * SL.tiles, ndim = I.ndim;
+  const double2* __restrict__ psi = I.psi;
+  const double dx = I.dx, kf = I.kfac;
+  double sum[kESums], mx = 0.0, fixed = 0.0;     // fixed: the L_z coordinate of the line
+#pragma unroll
+  for (int q = 0; q < kESums; ++q) sum[q] = 0.0;
+  double2 v[E];
+  int t;
+  bool valid;
+  if (slot == 0) {
+    const Tile<N, C, V, true> tl;
+    t = tl.t;
+    valid = tl.c < C;
+    const int line = tile * C + tl.c;
+    const int i = ndim == 2 ? line : line / N, j = line - i * N;
+    const double x = (double)(i - N / 2) * dx, y3 = (double)(j - N / 2) * dx;
+    if (ndim == 2) fixed = x;
+#pragma unroll
+    for (int q = 0; q < E; ++q) {
+      const int r = t + T * q;
+      v[q] = valid ? __ldg(psi + (size_t)line * N + r) : cmk(0.0, 0.0);
+      const double p = cabs2(v[q]);
+      const double c = (double)(r - N / 2) * dx;
+      // (x, y) = (x_i, x_r) in 2D; (x_i, x_j, x_r) in 3D
+      const double y = ndim == 2 ? c : y3;
+      const double rp = x * x + y * y;
+      double r2 = rp;
+      if (ndim == 3) {
+        r2 = r2 + c * c;
+        sum[E_PERP] += rp * p;
+        sum[E_Z2] += c * c * p;
       }
+      const double Vt = (I.s <= 0.0) ? 0.0 : ((I.s == 2.0) ? I.tc * r2 : I.tc * pow(r2, 0.5 * I.s));
+      sum[E_N0] += p;
+      sum[E_V] += Vt * p;
+      sum[E_2] += p * p;
+      sum[E_3] += p * p * p;
+      sum[E_R2] += r2 * p;
+      mx = fmax(mx, p);
     }
+    const typename Tile<N, C, V, true>::Fft fft{tl.line(sm), I.tabN[V], t};
+    fft.template forward<false>(v);
+  } else {
+    const Tile<N, C, V, false> tl;
+    t = tl.t;
+    valid = tl.c < C;
+    // slot 1: axis 0 (x); slot 2 (3D): axis 1 (y)
+    int base, str;
+    if (ndim == 2) {
+      base = tile * C + tl.c; str = N;
+      fixed = (double)(base - N / 2) * dx;
+    } else {
+      constexpr int tpl = N / C;
+      const int a = tile / tpl, k = (tile - a * tpl) * C + tl.c;
+      base = slot == 1 ? a * N + k : a * N * N + k;
+      str = slot == 1 ? N * N : N;
+      fixed = (double)(a - N / 2) * dx;
+    }
+#pragma unroll
+    for (int q = 0; q < E; ++q) v[q] = valid ? __ldg(psi + base + (t + T * q) * str) : cmk(0.0, 0.0);
+    const typename Tile<N, C, V, false>::Fft fft{tl.line(sm), I.tabN[V], t};
+    fft.template forward<false>(v);
   }
+  double sl = 0.0;
+#pragma unroll
+  for (int q = 0; q < E; ++q) {
+    const int r = t + T * q, mm = (r < (N + 1) / 2) ? r : r - N;
+    const double kk = kTwoPi * ((double)mm * kf), a2 = cabs2(v[q]);
+    sum[E_K] += kk * kk * a2;
+    sl += kk * a2;
+  }
+  sum[E_L] = fixed * sl;
+  block_sums<W, kESums>(sum);
+  __shared__ double wm[W];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if ((threadIdx.x & 31) == 0) wm[threadIdx.x >> 5] = mx;
   __syncthreads();
-  {
-    double2* b = sm + w * LS;
-    const double2* tw = I.twM;
-    const int mode = (op == 5 || op == 4) ? 1 : ((op == 0 || op == 2) ? 0 : 2);
-    int a1 = 0, a2 = 0;
-    if (mode == 2) line_ab(w, a1, a2);
-    const bool valid = (op == 1) ? (a1 < Mh) : (a2 < Mh);
-    const double* kl = ks + w * KP;
-    line_xform<M, V>(b, tw, lane, mode, [&](int r, double2 x) {
-      if (!valid) return x;
-      return cscale(x, kl[(r <= M / 2) ? r : M - r]);
-    });
-  }
-  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < W; ++w) mx = fmax(mx, wm[w]);
 #pragma unroll
-  for (int q = 0; q < PER; ++q) {
-    const int e = tid + q * NT;
-    if (!(TOT % NT == 0 || e < TOT)) continue;
-    int r, c;
-    if (contig) s_map<M, LN, true>(e, r, c); else s_map<M, LN, false>(e, r, c);
-    const double2 v = sm[c * LS + swz(r)];
-    if (op == 0) {
-      const int line = t * LN + c;
-      if (r < Mh && line < ndim_lines(I)) I.cb1[(size_t)line * Mh + r] = v;
-    } else if (op == 5) {
-      const int line = t * LN + c, j = r - i0;
-      if (j >= 0 && j < N && line < ndim_lines(I)) I.phi_out[(size_t)line * N + j] = I.conv_scale * v.x;
-    } else if (op == 1) {
-      int kj, u;
-      line_ab(c, kj, u);
-      const int i = r - i0;
-      if (kj < Mh && i >= 0 && i < N) I.cb1[(size_t)i * Mh + kj] = v;
-    } else if (op == 2) {
-      int i, kk;
-      line_ab(c, i, kk);
-      if (kk < Mh) I.cb2[((size_t)i * M + r) * Mh + kk] = v;
-    } else if (op == 3) {
-      int jj, kk;
-      line_ab(c, jj, kk);
-      const int i = r - i0;
-      if (kk < Mh && i >= 0 && i < N) I.cb2[((size_t)i * M + jj) * Mh + kk] = v;
-    } else {  // op 4
-      int i, kk;
-      line_ab(c, i, kk);
-      const int j = r - i0;
-      if (kk < Mh && j >= 0 && j < N) I.cb1[((size_t)i * N + j) * Mh + kk] = v;
+    for (int q = 0; q < kESums; ++q) I.part[(size_t)q * gridDim.x + blockIdx.x] = sum[q];
+    I.part[(size_t)kESums * gridDim.x + blockIdx.x] = mx;
+  }
+}
+
+// Sum of |H - mu psi|^2: one partial per block at part[blockIdx.x] (mu on the device).
+constexpr int kResidThreads = 256;
+static __global__ void __launch_bounds__(kResidThreads)
+    k_stream_resid(const double2* __restrict__ psi, const double2* __restrict__ H, int n, const double* mu,
+                   double* part) {
+  const double m = *mu;
+  double g[1] = {0.0};
+  const int step = gridDim.x * kResidThreads;
+  for (int f0 = blockIdx.x * kResidThreads + threadIdx.x; f0 < n; f0 += 4 * step) {
+    double2 p[4], h[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int f = f0 + u * step;
+      p[u] = f < n ? __ldg(psi + f) : cmk(0.0, 0.0);
+      h[u] = f < n ? __ldg(H + f) : cmk(0.0, 0.0);
     }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) g[0] += cabs2(csub(h[u], cscale(p[u], m)));
+  }
+  block_sums<kResidThreads / 32, 1>(g);
+  if (threadIdx.x == 0) part[blockIdx.x] = g[0];
+}
+
+// Totals of lists of partials: block b adds cnt[b] values at part[b], thread by thread
+// in a fixed order (or takes their maximum), into out[b] (mapped host memory or device).
+struct SumArgs {
+  static constexpr int kMax = 24;
+  const double* part[kMax];
+  int cnt[kMax], is_max[kMax];
+  double scale[kMax];
+  double* out;
+};
+static __global__ void __launch_bounds__(256) k_stream_sum(const __grid_constant__ SumArgs A) {
+  const int b = blockIdx.x, n = A.cnt[b];
+  const double* p = A.part[b];
+  const bool is_max = A.is_max[b];
+  double s = 0.0;
+  for (int t = threadIdx.x; t < n; t += 256) s = is_max ? fmax(s, p[t]) : s + p[t];
+  __shared__ double red[8];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const double y = __shfl_xor_sync(0xffffffffu, s, o);
+    s = is_max ? fmax(s, y) : s + y;
+  }
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w) s = is_max ? fmax(s, red[w]) : s + red[w];
+    A.out[b] = s * A.scale[b];
   }
 }
 

@@ -104,9 +104,9 @@ class HamiltonianBatch:
         return outs
 
     def schedule(self, N):
-        """Pass schedule of grid size N: lines per tile and radix order of the H psi
+        """Pass schedule of grid size N: lines per tile and factorization of the H psi
         passes; lines per tile of the convolution's contiguous and strided passes
-        and its radix order; whether tuned; and the timed candidates as (lines,
+        and its factorization; whether tuned; and the timed candidates as (lines,
         order, strided lines, ms), lines < 0 for a convolution candidate (its
         contiguous width negated)."""
         ln, v, cl, csl, cv, tu, nc = (ctypes.c_int() for _ in range(7))

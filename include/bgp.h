@@ -152,18 +152,18 @@ int bgp_apply_H_batch(bgp_plan* plan, int n, const int* idx, const void* const* 
                       const double* const* phi, int phi_mode, double* mu_dev, void* stream);
 
 /* Pass schedule of the batched apply for line length N (autotuner of the
- * project, no counterpart in the reference): lines per tile (1, 2, 4, 8, 16) and the
- * line FFT's radix order (0: Stockham stages, largest radix first; 1: reversed;
- * 2: radix 4 first; 3: register-resident transform, N = 32 R: an R-point DFT per
- * lane and a 32-point transform across the lanes; 4-7: the same four at twice the
- * resident warps, with half the registers), and the convolution's lines
- * per tile of its contiguous passes (1, 2, 4, 8) and of its strided passes (1, 2,
- * 4, 8, 16; 16 where the tile fits in shared memory) and its radix order (0 or 3);
- * tuned = 0 not yet, 1 tuned, 2 fixed by bgp_plan_stream_set. cand (nullable)
- * receives up to *ncand (lines, order, strided lines, ms) quadruples of the
- * timed candidates (lines < 0: convolution candidates, whose -lines is the
- * contiguous width; strided lines 0 for the H psi candidates); *ncand is set
- * to their number. */
+ * project, no counterpart in the reference): lines per tile and the line
+ * transform's factorization of the H psi passes, and the convolution's lines per
+ * tile of its contiguous and of its strided passes and its factorization. Tiles
+ * of 2, 4 and 8 lines (strided convolution passes: 4 and 8) in two factorizations
+ * are compiled; the codes accepted are 1, 2, 4, 8 and 16 lines (contiguous
+ * convolution passes: up to 8) and orders 0 to 7 (convolution: 0 or 3), which run
+ * as the nearest compiled width and as factorization order mod 2 (convolution: 0
+ * the first, 3 the second). tuned = 0 not yet, 1 tuned, 2 fixed by
+ * bgp_plan_stream_set. cand (nullable) receives up to *ncand (lines, order,
+ * strided lines, ms) quadruples of the timed candidates (lines < 0: convolution
+ * candidates, whose -lines is the contiguous width; strided lines 0 for the H psi
+ * candidates); *ncand is set to their number. */
 int bgp_plan_stream_schedule(bgp_plan* plan, int N, int* lines, int* radix_order, int* conv_lines,
                              int* conv_strided_lines, int* conv_order, int* tuned, float* cand, int* ncand);
 /* Fix the schedule of line length N (lines = 0: tune again on the next call). */
