@@ -27,6 +27,7 @@ constexpr int kProfSlots = 20 * 5;   // phase profiler: 20 phase kinds x 5 count
 constexpr int kYieldDiv = 4;         // a solve launch yields once 1/kYieldDiv of it has finished
 constexpr int kTuneYield[3] = {2, 4, 8};  // relaunch schedules the autotuner tries
 constexpr int kMaxSegments = 256;    // relaunch limit of one solve
+constexpr int kResidBlocks = 592;    // blocks of the residual's sum: 4 per SM
 
 thread_local std::string g_err;
 int fail(int code, const std::string& msg) {
@@ -106,11 +107,6 @@ __global__ void __launch_bounds__(kThreads) k_cube_fft(Inst I, int ax, double2* 
     if (ax == I.ndim - 1) tile_run<L, true>(op, dyn_sm, t);
     else tile_run<L, false>(op, dyn_sm, t);
   }
-}
-
-__global__ void k_scale_c(double2* a, long long n, double s) {
-  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x)
-    a[q] = cscale(a[q], s);
 }
 
 // ---------------------------------------------------------------- host state
@@ -222,6 +218,10 @@ struct bgp_plan {
   long long launches = 0;                  // kernel launches issued by this plan
   SolveOut* d_out = nullptr;
   double* d_res = nullptr;                // n_inst x (kNRec + 1)
+  double* d_part = nullptr;               // partial sums of the operators' stream passes
+  size_t part_energy = 0, part_conv = 0;  // its sections: energy sums; one convolution's sums
+  double* h_sums = nullptr;               // totals on the host (mapped: the device writes them)
+  double* d_sums = nullptr;               // the same memory as the device sees it
   int max_team = 0;
   int lmax = 0;
   size_t smem = 0;
@@ -595,6 +595,16 @@ int bgp_plan_create(const bgp_instance_desc* desc, int n_inst, bgp_plan** plan) 
   if ((rc = palloc_t(p, (size_t)1, &p->d_finished))) return bail(rc);
   if ((rc = palloc_t(p, (size_t)n_inst, &p->d_out))) return bail(rc);
   if ((rc = palloc_t(p, (size_t)n_inst * (kNRec + 1), &p->d_res))) return bail(rc);
+  // tiles of at least 4 lines in the energy passes, 2 in the convolution's last pass
+  for (const Inst& I : p->inst) {
+    const size_t lines = I.ndim == 2 ? (size_t)I.N : (size_t)I.N * I.N;
+    p->part_energy = std::max(p->part_energy, (kESums + 1) * I.ndim * (lines / 4));
+    p->part_conv = std::max(p->part_conv, std::max(lines / 2, (size_t)kResidBlocks));
+  }
+  if ((rc = palloc_t(p, p->part_energy + 2 * p->part_conv, &p->d_part))) return bail(rc);
+  if (cudaHostAlloc((void**)&p->h_sums, sizeof(double) * SumArgs::kMax, cudaHostAllocMapped) != cudaSuccess ||
+      cudaHostGetDevicePointer((void**)&p->d_sums, p->h_sums, 0) != cudaSuccess)
+    return bail(fail(BGP_ERR_OOM, "pinned host memory for the operators' sums"));
   for (int i = 0; i < n_inst; ++i) {
     p->inst[i].out = p->d_out + i;
     p->inst[i].res = p->d_res + (size_t)i * (kNRec + 1);
@@ -615,6 +625,7 @@ int bgp_plan_destroy(bgp_plan* p) {
   for (cudaEvent_t q : p->ovl_ev) cudaEventDestroy(q);
   for (cudaEvent_t q : p->side_ev) cudaEventDestroy(q);
   for (void* q : p->allocs) cudaFree(q);
+  if (p->h_sums) cudaFreeHost(p->h_sums);
   delete p;
   return BGP_OK;
 }
@@ -664,149 +675,6 @@ int run_api(bgp_plan* p, int i, Inst& I, cudaStream_t st, double* res_host) {
   return BGP_OK;
 }
 }  // namespace
-
-int bgp_apply_H(bgp_plan* p, int i, const void* psi, void* hpsi, const double* phi, int phi_mode,
-                double* mu_out, void* stream) {
-  int rc = check_inst(p, i);
-  if (rc) return rc;
-  if (!psi || !hpsi) return fail(BGP_ERR_ARG, "null field pointer");
-  if (phi_mode == 1 && !phi) return fail(BGP_ERR_ARG, "phi_mode 1 needs phi");
-  Inst I = p->inst[i];
-  I.prog = kProgApplyH;
-  I.in_psi = (const double2*)psi;
-  I.out_c = (double2*)hpsi;
-  I.in_phi = phi;
-  I.use_phi = (I.kind == kNone || I.M == 0) ? (phi_mode == 1 ? 1 : 0) : phi_mode;
-  double res[kNRec + 1] = {0};
-  CK(cudaMemsetAsync(p->d_res + (size_t)i * (kNRec + 1), 0, sizeof(double) * (kNRec + 1), (cudaStream_t)stream));
-  rc = run_api(p, i, I, (cudaStream_t)stream, res);
-  if (rc) return rc;
-  if (mu_out) *mu_out = res[0];
-  return BGP_OK;
-}
-
-int bgp_energy(bgp_plan* p, int i, const void* psi, double* phi_out, bgp_energy_terms* terms,
-               void* stream) {
-  int rc = check_inst(p, i);
-  if (rc) return rc;
-  if (!psi || !terms) return fail(BGP_ERR_ARG, "null pointer");
-  Inst I = p->inst[i];
-  I.prog = kProgEnergy;
-  I.in_psi = (const double2*)psi;
-  I.out_r = phi_out;
-  double res[kNRec + 1] = {0};
-  CK(cudaMemsetAsync(p->d_res + (size_t)i * (kNRec + 1), 0, sizeof(double) * (kNRec + 1), (cudaStream_t)stream));
-  rc = run_api(p, i, I, (cudaStream_t)stream, res);
-  if (rc) return rc;
-  double comp[8];
-  energy_assemble(I, res, 1.0, comp);
-  terms->E = comp[0]; terms->Ekin = comp[1]; terms->Etrap = comp[2]; terms->Econtact = comp[3];
-  terms->Ethree = comp[4]; terms->Erot = comp[5]; terms->Egrav = comp[6]; terms->Lz = comp[7];
-  terms->mass = res[S_N0] * I.dv;
-  terms->r2mean = res[S_R2] * I.dv;
-  terms->peak = res[kNSum];
-  terms->rperp2 = res[S_PERP] * I.dv;
-  terms->z2 = res[S_Z2] * I.dv;
-  return BGP_OK;
-}
-
-int bgp_energy_grad(bgp_plan* p, int i, const void* psi, bgp_energy_terms* terms, void* dE_dpsi,
-                    double* dparams, void* stream) {
-  int rc = check_inst(p, i);
-  if (rc) return rc;
-  if (!psi || !terms || !dparams) return fail(BGP_ERR_ARG, "null pointer");
-  cudaStream_t st = (cudaStream_t)stream;
-  const Inst base = p->inst[i];
-  const bool kern = base.kind != kNone && base.M > 0;
-  // energy terms and the raw sums; the potential goes to the plan's phi buffer 0
-  Inst I = base;
-  I.prog = kProgEnergy;
-  I.in_psi = (const double2*)psi;
-  I.out_r = nullptr;
-  double res[kNRec + 1] = {0};
-  CK(cudaMemsetAsync(p->d_res + (size_t)i * (kNRec + 1), 0, sizeof(double) * (kNRec + 1), st));
-  rc = run_api(p, i, I, st, res);
-  if (rc) return rc;
-  double comp[8];
-  energy_assemble(I, res, 1.0, comp);
-  terms->E = comp[0]; terms->Ekin = comp[1]; terms->Etrap = comp[2]; terms->Econtact = comp[3];
-  terms->Ethree = comp[4]; terms->Erot = comp[5]; terms->Egrav = comp[6]; terms->Lz = comp[7];
-  terms->mass = res[S_N0] * I.dv;
-  terms->r2mean = res[S_R2] * I.dv;
-  terms->peak = res[kNSum];
-  terms->rperp2 = res[S_PERP] * I.dv;
-  terms->z2 = res[S_Z2] * I.dv;
-  dparams[0] = 0.5 * res[S_2] * I.dv;                                  // dE/dbeta2
-  dparams[1] = res[S_3] * I.dv / 3.0;                                  // dE/dbeta3
-  dparams[2] = (kern && base.G_C != 0.0) ? comp[6] / base.G_C : 0.0;   // dE/dG_C
-  dparams[3] = -comp[7];                                               // dE/dOmega
-  dparams[4] = 0.0;                                                    // dE/dl_z
-  if (dE_dpsi) {
-    // dE/dpsi* = H psi dV, with the potential of this psi
-    Inst J = base;
-    J.prog = kProgApplyH;
-    J.in_psi = (const double2*)psi;
-    J.out_c = (double2*)dE_dpsi;
-    J.in_phi = base.phi2;
-    J.use_phi = kern ? 1 : 0;
-    CK(cudaMemsetAsync(p->d_res + (size_t)i * (kNRec + 1), 0, sizeof(double) * (kNRec + 1), st));
-    rc = run_api(p, i, J, st, res);
-    if (rc) return rc;
-    k_scale_c<<<296, 256, 0, st>>>((double2*)dE_dpsi, (long long)base.n, base.dv);
-    CK(cudaGetLastError());
-  }
-  if (kern && base.kind == kQ2d && base.Wq) {
-    // dK/dl_z = -(K + W)/l_z, so dE/dl_z = -(Egrav + E_W)/l_z with E_W the energy of
-    // the virial kernel's potential
-    Inst J = base;
-    J.prog = kProgConvW;
-    J.in_psi = (const double2*)psi;
-    CK(cudaMemsetAsync(p->d_res + (size_t)i * (kNRec + 1), 0, sizeof(double) * (kNRec + 1), st));
-    rc = run_api(p, i, J, st, res);
-    if (rc) return rc;
-    const double EW = 0.5 * res[0] * base.dv;
-    const double lz = p->desc[i].l_z;
-    dparams[4] = -(comp[6] + EW) / lz;
-  }
-  CK(cudaStreamSynchronize(st));
-  return BGP_OK;
-}
-
-int bgp_residual(bgp_plan* p, int i, const void* psi, double* out3, void* stream) {
-  int rc = check_inst(p, i);
-  if (rc) return rc;
-  if (!psi || !out3) return fail(BGP_ERR_ARG, "null pointer");
-  Inst I = p->inst[i];
-  I.prog = kProgResidual;
-  I.in_psi = (const double2*)psi;
-  I.use_phi = 2;
-  double res[kNRec + 1] = {0};
-  CK(cudaMemsetAsync(p->d_res + (size_t)i * (kNRec + 1), 0, sizeof(double) * (kNRec + 1), (cudaStream_t)stream));
-  rc = run_api(p, i, I, (cudaStream_t)stream, res);
-  if (rc) return rc;
-  const double mu = res[0];
-  const double r = sqrt(res[1] * I.dv);
-  out3[0] = r;
-  out3[1] = mu;
-  out3[2] = r / fmax(1.0, fabs(mu));
-  return BGP_OK;
-}
-
-int bgp_convolve(bgp_plan* p, int i, const double* rho, double* out, int which, void* stream) {
-  int rc = check_inst(p, i);
-  if (rc) return rc;
-  Inst I = p->inst[i];
-  if (I.M == 0) return fail(BGP_ERR_ARG, "instance has no long-range kernel");
-  if (which == 1 && !I.Wq) return fail(BGP_ERR_ARG, "virial kernel exists for q2d only");
-  if (!rho || !out) return fail(BGP_ERR_ARG, "null pointer");
-  I.prog = kProgConv;
-  I.in_phi = rho;
-  I.out_r = out;
-  I.which_w = which;
-  double res[kNRec + 1] = {0};
-  CK(cudaMemsetAsync(p->d_res + (size_t)i * (kNRec + 1), 0, sizeof(double) * (kNRec + 1), (cudaStream_t)stream));
-  return run_api(p, i, I, (cudaStream_t)stream, res);
-}
 
 int bgp_precondition(bgp_plan* p, int i, const void* grad, const void* psi, const double* phi,
                      double shift_min, void* z, double* sigma_out, void* stream) {
@@ -860,6 +728,15 @@ const SKernel* stream_pad_kernel(int M, int C, int V, int mode, bool batch) {
   }
 }
 
+const SKernel* stream_energy_kernel(int N, int C, int V) {
+  switch (N) {
+#define X(n) case n: return bgp_septr_##n(C, V, 0, 0);
+    BGP_FOR_STREAM_N(X)
+#undef X
+    default: return nullptr;
+  }
+}
+
 // A pass schedule in compiled terms: tile widths and factorization variants.
 struct Sched {
   int c, v;          // H psi passes
@@ -871,6 +748,19 @@ struct Sched {
 Sched sched_of(const bgp_plan::StreamSched& sc) {
   auto w = [](int ln, int lo) { return ln < lo ? lo : (ln > 8 ? 8 : ln); };
   return Sched{w(sc.ln, 2), sc.v & 1, w(sc.cln, 2), w(sc.csln, 4), sc.cv ? 1 : 0};
+}
+
+// The schedule of the single-instance operators, by size. A grid of half a million
+// points or more fills the GPU with 8-line tiles (128-byte rows) and takes the
+// factorization with the fewest exchanges; a smaller one is a few microseconds of
+// latency: narrower tiles spread it over more SMs, and lengths 2^a take the
+// factorization with more threads per line. The autotuner picks the same on 128^3
+// (8 lines; 4 lines 3 % slower) and 256^2 (H psi 4 or 8 lines within 2 %; the quasi-2D
+// convolution 2 and 4 lines 17.5 us, 8 and 8 lines 19 us).
+Sched sched_rule(const Inst& I) {
+  if (I.n >= (1 << 19)) return Sched{8, 0, 8, 8, 0};
+  const int v = (I.N & (I.N - 1)) == 0;
+  return Sched{4, v, 2, 4, v};
 }
 
 // per-instance total of the tiles' partial sums, in tile order: mu = sum dV
@@ -896,7 +786,7 @@ __global__ void k_stream_mu(const __grid_constant__ SLaunchT<NB> SL, int tiles, 
 // One pass; chained: it may start while the launch before it on the stream still runs
 // (the pass itself waits, griddepcontrol, before it reads what that one writes).
 template <int NB>
-int stream_launch(const SKernel* kern, int tiles, SLaunchT<NB>& SL, cudaStream_t st, bool chained) {
+int stream_launch(const SKernel* kern, int tiles, SLaunchT<NB>& SL, cudaStream_t st, bool chained, int axes = 1) {
   if (!kern) return fail(BGP_ERR_UNSUPPORTED, "stream pass not compiled for this size / schedule");
   SL.tiles = tiles;
   if (kern->smem > 48 * 1024)
@@ -905,7 +795,7 @@ int stream_launch(const SKernel* kern, int tiles, SLaunchT<NB>& SL, cudaStream_t
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(tiles * SL.ninst);
+  cfg.gridDim = dim3(tiles * SL.ninst * axes);
   cfg.blockDim = dim3(kern->threads);
   cfg.dynamicSmemBytes = kern->smem;
   cfg.stream = st;
@@ -1054,7 +944,264 @@ void stream_inst(const bgp_plan* p, const Inst& I, SInst& S) {
 }
 }  // namespace
 
+namespace {
+// ---------------------------------------------- single-instance operators
+bool has_kernel(const Inst& I) { return I.kind != kNone && I.M > 0; }
+
+// One instance's launch block for the operators: psi as the state (and the density of
+// a convolution).
+void op_init(const bgp_plan* p, const Inst& I, const void* psi, SLaunchT<1>& SL) {
+  SL.ninst = 1;
+  stream_inst(p, I, SL.insts[0]);
+  SL.insts[0].psi = (const double2*)psi;
+}
+
+// The same for the plain convolution out = dV (K * rho) of a given density.
+void op_density(const bgp_plan* p, const Inst& I, const double* rho, double* out, int which_w, SLaunchT<1>& SL) {
+  op_init(p, I, nullptr, SL);
+  SInst& S = SL.insts[0];
+  const double Md = (double)I.M;
+  S.rho = rho;
+  S.phi_out = out;
+  S.Kq = which_w ? I.Wq : I.Kq;
+  S.conv_scale = I.dv / (I.ndim == 2 ? Md * Md : Md * Md * Md);
+}
+
+// the list of totals one k_stream_sum launch forms
+struct Sums {
+  SumArgs A{};
+  int n = 0;
+  int add(const double* part, int cnt, double scale = 1.0, bool is_max = false) {
+    A.part[n] = part; A.cnt[n] = cnt; A.scale[n] = scale; A.is_max[n] = is_max;
+    return n++;
+  }
+  // totals on the host once the stream's work is done
+  int run(bgp_plan* p, cudaStream_t st) {
+    if (n) {
+      A.out = p->d_sums;
+      k_stream_sum<<<n, 256, 0, st>>>(A);
+      CK(cudaGetLastError());
+      p->launches++;
+    }
+    CK(cudaStreamSynchronize(st));
+    return BGP_OK;
+  }
+};
+
+// potential of the instance's state by the table Kq, and its sum against the density
+// into the gpart section `sec`
+int op_conv(bgp_plan* p, SLaunchT<1>& SL, const Sched& S, int sec, Sums* sums, int* slot, cudaStream_t st) {
+  SInst& I = SL.insts[0];
+  I.gpart = sums ? p->d_part + p->part_energy + sec * p->part_conv : nullptr;
+  int rc = stream_conv(SL, S, st);
+  if (rc) return rc;
+  p->launches += I.ndim == 2 ? 3 : 5;
+  if (sums) *slot = sums->add(I.gpart, (I.ndim == 2 ? I.N : I.N * I.N) / S.cr);
+  return BGP_OK;
+}
+
+// H psi of the launch block (SL.insts[0].H, phi, part set)
+int op_hpsi(bgp_plan* p, SLaunchT<1>& SL, const Sched& S, cudaStream_t st) {
+  int rc = stream_run(SL, S, false, nullptr, 0, st);
+  p->launches += SL.insts[0].ndim;
+  return rc;
+}
+
+// the energy sums: total q of slot0 + q (kESums sums of every axis slot, then the peak)
+struct EnergySlots { int first[3][kESums], peak; };
+int op_energy(bgp_plan* p, SLaunchT<1>& SL, const Sched& S, Sums& sums, EnergySlots& es, cudaStream_t st) {
+  SInst& I = SL.insts[0];
+  const int C = S.c, tiles = I.n / (I.N * C), grid = tiles * I.ndim;
+  double* keep = I.part;
+  I.part = p->d_part;
+  int rc = stream_launch(stream_energy_kernel(I.N, C, S.v), tiles, SL, st, false, I.ndim);
+  I.part = keep;
+  if (rc) return rc;
+  p->launches++;
+  for (int a = 0; a < I.ndim; ++a)
+    for (int q = 0; q < kESums; ++q) {
+      const bool spectral = q == E_K || q == E_L;
+      es.first[a][q] = (a == 0 || spectral) ? sums.add(p->d_part + (size_t)q * grid + (size_t)a * tiles, tiles) : -1;
+    }
+  es.peak = sums.add(p->d_part + (size_t)kESums * grid, grid, 1.0, true);
+  return BGP_OK;
+}
+
+// the record of energy_assemble from the totals
+void op_energy_record(const bgp_plan* p, const Inst& I, const EnergySlots& es, double grav, double* rec) {
+  const double* h = p->h_sums;
+  for (int q = 0; q <= kNSum; ++q) rec[q] = 0.0;
+  auto at = [&](int a, int q) { return h[es.first[a][q]]; };
+  rec[S_N0] = at(0, E_N0); rec[S_V] = at(0, E_V); rec[S_2] = at(0, E_2); rec[S_3] = at(0, E_3);
+  rec[S_R2] = at(0, E_R2); rec[S_PERP] = at(0, E_PERP); rec[S_Z2] = at(0, E_Z2);
+  rec[S_KX] = at(1, E_K); rec[S_LX] = at(1, E_L);
+  const int y = I.ndim == 2 ? 0 : 2;            // axis slot of the y lines
+  rec[S_KY] = at(y, E_K); rec[S_LY] = at(y, E_L);
+  if (I.ndim == 3) rec[S_KZ] = at(0, E_K);
+  rec[S_G] = grav;
+  rec[kNSum] = h[es.peak];
+}
+
+void op_terms(const Inst& I, const double* res, bgp_energy_terms* terms) {
+  double comp[8];
+  energy_assemble(I, res, 1.0, comp);
+  terms->E = comp[0]; terms->Ekin = comp[1]; terms->Etrap = comp[2]; terms->Econtact = comp[3];
+  terms->Ethree = comp[4]; terms->Erot = comp[5]; terms->Egrav = comp[6]; terms->Lz = comp[7];
+  terms->mass = res[S_N0] * I.dv;
+  terms->r2mean = res[S_R2] * I.dv;
+  terms->peak = res[kNSum];
+  terms->rperp2 = res[S_PERP] * I.dv;
+  terms->z2 = res[S_Z2] * I.dv;
+}
+}  // namespace
+
 extern "C" {
+
+int bgp_apply_H(bgp_plan* p, int i, const void* psi, void* hpsi, const double* phi, int phi_mode,
+                double* mu_out, void* stream) {
+  int rc = check_inst(p, i);
+  if (rc) return rc;
+  if (!psi || !hpsi) return fail(BGP_ERR_ARG, "null field pointer");
+  if (phi_mode == 1 && !phi) return fail(BGP_ERR_ARG, "phi_mode 1 needs phi");
+  const Inst& I = p->inst[i];
+  cudaStream_t st = (cudaStream_t)stream;
+  const Sched S = sched_rule(I);
+  SLaunchT<1> SL{};
+  op_init(p, I, psi, SL);
+  if (phi_mode == 2 && has_kernel(I)) {
+    if ((rc = op_conv(p, SL, S, 0, nullptr, nullptr, st))) return rc;
+    SL.insts[0].phi = I.phi2;
+  } else {
+    SL.insts[0].phi = phi_mode == 1 ? phi : nullptr;
+  }
+  SL.insts[0].H = (double2*)hpsi;
+  if ((rc = op_hpsi(p, SL, S, st))) return rc;
+  Sums sums;
+  const int mu = sums.add(I.part, I.n / (I.N * S.c), I.dv);
+  if ((rc = sums.run(p, st))) return rc;
+  if (mu_out) *mu_out = p->h_sums[mu];
+  return BGP_OK;
+}
+
+int bgp_energy(bgp_plan* p, int i, const void* psi, double* phi_out, bgp_energy_terms* terms,
+               void* stream) {
+  int rc = check_inst(p, i);
+  if (rc) return rc;
+  if (!psi || !terms) return fail(BGP_ERR_ARG, "null pointer");
+  const Inst& I = p->inst[i];
+  cudaStream_t st = (cudaStream_t)stream;
+  const Sched S = sched_rule(I);
+  SLaunchT<1> SL{};
+  op_init(p, I, psi, SL);
+  Sums sums;
+  EnergySlots es;
+  int grav = -1;
+  if ((rc = op_energy(p, SL, S, sums, es, st))) return rc;
+  if (has_kernel(I)) {
+    if (phi_out) SL.insts[0].phi_out = phi_out;
+    if ((rc = op_conv(p, SL, S, 0, &sums, &grav, st))) return rc;
+  }
+  if ((rc = sums.run(p, st))) return rc;
+  double res[kNRec];
+  op_energy_record(p, I, es, grav >= 0 ? p->h_sums[grav] : 0.0, res);
+  op_terms(I, res, terms);
+  return BGP_OK;
+}
+
+int bgp_energy_grad(bgp_plan* p, int i, const void* psi, bgp_energy_terms* terms, void* dE_dpsi,
+                    double* dparams, void* stream) {
+  int rc = check_inst(p, i);
+  if (rc) return rc;
+  if (!psi || !terms || !dparams) return fail(BGP_ERR_ARG, "null pointer");
+  cudaStream_t st = (cudaStream_t)stream;
+  const Inst& I = p->inst[i];
+  const Sched S = sched_rule(I);
+  const bool kern = has_kernel(I), width = kern && I.kind == kQ2d && I.Wq;
+  SLaunchT<1> SL{};
+  op_init(p, I, psi, SL);
+  Sums sums;
+  EnergySlots es;
+  int grav = -1, gravW = -1;
+  if ((rc = op_energy(p, SL, S, sums, es, st))) return rc;
+  if (width) {
+    // dK/dl_z = -(K + W)/l_z, so dE/dl_z = -(Egrav + E_W)/l_z with E_W the energy of
+    // the virial kernel's potential, of which only the sum is wanted
+    SInst& Q = SL.insts[0];
+    Q.Kq = I.Wq;
+    Q.phi_out = nullptr;
+    if ((rc = op_conv(p, SL, S, 1, &sums, &gravW, st))) return rc;
+    Q.Kq = I.Kq;
+    Q.phi_out = I.phi2;
+  }
+  if (kern && (rc = op_conv(p, SL, S, 0, &sums, &grav, st))) return rc;
+  if (dE_dpsi) {
+    // dE/dpsi* = H psi dV, with the potential of this psi
+    SInst& Q = SL.insts[0];
+    Q.phi = kern ? I.phi2 : nullptr;
+    Q.H = (double2*)dE_dpsi;
+    Q.hscale = I.dv;
+    Q.part = nullptr;
+    if ((rc = op_hpsi(p, SL, S, st))) return rc;
+  }
+  if ((rc = sums.run(p, st))) return rc;
+  double res[kNRec];
+  op_energy_record(p, I, es, grav >= 0 ? p->h_sums[grav] : 0.0, res);
+  op_terms(I, res, terms);
+  dparams[0] = 0.5 * res[S_2] * I.dv;                                       // dE/dbeta2
+  dparams[1] = res[S_3] * I.dv / 3.0;                                       // dE/dbeta3
+  dparams[2] = (kern && I.G_C != 0.0) ? terms->Egrav / I.G_C : 0.0;         // dE/dG_C
+  dparams[3] = -terms->Lz;                                                  // dE/dOmega
+  dparams[4] = 0.0;                                                         // dE/dl_z
+  if (width) dparams[4] = -(terms->Egrav + 0.5 * p->h_sums[gravW] * I.dv) / p->desc[i].l_z;
+  return BGP_OK;
+}
+
+int bgp_residual(bgp_plan* p, int i, const void* psi, double* out3, void* stream) {
+  int rc = check_inst(p, i);
+  if (rc) return rc;
+  if (!psi || !out3) return fail(BGP_ERR_ARG, "null pointer");
+  const Inst& I = p->inst[i];
+  cudaStream_t st = (cudaStream_t)stream;
+  const Sched S = sched_rule(I);
+  SLaunchT<1> SL{};
+  op_init(p, I, psi, SL);
+  if (has_kernel(I)) {
+    if ((rc = op_conv(p, SL, S, 0, nullptr, nullptr, st))) return rc;
+    SL.insts[0].phi = I.phi2;
+  }
+  double2* H = I.pool + I.n;                     // pool field 1 (field 0 is the accumulator)
+  SL.insts[0].H = H;
+  if ((rc = op_hpsi(p, SL, S, st))) return rc;
+  double* mu = p->d_res + (size_t)i * (kNRec + 1);
+  k_stream_mu<1><<<1, 256, 0, st>>>(SL, I.n / (I.N * S.c), mu, 0);
+  const int blocks = std::min(kResidBlocks, (I.n + kResidThreads - 1) / kResidThreads);
+  k_stream_resid<<<blocks, kResidThreads, 0, st>>>((const double2*)psi, H, I.n, mu, p->d_part);
+  CK(cudaGetLastError());
+  p->launches += 2;
+  Sums sums;
+  const int s_mu = sums.add(mu, 1), s_r = sums.add(p->d_part, blocks);
+  if ((rc = sums.run(p, st))) return rc;
+  const double m = p->h_sums[s_mu], r = sqrt(p->h_sums[s_r] * I.dv);
+  out3[0] = r;
+  out3[1] = m;
+  out3[2] = r / fmax(1.0, fabs(m));
+  return BGP_OK;
+}
+
+int bgp_convolve(bgp_plan* p, int i, const double* rho, double* out, int which, void* stream) {
+  int rc = check_inst(p, i);
+  if (rc) return rc;
+  const Inst& I = p->inst[i];
+  if (I.M == 0) return fail(BGP_ERR_ARG, "instance has no long-range kernel");
+  if (which == 1 && !I.Wq) return fail(BGP_ERR_ARG, "virial kernel exists for q2d only");
+  if (!rho || !out) return fail(BGP_ERR_ARG, "null pointer");
+  cudaStream_t st = (cudaStream_t)stream;
+  SLaunchT<1> SL{};
+  op_density(p, I, rho, out, which, SL);
+  if ((rc = op_conv(p, SL, sched_rule(I), 0, nullptr, nullptr, st))) return rc;
+  CK(cudaStreamSynchronize(st));
+  return BGP_OK;
+}
 
 // H psi of several instances of a plan, enqueued without host synchronisation
 int bgp_apply_H_batch(bgp_plan* p, int n, const int* idx, const void* const* psi, void* const* hpsi,
@@ -1276,14 +1423,9 @@ int bgp_tf_density(bgp_plan* p, int i, int nonlocal, double Omega, int iters, do
     void* sargs[] = {&A, &two_s2};
     if ((rc = tf_launch((void*)k_tf_seed, grid, sargs, p, I, st))) return rc;
     for (int it = 0; it < iters; ++it) {
-      Inst J = I;
-      J.prog = kProgConv;
-      J.in_phi = n_out;
-      J.out_r = conv;
-      J.which_w = 0;
-      double res[kNRec + 1] = {0};
-      CK(cudaMemsetAsync(p->d_res + (size_t)i * (kNRec + 1), 0, sizeof(double) * (kNRec + 1), st));
-      if ((rc = run_api(p, i, J, st, res))) return rc;
+      SLaunchT<1> SL{};
+      op_density(p, I, n_out, conv, 0, SL);
+      if ((rc = op_conv(p, SL, sched_rule(I), 0, nullptr, nullptr, st))) return rc;
       void* args[] = {&A};
       if ((rc = tf_launch((void*)k_tf_iter, grid, args, p, I, st))) return rc;
       if ((rc = read_state())) return rc;

@@ -33,12 +33,7 @@ enum Kind : int { kNone = 0, kNewton = 1, kLog = 2, kQ2d = 3 };
 
 enum Prog : int {
   kProgSolve = 0,
-  kProgApplyH = 1,   // out = H psi (phi from in_phi, or computed when use_phi == 2)
-  kProgEnergy = 2,   // energy sums of psi (no normalisation) + phi
-  kProgResidual = 3, // H psi, mu, ||H psi - mu psi||
   kProgPrecond = 4,  // z = P_T[(k^2/2 + sigma)^-1 grad], sigma
-  kProgConv = 5,     // out_phi = scale * (K * rho) on the zero-padded grid
-  kProgConvW = 6,    // sum of (potential of W * |psi|^2) |psi|^2 (q2d virial kernel W)
 };
 
 enum Stop : int { kStopMaxit = 0, kStopConverged = 1, kStopEnergy = 2, kStopStalled = 3,
@@ -99,12 +94,11 @@ struct Inst {
   int yield_at;                   // yield once this many instances of the launch finished
   int* finished;                  // instances of this launch that have finished
   // API operands
-  int prog, use_phi, which_w;
+  int prog, use_phi;
   const double2* in_psi;          // psi (API) / psi0 (solve)
   const double2* in_grad;         // precond input
   const double* in_phi;           // given potential
   double2* out_c;                 // complex output (H psi, z, final psi)
-  double* out_r;                  // real output (phi)
   SolverParams sp;
   SolveOut* out;
 };

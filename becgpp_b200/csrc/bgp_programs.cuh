@@ -95,7 +95,7 @@ __device__ __noinline__ bool phase_end(Ctx& C, Acc a) {
   return ok;
 }
 // slots used by each kind of phase
-constexpr int kRedH = 1, kRedG = 5, kRedZ = 2, kRedT = 13, kRedD = 15;
+constexpr int kRedH = 1, kRedG = 5, kRedZ = 2, kRedT = 10, kRedD = 15;
 
 // phase boundary without a reduction record: only the team barrier
 static __device__ __noinline__ bool phase_sync(Ctx& C) {
@@ -173,7 +173,7 @@ BGP_D void tsum_add(Ctl& S, const double* tot) {
 // --------------------------------------------------------------- energy phases
 // mode: 0 trial (w = psi - t dirc; Q.psi, Q.t and the direction terms set by the
 //         caller), 1 initial state (w = Q.cin, copied to Q.W),
-//       2 API energy (w = Q.cin, nothing written).
+//       2 energy of a given state (w = Q.cin, nothing written).
 // Sums of w over every axis and, with a kernel, the convolution of |w|^2 (to
 // phi_out, unscaled by c) with its sum  sum phi_w |w|^2. Totals in S.tsum.
 template <int N, int M>
@@ -1007,76 +1007,19 @@ fail:
   }
 }
 
-// ------------------------------------------------------------- API programs
+// ---------------------------------------------------- preconditioner program
 template <int N, int M>
-BGP_D void prog_api(Ctx& C, Ctl& S) {
+BGP_D void prog_precond(Ctx& C, Ctl& S) {
   const Inst& I = C.I;
   PassArgs& Q = C.Q;
   const int tid = threadIdx.x;
-  const bool kern = (I.kind != kNone) && (M > 0);
   double* res = I.res;
   if (tid == 0) {
     Q.psi = I.in_psi; Q.psc = 1.0; Q.cin = I.in_psi;
     Q.cz = Q.cd = Q.cg = 0.0; Q.use_psi = 0; Q.t = 0.0; Q.fp32 = 0;
   }
   __syncthreads();
-  if (I.prog == kProgEnergy) {
-    double* phi_out = I.out_r ? I.out_r : phi_buf(I, 0);
-    if (!energy_phases<N, M>(C, S, 2, 0, nullptr, nullptr, phi_out)) goto fail;
-    if (C.T.rank == 0 && tid < kNRec) res[tid] = S.tsum[tid];
-    return;
-  }
-  if (I.prog == kProgConv) {
-    if (tid == 0) {
-      Q.rmode = 2; Q.rin = I.in_phi;
-      Q.Kq = I.which_w ? I.Wq : I.Kq;
-      const double Md = (M > 0) ? (double)M : 1.0;
-      Q.cscale = I.dv / ((BGP_DIM(I) == 2) ? Md * Md : Md * Md * Md);
-      Q.cout = I.out_r;
-    }
-    __syncthreads();
-    if (!conv_phases<N, M>(C)) goto fail;
-    return;
-  }
-  if (I.prog == kProgConvW) {
-    // potential of the virial kernel, -G_C dV (W * rho), and its sum against rho
-    if (tid == 0) {
-      Q.rmode = 0; Q.smode = 0;
-      Q.Kq = I.Wq; Q.cscale = I.conv_scale; Q.cout = phi_buf(I, 1);
-    }
-    __syncthreads();
-    if (!conv_phases<N, M>(C, 1)) goto fail;
-    if (C.T.rank == 0 && tid == 0) res[0] = C.tot[S_G];
-    return;
-  }
-  if (I.prog == kProgApplyH || I.prog == kProgResidual) {
-    const double* phi = nullptr;
-    if (kern && I.use_phi == 2) {
-      if (tid == 0) {
-        Q.rmode = 0; Q.Kq = I.Kq; Q.cscale = I.conv_scale; Q.cout = phi_buf(I, 0);
-      }
-      __syncthreads();
-      if (!conv_phases<N, M>(C)) goto fail;
-      phi = phi_buf(I, 0);
-    } else if (I.use_phi == 1) {
-      phi = I.in_phi;
-    }
-    double2* H = (I.prog == kProgApplyH) ? I.out_c : pool_buf(I, 1);
-    if (tid == 0) { Q.A = pool_buf(I, 0); Q.H = H; Q.phi = phi; Q.phisc = 1.0; }
-    __syncthreads();
-    if (!hpsi_phases<N>(C)) goto fail;
-    const double mu = C.tot[0] * I.dv;
-    if (I.prog == kProgApplyH) {
-      if (C.T.rank == 0 && tid == 0) { res[0] = mu; res[1] = C.tot[kNSum]; }
-      return;
-    }
-    if (tid == 0) { Q.mu = mu; Q.gin = nullptr; Q.Gout = nullptr; Q.A = pool_buf(I, 2); Q.keys_on = 0; Q.win_on = 0; }
-    __syncthreads();
-    if (!grad_phase<N>(C, 0.0)) goto fail;
-    if (C.T.rank == 0 && tid == 0) { res[0] = mu; res[1] = C.tot[0]; }
-    return;
-  }
-  if (I.prog == kProgPrecond) {
+  {
     const double* phi = (I.use_phi == 1) ? I.in_phi : nullptr;
     // max rho of psi (rank 0 also clears the histograms)
     {
