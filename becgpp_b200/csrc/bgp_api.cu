@@ -1391,6 +1391,9 @@ int bgp_tf_density(bgp_plan* p, int i, int nonlocal, double Omega, int iters, do
   int nb = 0;
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_tf_iter, kThreads, 0));
   int grid = std::min(nb * p->dev->sms, p->grid_cap);
+  // no more CTAs than kTfHold points a thread keep busy: a barrier's arrivals queue on one
+  // address (256^2, 25 steps: 5.8 ms with 4 points a thread, 6.3 with 2, 8.0 with 1)
+  grid = std::min(grid, std::max(1, (I.n + kTfHold * kThreads - 1) / (kTfHold * kThreads)));
   if (grid < 1) return fail(BGP_ERR_CUDA, "Thomas-Fermi kernel does not fit on an SM");
   double* state = p->d_res + (size_t)i * (kNRec + 1);
   double* conv = I.phi2 + I.n;   // the plan's second potential field as the convolution output
