@@ -71,6 +71,7 @@ _SIGS = {
     "bgp_apply_H": ([_P, ctypes.c_int, _P, _P, _P, ctypes.c_int, ctypes.POINTER(ctypes.c_double), _P],
                     ctypes.c_int),
     "bgp_energy": ([_P, ctypes.c_int, _P, _P, ctypes.POINTER(EnergyTerms), _P], ctypes.c_int),
+    "bgp_energy_observables": ([_P, ctypes.c_int, _P, ctypes.POINTER(EnergyTerms), _P], ctypes.c_int),
     "bgp_residual": ([_P, ctypes.c_int, _P, ctypes.POINTER(ctypes.c_double), _P], ctypes.c_int),
     "bgp_energy_grad": ([_P, ctypes.c_int, _P, ctypes.POINTER(EnergyTerms), _P,
                          ctypes.POINTER(ctypes.c_double), _P], ctypes.c_int),
@@ -80,8 +81,8 @@ _SIGS = {
     "bgp_solve": ([_P, ctypes.POINTER(_P), ctypes.POINTER(_P), ctypes.POINTER(SolverParams),
                    ctypes.POINTER(SolveResult), ctypes.POINTER(ctypes.c_double), _P], ctypes.c_int),
     "bgp_apply_H_noalloc": ([ctypes.POINTER(InstanceDesc), _P, _P, _P, _P], ctypes.c_int),
-    "bgp_apply_H_batch": ([_P, ctypes.c_int, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(_P), ctypes.POINTER(_P),
-                           ctypes.POINTER(_P), ctypes.c_int, _P, _P], ctypes.c_int),
+    # (arrays of pointers and indices as plain addresses: ctypes arrays, byref() or integers)
+    "bgp_apply_H_batch": ([_P, ctypes.c_int, _P, _P, _P, _P, ctypes.c_int, _P, _P], ctypes.c_int),
     "bgp_plan_stream_schedule": ([_P, ctypes.c_int, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int),
                                   ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int),
                                   ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int),
@@ -149,8 +150,22 @@ def require_cuda():
                            "no CPU fallback")
 
 
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def stream_ptr():
+    if _raw_stream is not None:          # (building the Stream object takes several us)
+        return ctypes.c_void_p(_raw_stream(torch.cuda.current_device()))
     return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+
+def dev_c128(p):
+    """p as a contiguous complex128 tensor on the current CUDA device (p itself when it
+    is one already)."""
+    if p.dtype is torch.complex128 and p.is_cuda and p.is_contiguous() and p.get_device() == torch.cuda.current_device():
+        return p
+    require_cuda()
+    return p.to(device="cuda", dtype=torch.complex128).contiguous()
 
 
 def ptr(t):

@@ -40,7 +40,7 @@ def energy_and_grad(psi, G, beta2, beta3, G_C, Omega, l_z=None, want_psi_grad=Tr
     """E, its terms, dE/dpsi* (= H psi dV, or None) and dE/d(beta2, beta3, G_C,
     Omega, l_z) at psi (as given, not normalised)."""
     _lib.require_cuda()
-    psi = psi.to(device="cuda", dtype=torch.complex128).contiguous()
+    psi = _lib.dev_c128(psi)
     Gx, phys = _phys_grid(G, beta2, beta3, G_C, Omega, l_z)
     plan = plan_for(Gx, phys)
     terms = _lib.EnergyTerms()
@@ -76,10 +76,12 @@ class EnergyFunction(torch.autograd.Function):
         (dpsi,) = ctx.saved_tensors
         g_psi = (2.0 * gE) * dpsi if ctx.has_psi else None
         out = [g_psi]
+        # each parameter's gradient on its own device: gE is brought there once
+        on = {gE.device: gE}
         for name, dev in zip(PARAMS, ctx.devices):
-            v = ctx.dparams[name]
-            out.append(gE * torch.tensor(v, dtype=torch.float64, device=gE.device) if dev is not None
-                       else None)
+            if dev is not None and dev not in on:
+                on[dev] = gE.to(dev)
+            out.append(on[dev] * ctx.dparams[name] if dev is not None else None)
         out.append(None)  # G
         return tuple(out)
 

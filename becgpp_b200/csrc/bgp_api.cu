@@ -661,6 +661,18 @@ int bgp_prof_read(bgp_plan* p, int i, unsigned long long* out, int reset) {
 long long bgp_plan_launches(const bgp_plan* p) { return p ? p->launches : 0; }
 
 namespace {
+void op_terms(const Inst& I, const double* res, bgp_energy_terms* terms) {
+  double comp[8];
+  energy_assemble(I, res, 1.0, comp);
+  terms->E = comp[0]; terms->Ekin = comp[1]; terms->Etrap = comp[2]; terms->Econtact = comp[3];
+  terms->Ethree = comp[4]; terms->Erot = comp[5]; terms->Egrav = comp[6]; terms->Lz = comp[7];
+  terms->mass = res[S_N0] * I.dv;
+  terms->r2mean = res[S_R2] * I.dv;
+  terms->peak = res[kNSum];
+  terms->rperp2 = res[S_PERP] * I.dv;
+  terms->z2 = res[S_Z2] * I.dv;
+}
+
 int run_api(bgp_plan* p, int i, Inst& I, cudaStream_t st, double* res_host) {
   Inst save = p->inst[i];
   p->inst[i] = I;
@@ -675,6 +687,21 @@ int run_api(bgp_plan* p, int i, Inst& I, cudaStream_t st, double* res_host) {
   return BGP_OK;
 }
 }  // namespace
+
+int bgp_energy_observables(bgp_plan* p, int i, const void* psi, bgp_energy_terms* terms, void* stream) {
+  int rc = check_inst(p, i);
+  if (rc) return rc;
+  if (!psi || !terms) return fail(BGP_ERR_ARG, "null pointer");
+  Inst I = p->inst[i];
+  I.prog = kProgEnergy;
+  I.in_psi = (const double2*)psi;
+  double res[kNRec + 1] = {0};
+  CK(cudaMemsetAsync(p->d_res + (size_t)i * (kNRec + 1), 0, sizeof(double) * (kNRec + 1), (cudaStream_t)stream));
+  rc = run_api(p, i, I, (cudaStream_t)stream, res);
+  if (rc) return rc;
+  op_terms(I, res, terms);
+  return BGP_OK;
+}
 
 int bgp_precondition(bgp_plan* p, int i, const void* grad, const void* psi, const double* phi,
                      double shift_min, void* z, double* sigma_out, void* stream) {
@@ -736,6 +763,8 @@ const SKernel* stream_energy_kernel(int N, int C, int V) {
     default: return nullptr;
   }
 }
+
+bool has_kernel(const Inst& I) { return I.kind != kNone && I.M > 0; }
 
 // A pass schedule in compiled terms: tile widths and factorization variants.
 struct Sched {
@@ -926,6 +955,20 @@ int stream_autotune(bgp_plan::StreamSched& sc, SLaunchT<NB>& SL, bool conv, cuda
   return rc;
 }
 
+// the plan's side stream of size group g >= 1 (and its join event side_ev[g])
+int side_stream(bgp_plan* p, int g, cudaStream_t* out) {
+  while ((int)p->side_st.size() < g) {
+    cudaStream_t q;
+    CK(cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking));
+    p->side_st.push_back(q);
+    cudaEvent_t e;
+    CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    p->side_ev.push_back(e);
+  }
+  *out = p->side_st[g - 1];
+  return BGP_OK;
+}
+
 // stream descriptor of an instance (the caller sets psi, H and phi)
 void stream_inst(const bgp_plan* p, const Inst& I, SInst& S) {
   S.ndim = I.ndim; S.N = I.N; S.n = I.n; S.M = I.M; S.Mh = I.Mh; S.i0 = I.i0;
@@ -946,8 +989,6 @@ void stream_inst(const bgp_plan* p, const Inst& I, SInst& S) {
 
 namespace {
 // ---------------------------------------------- single-instance operators
-bool has_kernel(const Inst& I) { return I.kind != kNone && I.M > 0; }
-
 // One instance's launch block for the operators: psi as the state (and the density of
 // a convolution).
 void op_init(const bgp_plan* p, const Inst& I, const void* psi, SLaunchT<1>& SL) {
@@ -1042,17 +1083,6 @@ void op_energy_record(const bgp_plan* p, const Inst& I, const EnergySlots& es, d
   rec[kNSum] = h[es.peak];
 }
 
-void op_terms(const Inst& I, const double* res, bgp_energy_terms* terms) {
-  double comp[8];
-  energy_assemble(I, res, 1.0, comp);
-  terms->E = comp[0]; terms->Ekin = comp[1]; terms->Etrap = comp[2]; terms->Econtact = comp[3];
-  terms->Ethree = comp[4]; terms->Erot = comp[5]; terms->Egrav = comp[6]; terms->Lz = comp[7];
-  terms->mass = res[S_N0] * I.dv;
-  terms->r2mean = res[S_R2] * I.dv;
-  terms->peak = res[kNSum];
-  terms->rperp2 = res[S_PERP] * I.dv;
-  terms->z2 = res[S_Z2] * I.dv;
-}
 }  // namespace
 
 extern "C" {
@@ -1223,12 +1253,19 @@ int bgp_apply_H_batch(bgp_plan* p, int n, const int* idx, const void* const* psi
   // the first runs on the caller's stream, each further one on a side stream that
   // waits for the work enqueued before the call and that the caller's stream waits for
   std::vector<char> done(n, 0);
-  if (p->side_ev.empty()) {
-    cudaEvent_t e;
-    CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    p->side_ev.push_back(e);
+  bool forks = n > kStreamBatch;               // more than one group
+  for (int a = 1; a < n && !forks; ++a) {
+    const Inst &A = p->inst[idx[0]], &B = p->inst[idx[a]];
+    forks = A.ndim != B.ndim || A.N != B.N || (phi_mode == 2 && has_kernel(A) != has_kernel(B));
   }
-  CK(cudaEventRecord(p->side_ev[0], st));   // the fork: the work enqueued before this call
+  if (forks) {
+    if (p->side_ev.empty()) {
+      cudaEvent_t e;
+      CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+      p->side_ev.push_back(e);
+    }
+    CK(cudaEventRecord(p->side_ev[0], st));    // the fork: the work enqueued before this call
+  }
   int ngroup = 0;
   for (int a = 0; a < n; ++a) {
     if (done[a]) continue;
@@ -1246,15 +1283,8 @@ int bgp_apply_H_batch(bgp_plan* p, int n, const int* idx, const void* const* psi
     }
     cudaStream_t gs = st;
     if (gi > 0) {
-      while ((int)p->side_st.size() < gi) {
-        cudaStream_t q;
-        CK(cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking));
-        p->side_st.push_back(q);
-        cudaEvent_t e;
-        CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        p->side_ev.push_back(e);
-      }
-      gs = p->side_st[gi - 1];
+      int rc = side_stream(p, gi, &gs);
+      if (rc) return rc;
       CK(cudaStreamWaitEvent(gs, p->side_ev[0], 0));
     }
     cudaStream_t os = nullptr;

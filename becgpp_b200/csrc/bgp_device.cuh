@@ -33,6 +33,7 @@ enum Kind : int { kNone = 0, kNewton = 1, kLog = 2, kQ2d = 3 };
 
 enum Prog : int {
   kProgSolve = 0,
+  kProgEnergy = 2,   // energy sums of psi (no normalisation)
   kProgPrecond = 4,  // z = P_T[(k^2/2 + sigma)^-1 grad], sigma
 };
 

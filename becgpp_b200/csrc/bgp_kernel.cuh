@@ -10,12 +10,12 @@ BGP_NS_BEGIN
 template <int N, int M>
 __device__ void run_prog(Ctx& C, Ctl& S) {
 #if defined(BGP_ONLY_API)
-  prog_precond<N, M>(C, S);
+  prog_api<N, M>(C, S);
 #elif defined(BGP_ONLY_SOLVE)
   prog_solve<N, M>(C, S);
 #else
   if (C.I.prog == kProgSolve) prog_solve<N, M>(C, S);
-  else prog_precond<N, M>(C, S);
+  else prog_api<N, M>(C, S);
 #endif
 }
 

@@ -13,8 +13,7 @@
 
 BGP_NS_BEGIN
 
-// Reduction-record slots of the energy sums (trial / energy passes); the last three
-// belong to the observables of the energy entry points only
+// Reduction-record slots of the energy sums (trial / energy passes)
 enum : int { S_N0 = 0, S_V = 1, S_2 = 2, S_3 = 3, S_KX = 4, S_KY = 5, S_KZ = 6, S_LY = 7, S_LX = 8,
              S_G = 9, S_R2 = 10, S_PERP = 11, S_Z2 = 12 };
 
@@ -264,10 +263,20 @@ struct OpT {
     }
     if (write_w) stp(W, f, w, sp);
     const double q = cabs2(w);
+    const double x = xcoord(g, i), y = xcoord(g, j);
     acc.s[S_N0] += q;
     acc.s[S_V] += potential(g, i, j, k) * q;
     acc.s[S_2] += q * q;
     acc.s[S_3] += q * q * q;
+    const double rp = x * x + y * y;
+    double r2 = rp;
+    if (BGP_DIM(g) == 3) {
+      const double z = xcoord(g, k);
+      r2 = r2 + z * z;
+      acc.s[S_PERP] += rp * q;
+      acc.s[S_Z2] += z * z * q;
+    }
+    acc.s[S_R2] += r2 * q;
     acc.mx = fmax(acc.mx, q);
     return w;
   }

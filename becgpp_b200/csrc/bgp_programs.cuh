@@ -95,7 +95,7 @@ __device__ __noinline__ bool phase_end(Ctx& C, Acc a) {
   return ok;
 }
 // slots used by each kind of phase
-constexpr int kRedH = 1, kRedG = 5, kRedZ = 2, kRedT = 10, kRedD = 15;
+constexpr int kRedH = 1, kRedG = 5, kRedZ = 2, kRedT = 13, kRedD = 15;
 
 // phase boundary without a reduction record: only the team barrier
 static __device__ __noinline__ bool phase_sync(Ctx& C) {
@@ -1007,9 +1007,9 @@ fail:
   }
 }
 
-// ---------------------------------------------------- preconditioner program
+// ------------------------------------------------------------- API programs
 template <int N, int M>
-BGP_D void prog_precond(Ctx& C, Ctl& S) {
+BGP_D void prog_api(Ctx& C, Ctl& S) {
   const Inst& I = C.I;
   PassArgs& Q = C.Q;
   const int tid = threadIdx.x;
@@ -1019,7 +1019,12 @@ BGP_D void prog_precond(Ctx& C, Ctl& S) {
     Q.cz = Q.cd = Q.cg = 0.0; Q.use_psi = 0; Q.t = 0.0; Q.fp32 = 0;
   }
   __syncthreads();
-  {
+  if (I.prog == kProgEnergy) {
+    if (!energy_phases<N, M>(C, S, 2, 0, nullptr, nullptr, phi_buf(I, 0))) goto fail;
+    if (C.T.rank == 0 && tid < kNRec) res[tid] = S.tsum[tid];
+    return;
+  }
+  if (I.prog == kProgPrecond) {
     const double* phi = (I.use_phi == 1) ? I.in_phi : nullptr;
     // max rho of psi (rank 0 also clears the histograms)
     {

@@ -222,15 +222,22 @@ _PLANS = OrderedDict()
 _MAX_PLANS = 4
 
 
+def _plan_key(G, cfg):
+    """The values of instance_desc(G, cfg), in its field order."""
+    kind = G["kernel"]
+    return (int(G["ndim"]), int(G["N"]), int(G["pad"]), KERNEL_CODES[kind], float(G["L"]), float(G["s"]),
+            float(G.get("trap_coeff", 0.5)), float(cfg["beta2"]), float(cfg["beta3"]), float(cfg["Omega"]),
+            float(cfg["G_C"]) if kind != "none" else 0.0, float(G.get("l_z", 0.0)))
+
+
 def plan_for(G, cfg):
     """Cached single-instance plan for grid G with the physics of cfg."""
-    d = instance_desc(G, cfg)
-    key = desc_key(d)
+    key = _plan_key(G, cfg)
     p = _PLANS.get(key)
     if p is None:
         while len(_PLANS) >= _MAX_PLANS:
             _PLANS.popitem(last=False)[1].close()
-        p = Plan([d])
+        p = Plan([instance_desc(G, cfg)])
         _PLANS[key] = p
     else:
         _PLANS.move_to_end(key)

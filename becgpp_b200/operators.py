@@ -5,6 +5,7 @@ field operation runs in libbgp (FP64). Scalars come back as 0-dim float64
 tensors where the reference returns tensors, and as Python floats where it
 calls ``.item()``.
 """
+import array
 import ctypes
 import math
 
@@ -14,33 +15,28 @@ from . import _lib
 from .grid import dV, plan_for
 
 
-def _dev_c128(p):
-    _lib.require_cuda()
-    return p.to(device="cuda", dtype=torch.complex128).contiguous()
+_dev_c128 = _lib.dev_c128
+_INDEX0 = (ctypes.c_int * 1)(0)      # the only instance of a single-instance plan
 
 
 def _physics(beta2, beta3, Omega, G_C):
     return dict(beta2=float(beta2), beta3=float(beta3), Omega=float(Omega), G_C=float(G_C))
 
 
-def _energy_terms(p, G, phys, want_phi=True):
-    p = _dev_c128(p)
-    plan = plan_for(G, phys)
-    kern = G["kernel"] != "none" and abs(phys["G_C"]) > 1e-15
-    phi = torch.zeros(p.shape, dtype=torch.float64, device=p.device)
-    t = _lib.EnergyTerms()
-    _lib.check(_lib.lib().bgp_energy(plan.handle, 0, _lib.ptr(p), _lib.ptr(phi) if kern else None,
-                                     ctypes.byref(t), _lib.stream_ptr()), "bgp_energy")
-    return t, phi
-
-
 def energy_components(p, G, beta2, beta3, Omega, G_C):
     """E and its terms for state p as given (not normalised) and the long-range
     potential phi (becgpp/operators.py:10-29)."""
-    t, phi = _energy_terms(p, G, _physics(beta2, beta3, Omega, G_C))
-    f = lambda v: torch.tensor(v, dtype=torch.float64)
-    return dict(E=f(t.E), Ekin=f(t.Ekin), Etrap=f(t.Etrap), Econtact=f(t.Econtact),
-                Ethree=f(t.Ethree), Erot=f(t.Erot), Egrav=f(t.Egrav), Lz=f(t.Lz), phi=phi)
+    p = _dev_c128(p)
+    phys = _physics(beta2, beta3, Omega, G_C)
+    plan = plan_for(G, phys)
+    kern = G["kernel"] != "none" and abs(phys["G_C"]) > 1e-15
+    phi = (torch.empty if kern else torch.zeros)(p.shape, dtype=torch.float64, device=p.device)
+    t = _lib.EnergyTerms()
+    _lib.check(_lib.lib().bgp_energy(plan.handle, 0, _lib.ptr(p), _lib.ptr(phi) if kern else None,
+                                     ctypes.byref(t), _lib.stream_ptr()), "bgp_energy")
+    names = ("E", "Ekin", "Etrap", "Econtact", "Ethree", "Erot", "Egrav", "Lz")
+    vals = torch.tensor([getattr(t, k) for k in names], dtype=torch.float64).unbind(0)
+    return dict(zip(names, vals), phi=phi)
 
 
 def energy_t(p, G, beta2, beta3, Omega, G_C):
@@ -63,9 +59,9 @@ def apply_H(psi, G, cfg, phi=None):
     else:
         ph = None
         mode = 2 if kern else 0
-    P = ctypes.c_void_p * 1
-    _lib.check(_lib.lib().bgp_apply_H_batch(plan.handle, 1, (ctypes.c_int * 1)(0), P(psi.data_ptr()),
-                                            P(out.data_ptr()), P(ph.data_ptr()) if ph is not None else None,
+    P, ref = ctypes.c_void_p, ctypes.byref
+    _lib.check(_lib.lib().bgp_apply_H_batch(plan.handle, 1, _INDEX0, ref(P(psi.data_ptr())), ref(P(out.data_ptr())),
+                                            ref(P(ph.data_ptr())) if ph is not None else None,
                                             mode, None, _lib.stream_ptr()), "bgp_apply_H_batch")
     return out
 
@@ -85,22 +81,36 @@ class HamiltonianBatch:
         self.plan = Plan([instance_desc(G, c) for G, c in zip(self.grids, self.cfgs)])
         self.n = len(self.cfgs)
         self._idx = (ctypes.c_int * self.n)(*range(self.n))
+        self._shapes = [(int(G["N"]),) * int(G["ndim"]) for G in self.grids]
+        self._groups = {}                 # field shape -> instances
+        for i, s in enumerate(self._shapes):
+            self._groups.setdefault(s, []).append(i)
+
+    def _outputs(self, psis):
+        """One output per state: the fields of one shape are slices of one allocation."""
+        if any(tuple(p.shape) != s for p, s in zip(psis, self._shapes)):
+            return [torch.empty_like(p) for p in psis]
+        outs = [None] * self.n
+        for s, idx in self._groups.items():
+            block = torch.empty((len(idx),) + s, dtype=torch.complex128, device=psis[idx[0]].device)
+            for i, o in zip(idx, block.unbind(0)):
+                outs[i] = o
+        return outs
 
     def apply(self, psis, out=None, phis=None, mu=None):
         """out[i] = H psis[i]. phis: None (potential computed from |psi|^2 where
         the kernel is on) or a list of potentials; mu: optional device float64
         tensor of n entries receiving Re<psi, H psi> dV."""
         psis = [_dev_c128(p) for p in psis]
-        outs = out if out is not None else [torch.empty_like(p) for p in psis]
-        P = ctypes.c_void_p * self.n
-        ph = None
-        mode = 2
-        if phis is not None:
-            ph = P(*[q.data_ptr() for q in phis])
-            mode = 1
-        _lib.check(_lib.lib().bgp_apply_H_batch(self.plan.handle, self.n, self._idx,
-                                                P(*[p.data_ptr() for p in psis]), P(*[o.data_ptr() for o in outs]),
-                                                ph, mode, _lib.ptr(mu), _lib.stream_ptr()), "bgp_apply_H_batch")
+        outs = out if out is not None else self._outputs(psis)
+        address = lambda ts: array.array("Q", [t.data_ptr() for t in ts])
+        a_psi, a_out = address(psis), address(outs)
+        a_phi = address(phis) if phis is not None else None
+        _lib.check(_lib.lib().bgp_apply_H_batch(self.plan.handle, self.n, self._idx, a_psi.buffer_info()[0],
+                                                a_out.buffer_info()[0],
+                                                a_phi.buffer_info()[0] if a_phi is not None else None,
+                                                1 if a_phi is not None else 2, _lib.ptr(mu), _lib.stream_ptr()),
+                   "bgp_apply_H_batch")
         return outs
 
     def schedule(self, N):
@@ -147,10 +157,18 @@ def compute_residual(psi, G, cfg):
 def observables(p, G, cfg):
     """E, mu, L_z, rrms, peak, the virial identity and the energy terms
     (becgpp/operators.py:55-103)."""
+    return observables_in(plan_for(G, _physics(cfg["beta2"], cfg["beta3"], cfg["Omega"], cfg["G_C"])), 0, p, G, cfg)
+
+
+def observables_in(plan, inst, p, G, cfg):
+    """observables of a state by instance `inst` of a plan that holds its grid and physics
+    (a solved batch has one; a plan per instance costs more than the sums)."""
     from .interactions import kernel_convolution
     gc = float(cfg["G_C"])
-    phys = _physics(cfg["beta2"], cfg["beta3"], cfg["Omega"], gc)
-    t, _ = _energy_terms(p, G, phys)
+    p = _dev_c128(p)
+    t = _lib.EnergyTerms()
+    _lib.check(_lib.lib().bgp_energy_observables(plan.handle, int(inst), _lib.ptr(p), ctypes.byref(t),
+                                                 _lib.stream_ptr()), "bgp_energy_observables")
     d, s, dv = float(G["ndim"]), float(G["s"]), dV(G)
     mass = t.mass
     mu = t.E + t.Econtact + 2.0 * t.Ethree + t.Egrav

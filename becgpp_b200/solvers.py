@@ -16,7 +16,7 @@ import torch
 from . import _lib
 from ._lib import CG_BETA_CODES, STOP_NAMES, SolverParams, SolveResult
 from .grid import Plan, instance_desc, make_grid, plan_for
-from .operators import compute_residual, observables
+from .operators import observables_in
 from .seeds import make_seed
 
 SOLVER_KEYS = ("maxit", "res_tol", "energy_tol", "conv_window", "step", "step_max",
@@ -50,9 +50,7 @@ def solver_params(cfg, trace_cap=None):
     return p
 
 
-def _c128(p):
-    _lib.require_cuda()
-    return p.to(device="cuda", dtype=torch.complex128).contiguous()
+_c128 = _lib.dev_c128
 
 
 class BatchSolver:
@@ -111,19 +109,19 @@ class BatchSolver:
         results = []
         for i in range(self.n):
             results.append(_finish(outs[i], self.grids[i], self.cfgs[i], res[i], wall, tr, i,
-                                   self.params))
+                                   self.params, self.plan))
         return results
 
     def close(self):
         self.plan.close()
 
 
-def _finish(psi, G, cfg, r, wall, tr, i, params):
+def _finish(psi, G, cfg, r, wall, tr, i, params, plan):
     if r.status != 0:
         raise RuntimeError("device solver reported an error")
     resid_abs, resid_rel = float(r.resid_abs_final), float(r.resid_rel_final)
     converged = bool(r.converged or resid_rel < float(cfg["res_tol"]))
-    obs = observables(psi, G, cfg)
+    obs = observables_in(plan, i, psi, G, cfg)
     obs.update(iters=int(r.iters), walltime=wall, resid_abs=resid_abs, resid_rel=resid_rel,
                min_resid=float(r.min_resid), converged=converged,
                stop_reason=STOP_NAMES[int(r.stop_reason)], preconditioner_shift=float(r.sigma),
@@ -154,7 +152,7 @@ def ground_state(cfg, G=None, psi0=None, verbose=True):
     _lib.check(_lib.lib().bgp_solve(plan.handle, P(psi.data_ptr()), P(out.data_ptr()),
                                     ctypes.byref(params), res, tr, _lib.stream_ptr()), "bgp_solve")
     wall = time.time() - t0
-    psi, G, obs = _finish(out, G, cfg, res[0], wall, tr, 0, params)
+    psi, G, obs = _finish(out, G, cfg, res[0], wall, tr, 0, params, plan)
     if verbose:
         print(f"[gs] {obs['stop_reason']} it={obs['iters']}: E={obs['E']:.10g} "
               f"res={obs['resid_rel']:.3e}")

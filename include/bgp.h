@@ -175,6 +175,13 @@ int bgp_plan_stream_set(bgp_plan* plan, int N, int lines, int radix_order, int c
 int bgp_energy(bgp_plan* plan, int inst, const void* psi, double* phi_out,
                bgp_energy_terms* terms, void* stream);
 
+/* Energy terms of a solved state for its observables: the terms of bgp_energy from
+ * the sums of the solver's own energy program, in its order of summation (L_z of a
+ * state without rotation is a cancellation down to the last bits, and so stays
+ * reproducible with the solve). */
+int bgp_energy_observables(bgp_plan* plan, int inst, const void* psi, bgp_energy_terms* terms,
+                           void* stream);
+
 /* Gradient of the energy functional at psi (as given, not normalised); no
  * counterpart in the reference, derived from energy_components
  * (becgpp/operators.py:10-29). terms = the energy terms of bgp_energy;
