@@ -27,6 +27,7 @@ constexpr int kProfSlots = 20 * 5;   // phase profiler: 20 phase kinds x 5 count
 constexpr int kYieldDiv = 4;         // a solve launch yields once 1/kYieldDiv of it has finished
 constexpr int kTuneYield[3] = {2, 4, 8};  // relaunch schedules the autotuner tries
 constexpr int kMaxSegments = 256;    // relaunch limit of one solve
+constexpr int kTfAhead = 8;          // Thomas-Fermi steps enqueued between looks at their state
 constexpr int kResidBlocks = 592;    // blocks of the residual's sum: 4 per SM
 
 thread_local std::string g_err;
@@ -1434,8 +1435,7 @@ int bgp_tf_density(bgp_plan* p, int i, int nonlocal, double Omega, int iters, do
   A.b2 = I.beta2; A.b3 = I.beta3; A.gc = I.G_C; A.relax = relax;
   A.conv = nonlocal ? conv : nullptr;
   A.nf = n_out; A.part = I.part; A.bar = I.bar; A.abort_flag = p->d_abort; A.state = state;
-  double h[4] = {NAN, INFINITY, 0.0, 0.0};
-  int done = 0;
+  double h[5] = {NAN, INFINITY, 0.0, 0.0, 0.0};
   auto read_state = [&]() -> int {
     int ab = 0;
     CK(cudaMemcpyAsync(h, state, sizeof(h), cudaMemcpyDeviceToHost, st));
@@ -1449,27 +1449,28 @@ int bgp_tf_density(bgp_plan* p, int i, int nonlocal, double Omega, int iters, do
     void* args[] = {&A};
     if ((rc = tf_launch((void*)k_tf_iter, grid, args, p, I, st))) return rc;
     if ((rc = read_state())) return rc;
-    done = 1;
   } else {
     const double sigma = 0.15 * (I.dx * I.N / 2.0);   // 0.15 L
     double two_s2 = 2.0 * (sigma * sigma);
     void* sargs[] = {&A, &two_s2};
     if ((rc = tf_launch((void*)k_tf_seed, grid, sargs, p, I, st))) return rc;
+    // the host looks at the state every kTfAhead steps (a step after the last one returns
+    // at once): a wait per step was a tenth of the call, and much more on a busy host
     for (int it = 0; it < iters; ++it) {
       SLaunchT<1> SL{};
       op_density(p, I, n_out, conv, 0, SL);
       if ((rc = op_conv(p, SL, sched_rule(I), 0, nullptr, nullptr, st))) return rc;
       void* args[] = {&A};
       if ((rc = tf_launch((void*)k_tf_iter, grid, args, p, I, st))) return rc;
+      if ((it + 1) % kTfAhead != 0 && it + 1 < iters) continue;
       if ((rc = read_state())) return rc;
-      done = it + 1;
       if (h[2] != (double)kTfOk || h[3] != 0.0) break;
     }
   }
   info[0] = (h[2] == (double)kTfNoBracket) ? NAN : h[0];   // mu
   info[1] = h[3];                                          // converged
   info[2] = h[1];                                          // final dn
-  info[3] = (double)done;                                  // steps taken
+  info[3] = h[4];                                          // steps taken
   info[4] = h[2];                                          // status
   return BGP_OK;
 }

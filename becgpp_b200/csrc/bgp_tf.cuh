@@ -39,7 +39,7 @@ struct TfArgs {
   double* part;                  // 2 x 4 x gridDim.x partial sums
   unsigned long long* bar;       // team barrier counter
   int* abort_flag;               // status word (4 + gridDim.x ints)
-  double* state;                 // out: [0] mu, [1] dn, [2] status, [3] converged
+  double* state;                 // out: [0] mu, [1] dn, [2] status, [3] converged, [4] steps taken
 };
 
 enum TfStatus : int { kTfOk = 0, kTfNoBracket = 1, kTfEmpty = 2, kTfBarrier = 3 };
@@ -174,6 +174,9 @@ BGP_D bool grid_reduce(double (&v)[NV], const int (&op)[NV], double* part, int& 
 __global__ void __launch_bounds__(kThreads) k_tf_iter(TfArgs A) {
   __shared__ double sm[kTfSums * (kWarps + 1)];
   Team T{(int)blockIdx.x, (int)gridDim.x, A.bar, A.abort_flag};
+  // a step after the fixed point has converged or failed does nothing (the host enqueues
+  // several steps before it looks)
+  if (ld1(A.state + 2) != (double)kTfOk || ld1(A.state + 3) != 0.0) return;
   int slot = 0;
   const int n = A.n;
   const int first = blockIdx.x * kThreads + threadIdx.x, stride = gridDim.x * kThreads;
@@ -191,7 +194,7 @@ __global__ void __launch_bounds__(kThreads) k_tf_iter(TfArgs A) {
     for (int u = 0; u < kTfHold; ++u) hb[u] = first + u * stride < n ? base(first + u * stride) : 0.0;
   }
   auto fail = [&](int code) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) { A.state[2] = (double)code; A.state[3] = 0.0; }
+    if (blockIdx.x == 0 && threadIdx.x == 0) { A.state[2] = (double)code; A.state[3] = 0.0; A.state[4] += 1.0; }
   };
   // bracket of mu: [min base, max base + |b2| + |b3| + 1] (becgpp/thomasfermi.py:99-100)
   double lo, hi;
@@ -297,6 +300,7 @@ __global__ void __launch_bounds__(kThreads) k_tf_iter(TfArgs A) {
     A.state[1] = dn;
     A.state[2] = (double)kTfOk;
     A.state[3] = (A.mode == 0 || dn < 1e-9) ? 1.0 : 0.0;
+    A.state[4] += 1.0;
   }
 }
 
