@@ -785,11 +785,12 @@ Sched sched_of(const bgp_plan::StreamSched& sc) {
 // factorization with the fewest exchanges; a smaller one is a few microseconds of
 // latency: narrower tiles spread it over more SMs, and lengths 2^a take the
 // factorization with more threads per line. The autotuner picks the same on 128^3
-// (8 lines; 4 lines 3 % slower) and 256^2 (H psi 4 or 8 lines within 2 %; the quasi-2D
+// (8 lines; 4 lines 3 % slower), on 192^3 (padded lines of 384: the second factorization
+// 716 us, the first 772) and 256^2 (H psi 4 or 8 lines within 2 %; the quasi-2D
 // convolution 2 and 4 lines 17.5 us, 8 and 8 lines 19 us).
 Sched sched_rule(const Inst& I) {
-  if (I.n >= (1 << 19)) return Sched{8, 0, 8, 8, 0};
   const int v = (I.N & (I.N - 1)) == 0;
+  if (I.n >= (1 << 19)) return Sched{8, 0, 8, 8, I.ndim == 3 && !v};
   return Sched{4, v, 2, 4, v};
 }
 
@@ -1313,6 +1314,7 @@ int bgp_apply_H_batch(bgp_plan* p, int n, const int* idx, const void* const* psi
         S.psi = (const double2*)psi[b];
         S.H = (double2*)hpsi[b];
         S.phi = conv ? I.phi2 : (phi_mode == 1 ? phi[b] : nullptr);
+        if (!mu_dev) S.part = nullptr;         // (the sums cost the last pass of 256^3 4 %)
       }
       bgp_plan::StreamSched& sc = p->ssched[A0.N];
       if (sc.tuned == 0) {
