@@ -38,6 +38,7 @@ COMBOS = ((128, 0, 256, 0),)
 STREAM_LINES = (2, 4, 8)
 PAD_LINES = (4, 8)        # the padded, strided passes
 VARIANTS = (0, 1)
+SOLVER_SMALL = 4          # lines per tile of the solver's small configuration (kSvSmall)
 
 
 NVCC = os.environ.get("NVCC", "nvcc")
@@ -116,7 +117,7 @@ def generate():
                             cases.append(f"  if (c == {ln} && v == {v} && k == {k or 0} && batch == {int(nb != '1')}) {{\n"
                                          f"    constexpr int th = bgp::s_threads({length}, {ln}, {v});\n"
                                          f"    constexpr size_t sm = bgp::s_smem({length}, {ln}, {v});\n"
-                                         f"    static const bgp::SKernel e{{(void*)&{inst}, th, sm}};\n"
+                                         f"    static const bgp::SKernel e{{(void*)&{inst}, th, sm, bgp::s_min_blocks({length}, {ln}, {v})}};\n"
                                          f"    return &e;\n  }}")
             lines.append(f'extern "C" const bgp::SKernel* {fn}(int c, int v, int k, int batch) {{')
             lines += cases
@@ -138,6 +139,44 @@ def generate():
             stream_unit(os.path.join(GEN, f"s_conv_{m}.cu"), "bgp_stream.cuh",
                         [(f"bgp_srptr_{m}", "k_stream_real", n, STREAM_LINES, (0, 1)),
                          (f"bgp_spptr_{m}", "k_stream_pad", m, PAD_LINES, (0, 1, 2))])
+    # solver passes, three configurations per size (sv_step): tiles of 4 lines with the
+    # most threads per line, of 4 lines with fewer, and of 8 lines; where two factorizations
+    # coincide the first is used for both
+    def solver_unit(path, fn, entries):
+        lines, cases, seen = ['#include "bgp_solve.cuh"'], [], set()
+        for cfg in (0, 1, 2):
+            c = 8 if cfg == 2 else SOLVER_SMALL
+            for k, (kern, L, mode) in enumerate(entries):
+                pow2 = L & (L - 1) == 0
+                v = (2, 1 if pow2 else 2, 0 if not pow2 or fn.startswith("bgp_svc") else 1)[cfg]
+                args = [str(L), str(c), str(v)] + ([str(mode)] if mode is not None else [])
+                inst = f"bgp::{kern}<{', '.join(args)}>"
+                if inst not in seen:
+                    seen.add(inst)
+                    lines.append(f"template __global__ void {inst}(const __grid_constant__ bgp::SvLaunch);")
+                low = f"(sm < {8 * 1024} ? {8 * 1024} : sm)" if kern == "k_sv_hx" else "sm"
+                cases.append(f"  if (cfg == {cfg} && k == {k}) {{\n"
+                             f"    constexpr int th = bgp::s_threads({L}, {c}, {v});\n"
+                             f"    constexpr size_t sm = bgp::s_smem({L}, {c}, {v});\n"
+                             f"    static const bgp::SKernel e{{(void*)&{inst}, th, {low}, "
+                             f"bgp::{'s_min_blocks' if kern == 'k_sv_pad' else 'sv_blocks'}({L}, {c}, {v})}};\n"
+                             f"    return &e;\n  }}")
+        lines.append(f'extern "C" const bgp::SKernel* {fn}(int cfg, int k) {{')
+        lines += cases
+        lines.append("  return nullptr;\n}")
+        hdr.append(f'extern "C" const bgp::SKernel* {fn}(int cfg, int k);')
+        _write_if_changed(path, "\n".join(lines) + "\n")
+        units.append(path)
+
+    for n in SIZES_N:
+        solver_unit(os.path.join(GEN, f"sv_{n}.cu"), f"bgp_svptr_{n}",
+                    [("k_sv_trial", n, None), ("k_sv_hy", n, None), ("k_sv_hx", n, None), ("k_sv_p", n, 0),
+                     ("k_sv_p", n, 1), ("k_sv_p", n, 2), ("k_sv_px", n, None)])
+        if n <= MAX_N_WITH_KERNEL:
+            m = 2 * n
+            solver_unit(os.path.join(GEN, f"sv_conv_{m}.cu"), f"bgp_svcptr_{m}",
+                        [("k_sv_real", n, 0), ("k_sv_real", n, 1), ("k_sv_pad", m, 0), ("k_sv_pad", m, 1),
+                         ("k_sv_pad", m, 2)])
     _write_if_changed(os.path.join(GEN, "bgp_sizes_gen.h"), "\n".join(hdr) + "\n")
     return units
 
@@ -152,6 +191,8 @@ def _deps(src):
     # (the generated unit itself carries its instantiations, so build.py is no dependency)
     if os.path.basename(src).startswith(("k_", "k2_")):
         return [os.path.join(CSRC, f) for f in KERNEL_HEADERS]
+    if os.path.basename(src).startswith("sv_"):
+        return [os.path.join(CSRC, f) for f in KERNEL_HEADERS + ("bgp_solve.cuh", "bgp_stream.cuh", "bgp_lfft.cuh")]
     if os.path.basename(src).startswith("s_"):
         return [os.path.join(CSRC, f) for f in ("bgp_stream.cuh", "bgp_lfft.cuh", "bgp_device.cuh", "bgp_fft.cuh",
                                                 "bgp_common.cuh")]

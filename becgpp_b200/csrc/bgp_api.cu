@@ -18,6 +18,7 @@
 #include "bgp_table.cuh"
 #include "bgp_tf.cuh"
 #include "bgp_stream.cuh"
+#include "bgp_solve.cuh"
 
 using namespace bgp;
 
@@ -119,6 +120,7 @@ struct DevCtx {
   std::map<int, double2*> tw;   // twiddle tables by length
   std::map<int, float2*> tw32;  // the same rounded to FP32
   std::map<int, double2*> lf[kLVariants];   // line-transform tables of the stream passes
+  std::map<int, float2*> lf32[kLVariants];  // the same rounded to FP32
 };
 std::mutex g_mu;
 std::map<int, DevCtx> g_dev;
@@ -185,11 +187,17 @@ int lf_table(DevCtx* d) {
   CK(cudaMalloc(&dp, sizeof(double2) * len));
   CK(cudaMemcpy(dp, tab.data(), sizeof(double2) * len, cudaMemcpyHostToDevice));
   d->lf[V][L] = dp;
+  std::vector<float2> tf(len);
+  for (int q = 0; q < len; ++q) tf[q] = cmake<float2>((float)tab[q].x, (float)tab[q].y);
+  float2* fp = nullptr;
+  CK(cudaMalloc(&fp, sizeof(float2) * len));
+  CK(cudaMemcpy(fp, tf.data(), sizeof(float2) * len, cudaMemcpyHostToDevice));
+  d->lf32[V][L] = fp;
   return BGP_OK;
 }
 int lf_tables(DevCtx* d, int L) {
   switch (L) {
-#define X(l) case l: { int rc = lf_table<l, 0>(d); return rc ? rc : lf_table<l, 1>(d); }
+#define X(l) case l: { int rc = lf_table<l, 0>(d); if (!rc) rc = lf_table<l, 1>(d); return rc ? rc : lf_table<l, 2>(d); }
     BGP_FOR_LINE_LENGTHS(X)
 #undef X
     default: return fail(BGP_ERR_UNSUPPORTED, "line length not compiled in");
@@ -221,6 +229,16 @@ struct bgp_plan {
   double* d_res = nullptr;                // n_inst x (kNRec + 1)
   double* d_part = nullptr;               // partial sums of the operators' stream passes
   size_t part_energy = 0, part_conv = 0;  // its sections: energy sums; one convolution's sums
+  // stream solver
+  SvInst* d_sv = nullptr;
+  SvCtl* d_ctl = nullptr;
+  SvSync* d_svsync = nullptr;
+  unsigned* d_svhist = nullptr;           // kSvBins per instance
+  unsigned long long* d_svcand = nullptr; // kSvCap per instance
+  std::vector<double*> svpart;            // partial sums per instance
+  int* d_act = nullptr;                   // active instances, group by group
+  int *h_state = nullptr, *d_state = nullptr; // instances' solver states (mapped host memory)
+  std::vector<cudaEvent_t> sv_ev;         // two per size group
   double* h_sums = nullptr;               // totals on the host (mapped: the device writes them)
   double* d_sums = nullptr;               // the same memory as the device sees it
   int max_team = 0;
@@ -627,6 +645,8 @@ int bgp_plan_destroy(bgp_plan* p) {
   for (cudaEvent_t q : p->side_ev) cudaEventDestroy(q);
   for (void* q : p->allocs) cudaFree(q);
   if (p->h_sums) cudaFreeHost(p->h_sums);
+  if (p->h_state) cudaFreeHost(p->h_state);
+  for (cudaEvent_t q : p->sv_ev) cudaEventDestroy(q);
   delete p;
   return BGP_OK;
 }
@@ -926,7 +946,7 @@ int stream_autotune(bgp_plan::StreamSched& sc, SLaunchT<NB>& SL, bool conv, cuda
   sc.cand.clear();
   bgp_plan::StreamSched s = sc;
   for (int ln : {2, 4, 8}) {
-    for (int v = 0; v < kLVariants && !rc; ++v) {
+    for (int v = 0; v < 2 && !rc; ++v) {
       float ms = 0.f;
       s.ln = ln; s.v = v;
       if ((rc = timed(s, false, &ms))) break;
@@ -1477,6 +1497,254 @@ int bgp_tf_density(bgp_plan* p, int i, int nonlocal, double Omega, int iters, do
   return BGP_OK;
 }
 
+}  // extern "C"
+
+namespace {
+// ------------------------------------------------------------ stream solver
+const SKernel* solver_kernel(int N, int cfg, int k) {
+  switch (N) {
+#define X(n) case n: return bgp_svptr_##n(cfg, k);
+    BGP_FOR_STREAM_N(X)
+#undef X
+    default: return nullptr;
+  }
+}
+const SKernel* solver_conv_kernel(int M, int cfg, int k) {
+  switch (M) {
+#define X(m) case m: return bgp_svcptr_##m(cfg, k);
+    BGP_FOR_STREAM_M(X)
+#undef X
+    default: return nullptr;
+  }
+}
+enum : int { SK_TRIAL, SK_HY, SK_HX, SK_PYF, SK_PZ, SK_PYI, SK_PX };           // order of the generated tables
+enum : int { SC_FWD, SC_INV, SC_PB, SC_PC, SC_PD };
+
+constexpr int kSvSteps = 4;      // solver steps of a plane group enqueued at a time
+
+// instances of one (ndim, N, kernel): their launches share a stream
+struct SvGroup {
+  int ndim, N, M;
+  std::vector<int> ids;          // active instances
+  int act0 = 0;                  // their section of the plan's active list
+  cudaStream_t st = nullptr;
+  long long batches = 0;
+  bool dirty = true;             // the device's list is to be written
+};
+
+int sv_launch(bgp_plan* p, const SvGroup& g, const SKernel* k, int tiles, bool chained) {
+  if (!k) return fail(BGP_ERR_UNSUPPORTED, "solver pass not compiled for this size");
+  if (k->smem > 48 * 1024)
+    CK(cudaFuncSetAttribute(k->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k->smem));
+  const int na = (int)g.ids.size();
+  SvLaunch L{p->d_sv, p->d_ctl, p->d_svsync, p->d_act + g.act0, tiles, na, {}};
+  for (int q = 0; q < na && na <= kSvInline; ++q) L.inl[q] = g.ids[q];
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)std::min((long long)tiles * na, (long long)k->per_sm * p->dev->sms));
+  cfg.blockDim = dim3(k->threads);
+  cfg.dynamicSmemBytes = k->smem;
+  cfg.stream = g.st;
+  cfg.attrs = &at;
+  cfg.numAttrs = chained ? 1 : 0;
+  void* args[] = {&L};
+  CK(cudaLaunchKernelExC(&cfg, k->fn, args));
+  p->launches++;
+  return BGP_OK;
+}
+
+// A solver step of a group (see bgp_solve.cuh): the passes for which `want` has a state
+// bit (every bit: a whole step).
+int sv_step(bgp_plan* p, const SvGroup& g, bool chained, unsigned want = ~0u) {
+  const int N = g.N, M = g.M, lines = g.ndim == 2 ? N : N * N;
+  // tiles of 8 lines where half a million points fill the GPU with them; of 4 lines below,
+  // with the most threads per line (a few elements each) while every tile has an SM to
+  // itself. 256^2, us an iteration: alone 45 with the most threads, 53 with half as many;
+  // four together 93 and 68.
+  const int total = lines * (int)g.ids.size();
+  const int cfg = (long long)total * N >= (1 << 19) ? 2 : (total / kSvSmall > p->dev->sms ? 1 : 0);
+  const int C = cfg == 2 ? 8 : kSvSmall, t = lines / C;
+  int rc = BGP_OK;
+  auto has = [&](unsigned bits) { return (want & bits) != 0; };
+  auto run = [&](int k, int tiles) { if (!rc) { rc = sv_launch(p, g, solver_kernel(N, cfg, k), tiles, chained); chained = true; } };
+  auto crun = [&](int k, int tiles) { if (!rc) { rc = sv_launch(p, g, solver_conv_kernel(M, cfg, k), tiles, chained); chained = true; } };
+  auto conv = [&]() {
+    const int tpl = (N + 1 + C - 1) / C;
+    crun(SC_FWD, t);
+    if (g.ndim == 3) crun(SC_PB, N * tpl);
+    crun(SC_PC, (g.ndim == 2 ? 1 : M) * tpl);
+    if (g.ndim == 3) crun(SC_PD, N * tpl);
+    crun(SC_INV, t);
+  };
+  constexpr unsigned kTrial = 1u << ST_TRIAL | 1u << ST_INIT | 1u << ST_FINAL | 1u << ST_SWITCH, kH = 1u << ST_H | 1u << ST_MED;
+  if (g.ndim == 2) {
+    run(SK_TRIAL, 2 * t);
+    if (M) conv();                       // the trial state's own potential
+    run(SK_HX, t);
+    run(SK_PZ, t);
+    run(SK_PX, t);
+    return rc;
+  }
+  // a volume's potential (of the first, refreshed or returned state), then gradient,
+  // preconditioner and direction, the line search's two convolutions and its first trial
+  if (M && has(1u << ST_CONV)) conv();
+  if (has(1u << ST_CONV | kH)) { if (has(1u << ST_CONV | 1u << ST_H)) run(SK_HY, t); run(SK_HX, t); }
+  if (has(1u << ST_CONV | kH | 1u << ST_PRE)) { run(SK_PYF, t); run(SK_PZ, t); run(SK_PYI, t); run(SK_PX, t); }
+  if (M && has(1u << ST_CONV | kH | 1u << ST_PRE | 1u << ST_POLYB)) conv();
+  if (M && has(1u << ST_CONV | kH | 1u << ST_PRE | 1u << ST_POLYB | 1u << ST_POLYC)) conv();
+  if (has(1u << ST_CONV | kH | 1u << ST_PRE | 1u << ST_POLYB | 1u << ST_POLYC | kTrial)) run(SK_TRIAL, 3 * t);
+  return rc;
+}
+
+// the stream solver's state of a plan, allocated by its first mixed solve
+int sv_prepare(bgp_plan* p) {
+  if (p->d_sv) return BGP_OK;
+  const int n = (int)p->inst.size();
+  int rc = BGP_OK;
+  if ((rc = palloc_t(p, (size_t)n, &p->d_sv))) return rc;
+  if ((rc = palloc_t(p, (size_t)n, &p->d_ctl))) return rc;
+  if ((rc = palloc_t(p, (size_t)n, &p->d_svsync))) return rc;
+  if ((rc = palloc_t(p, (size_t)n * kSvBins, &p->d_svhist))) return rc;
+  if ((rc = palloc_t(p, (size_t)n * kSvCap, &p->d_svcand))) return rc;
+  if ((rc = palloc_t(p, (size_t)n, &p->d_act))) return rc;
+  for (const Inst& I : p->inst) {
+    // kDSums lists (the most a pass has) over its tiles of at least kSvSmall lines
+    double* q = nullptr;
+    if ((rc = palloc_t(p, (size_t)kDSums * (I.n / I.N / kSvSmall), &q))) return rc;
+    p->svpart.push_back(q);
+  }
+  if (cudaHostAlloc((void**)&p->h_state, sizeof(int) * n, cudaHostAllocMapped) != cudaSuccess ||
+      cudaHostGetDevicePointer((void**)&p->d_state, p->h_state, 0) != cudaSuccess)
+    return fail(BGP_ERR_OOM, "pinned host memory for the solver's flags");
+  return BGP_OK;
+}
+
+// All instances of the plan in the mixed form: results in p->d_out once the stream's work
+// is done.
+int sv_solve(bgp_plan* p, const void* const* psi0, void* const* psi_out, const SolverParams& P, double* d_trace,
+             cudaStream_t st) {
+  const int n = (int)p->inst.size();
+  if (n > p->grid_cap) return fail(BGP_ERR_ARG, "more instances than resident CTAs in one batch");
+  int prc = sv_prepare(p);
+  if (prc) return prc;
+  std::vector<SvInst> hi(n);
+  std::vector<SvCtl> hc(n);
+  std::vector<SvGroup> groups;
+  for (int i = 0; i < n; ++i) {
+    const Inst& I = p->inst[i];
+    SvInst& S = hi[i];
+    memset(&S, 0, sizeof(S));
+    S.ndim = I.ndim; S.N = I.N; S.n = I.n; S.M = I.M; S.Mh = I.Mh;
+    S.kern = has_kernel(I); S.poly = S.kern && I.ndim == 3;
+    S.dx = I.dx; S.dv = I.dv; S.kfac = I.kfac; S.s = I.s; S.tc = I.tc;
+    S.beta2 = I.beta2; S.beta3 = I.beta3; S.Omega = I.Omega; S.inv_n = I.inv_n; S.conv_scale = I.conv_scale;
+    S.pool = I.pool; S.phi2 = I.phi2; S.cb1 = I.cb1; S.cb2 = I.cb2; S.Kq = I.Kq; S.twM = I.twM;
+    for (int V = 0; V < kLVariants; ++V) {
+      S.tabN[V] = p->dev->lf[V][I.N];
+      S.tabF[V] = p->dev->lf32[V][I.N];
+      S.tabM[V] = I.M ? p->dev->lf[V][I.M] : nullptr;
+    }
+    S.keys = I.keys;
+    S.wcand = p->d_svcand + (size_t)i * kSvCap;
+    S.hist = p->d_svhist + (size_t)i * kSvBins;
+    S.part = p->svpart[i];
+    S.in_psi = (const double2*)psi0[i];
+    S.out_c = (double2*)psi_out[i];
+    S.sp = P;
+    S.trace = d_trace ? d_trace + (size_t)3 * P.trace_cap * i : nullptr;
+    S.out = p->d_out + i;
+    S.hstate = p->d_state + i;
+    SvCtl& c = hc[i];
+    memset(&c, 0, sizeof(c));
+    c.st = ST_INIT; c.kind = KD_INIT;
+    for (int q = 0; q < F_NLOG; ++q) { c.f[q] = -1; c.sc[q] = 1.0; }
+    c.f[F_A] = 0; c.f[F_H] = 1; c.f[F_W] = 2;
+    c.hf = -1;
+    c.fp32 = 1; c.fp64_from = -1;
+    c.phisc = 1.0;
+    c.stop = kStopMaxit;
+    c.alpha = P.alpha0; c.sigma = P.shift_min; c.med_eps = 1e-3;
+    ((volatile int*)p->h_state)[i] = ST_INIT;
+    const int M = S.kern ? I.M : 0;
+    SvGroup* g = nullptr;
+    for (SvGroup& q : groups) if (q.ndim == I.ndim && q.N == I.N && q.M == M) g = &q;
+    if (!g) { groups.emplace_back(); g = &groups.back(); g->ndim = I.ndim; g->N = I.N; g->M = M; }
+    g->ids.push_back(i);
+  }
+  CK(cudaMemcpyAsync(p->d_sv, hi.data(), sizeof(SvInst) * n, cudaMemcpyHostToDevice, st));
+  CK(cudaMemcpyAsync(p->d_ctl, hc.data(), sizeof(SvCtl) * n, cudaMemcpyHostToDevice, st));
+  CK(cudaMemsetAsync(p->d_svhist, 0, sizeof(unsigned) * kSvBins * (size_t)n, st));
+  CK(cudaMemsetAsync(p->d_svsync, 0, sizeof(SvSync) * (size_t)n, st));
+  // the first group on the caller's stream, the others on side streams that start after
+  // the work enqueued so far
+  if (p->side_ev.empty()) {
+    cudaEvent_t e;
+    CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    p->side_ev.push_back(e);
+  }
+  CK(cudaEventRecord(p->side_ev[0], st));
+  int act0 = 0;
+  for (size_t q = 0; q < groups.size(); ++q) {
+    SvGroup& g = groups[q];
+    g.act0 = act0;
+    act0 += (int)g.ids.size();
+    g.st = st;
+    if (q > 0) {
+      int rc = side_stream(p, (int)q, &g.st);
+      if (rc) return rc;
+      CK(cudaStreamWaitEvent(g.st, p->side_ev[0], 0));
+    }
+    while (p->sv_ev.size() < 2 * (q + 1)) {
+      cudaEvent_t e;
+      CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+      p->sv_ev.push_back(e);
+    }
+  }
+  // every step ends an iteration, a trial or a level of a median search of each of its
+  // instances, so this many batches are enough for any solve
+  const long long most = ((long long)P.maxit + 4) * ((long long)std::max(P.ls_max, 1) + 16) + 16;
+  for (bool busy = true; busy;) {
+    busy = false;
+    for (size_t q = 0; q < groups.size(); ++q) {
+      SvGroup& g = groups[q];
+      if (g.ids.empty()) continue;
+      // planes: whole steps, the host two batches behind (a pass is a few us). Volumes: a
+      // pass is tens of us and a skipped one a few, so the host waits for the state after
+      // every trial and enqueues what it asks for
+      const bool direct = g.ndim == 3;
+      cudaEvent_t ev = p->sv_ev[2 * q + (direct ? 0 : g.batches & 1)];
+      if (g.batches >= (direct ? 1 : 2)) CK(cudaEventSynchronize(ev));
+      std::vector<int> left;
+      for (int i : g.ids) if (((volatile int*)p->h_state)[i] != ST_DONE) left.push_back(i);
+      if (left.size() != g.ids.size()) { g.ids.swap(left); g.dirty = true; }
+      if (g.ids.empty()) continue;
+      if (g.batches > most) return fail(BGP_ERR_DEVICE, "solve did not finish within its step limit");
+      busy = true;
+      if (g.dirty)
+        CK(cudaMemcpyAsync(p->d_act + g.act0, g.ids.data(), sizeof(int) * g.ids.size(), cudaMemcpyHostToDevice, g.st));
+      unsigned want = direct ? 0u : ~0u;
+      if (direct) for (int i : g.ids) want |= 1u << ((volatile int*)p->h_state)[i];
+      for (int s = 0; s < (direct ? 1 : kSvSteps); ++s) {
+        int rc = sv_step(p, g, !(s == 0 && g.dirty), want);
+        if (rc) return rc;
+        g.dirty = false;
+      }
+      CK(cudaEventRecord(ev, g.st));
+      g.batches++;
+    }
+  }
+  for (size_t q = 1; q < groups.size(); ++q) {
+    CK(cudaEventRecord(p->side_ev[q], groups[q].st));
+    CK(cudaStreamWaitEvent(st, p->side_ev[q], 0));
+  }
+  return BGP_OK;
+}
+}  // namespace
+
+extern "C" {
+
 int bgp_solve(bgp_plan* p, const void* const* psi0, void* const* psi_out, const bgp_solver_params* sp,
               bgp_solve_result* results, double* trace, void* stream) {
   if (!p || !psi0 || !psi_out || !sp || !results) return fail(BGP_ERR_ARG, "null pointer");
@@ -1526,6 +1794,11 @@ int bgp_solve(bgp_plan* p, const void* const* psi0, void* const* psi_out, const 
     CK(cudaEventCreate(&ev0));
     CK(cudaEventCreate(&ev1));
     CK(cudaEventRecord(ev0, st));
+  }
+  if (P.mixed) {
+    rc = sv_solve(p, psi0, psi_out, P, d_trace, st);
+    act.clear();
+    if (rc) cudaDeviceSynchronize();   // nothing of it may still run when the call returns
   }
   for (int seg = 0; !act.empty() && seg < kMaxSegments; ++seg) {
     const int na = (int)act.size();

@@ -36,26 +36,27 @@ struct LPlan {
 
 // Compiled factorizations: variant 0 has the fewest exchanges its registers allow
 // (E <= 16), variant 1 is the alternative with more threads per line (or, for
-// lengths 2^a 3, another order); the autotuner times both. E is a multiple of every
-// radix, the first radix is even.
+// lengths 2^a 3, another order), the autotuner of the applies times both; variant 2 has
+// the most threads per line (the solver's passes on a grid too small to fill the GPU).
+// E is a multiple of every radix, the first radix is even.
 BGP_HD constexpr LPlan lplan(int L, int V) {
   switch (L) {
-    case 16: return V ? LPlan{8, 2, {2, 8}} : LPlan{4, 2, {4, 4}};
+    case 16: return V == 1 ? LPlan{8, 2, {2, 8}} : LPlan{4, 2, {4, 4}};
     case 24: return V ? LPlan{6, 3, {6, 2, 2}} : LPlan{12, 2, {6, 4}};
     case 32: return V ? LPlan{4, 3, {4, 4, 2}} : LPlan{8, 2, {8, 4}};
-    case 48: return V ? LPlan{12, 3, {4, 4, 3}} : LPlan{12, 2, {12, 4}};
+    case 48: return V ? (V == 1 ? LPlan{12, 3, {4, 4, 3}} : LPlan{6, 4, {6, 2, 2, 2}}) : LPlan{12, 2, {12, 4}};
     case 64: return V ? LPlan{4, 3, {4, 4, 4}} : LPlan{8, 2, {8, 8}};
-    case 96: return V ? LPlan{12, 3, {12, 4, 2}} : LPlan{12, 3, {6, 4, 4}};
-    case 128: return V ? LPlan{8, 3, {8, 4, 4}} : LPlan{16, 2, {16, 8}};
-    case 192: return V ? LPlan{12, 3, {4, 4, 12}} : LPlan{12, 3, {12, 4, 4}};
-    case 256: return V ? LPlan{8, 3, {8, 8, 4}} : LPlan{16, 2, {16, 16}};
-    case 384: return V ? LPlan{24, 3, {8, 8, 6}} : LPlan{12, 4, {6, 4, 4, 4}};
+    case 96: return V == 1 ? LPlan{12, 3, {12, 4, 2}} : LPlan{12, 3, {6, 4, 4}};
+    case 128: return V ? (V == 1 ? LPlan{8, 3, {8, 4, 4}} : LPlan{4, 4, {4, 4, 4, 2}}) : LPlan{16, 2, {16, 8}};
+    case 192: return V == 1 ? LPlan{12, 3, {4, 4, 12}} : LPlan{12, 3, {12, 4, 4}};
+    case 256: return V ? (V == 1 ? LPlan{8, 3, {8, 8, 4}} : LPlan{4, 4, {4, 4, 4, 4}}) : LPlan{16, 2, {16, 16}};
+    case 384: return V == 1 ? LPlan{24, 3, {8, 8, 6}} : LPlan{12, 4, {6, 4, 4, 4}};
     case 512: return V ? LPlan{8, 3, {8, 8, 8}} : LPlan{16, 3, {16, 8, 4}};
-    case 768: return V ? LPlan{24, 3, {8, 8, 12}} : LPlan{12, 4, {12, 4, 4, 4}};
+    case 768: return V == 1 ? LPlan{24, 3, {8, 8, 12}} : LPlan{12, 4, {12, 4, 4, 4}};
     default: return LPlan{1, 1, {1, 1, 1, 1}};   // not compiled
   }
 }
-constexpr int kLVariants = 2;
+constexpr int kLVariants = 3;
 
 // geometry of stage S: P = product of the earlier radices, Lr = what is left of the
 // point index after it
@@ -112,29 +113,30 @@ BGP_HD constexpr double lf_cos(int R, int m) {
 BGP_HD constexpr double lf_sin(int R, int m) { return lf_cos(48, ((48 / R) * m + 36) % 48); }
 
 // v times w_R^m (forward) or its conjugate (inverse), m and R compile-time
-template <int R, int M, bool INV>
-BGP_HD double2 lf_rot(double2 v) {
+template <int R, int M, bool INV, class T>
+BGP_HD T lf_rot(T v) {
+  using Rt = typename CT<T>::R;
   constexpr int m = M % R;
   if constexpr (m == 0) {
     return v;
   } else if constexpr (4 * m == R) {
     return rot90<INV>(v);
   } else if constexpr (2 * m == R) {
-    return cmk(-v.x, -v.y);
+    return cmake<T>(-v.x, -v.y);
   } else if constexpr (4 * m == 3 * R) {
     return rot90<!INV>(v);
   } else if constexpr (8 * m == R) {           // (1 -+ i) / sqrt 2
-    return cscale(cadd(v, rot90<INV>(v)), kR2);
+    return cscale(cadd(v, rot90<INV>(v)), (Rt)kR2);
   } else if constexpr (8 * m == 3 * R) {       // (-1 -+ i) / sqrt 2
-    return cscale(csub(rot90<INV>(v), v), kR2);
+    return cscale(csub(rot90<INV>(v), v), (Rt)kR2);
   } else {
     constexpr double c = lf_cos(R, m), s = lf_sin(R, m);
-    return cmul(v, cmk(c, INV ? s : -s));
+    return cmul(v, cmake<T>((Rt)c, (Rt)(INV ? s : -s)));
   }
 }
 
-template <int R, int A, bool INV>
-BGP_HD void lf_rot_all(double2* v) {           // v[a] *= w_R^a, a < A
+template <int R, int A, bool INV, class T>
+BGP_HD void lf_rot_all(T* v) {           // v[a] *= w_R^a, a < A
   if constexpr (A > 1) {
     lf_rot_all<R, A - 1, INV>(v);
     v[A - 1] = lf_rot<R, A - 1, INV>(v[A - 1]);
@@ -142,14 +144,14 @@ BGP_HD void lf_rot_all(double2* v) {           // v[a] *= w_R^a, a < A
 }
 
 // R-point transform of v[0..R-1], natural order in and out
-template <int R, bool INV>
-BGP_HD void lf_dft(double2* v) {
+template <int R, bool INV, class T>
+BGP_HD void lf_dft(T* v) {
   if constexpr (R == 1) {
   } else if constexpr (R == 2 || R == 3 || R == 4 || R == 8) {
     dft_small<R, INV>(v);
   } else if constexpr (R == 6) {
     // prime-factor map: n = 2 a + 3 b, k = 4 p + 3 q (mod 6)
-    double2 x[2][3] = {{v[0], v[2], v[4]}, {v[3], v[5], v[1]}};
+    T x[2][3] = {{v[0], v[2], v[4]}, {v[3], v[5], v[1]}};
     dft_small<3, INV>(x[0]);
     dft_small<3, INV>(x[1]);
 #pragma unroll
@@ -159,7 +161,7 @@ BGP_HD void lf_dft(double2* v) {
     }
   } else if constexpr (R == 12) {
     // prime-factor map: n = 4 a + 3 b, k = 4 p + 9 q (mod 12)
-    double2 x[4][3];
+    T x[4][3];
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
 #pragma unroll
@@ -168,7 +170,7 @@ BGP_HD void lf_dft(double2* v) {
     }
 #pragma unroll
     for (int p = 0; p < 3; ++p) {
-      double2 y[4] = {x[0][p], x[1][p], x[2][p], x[3][p]};
+      T y[4] = {x[0][p], x[1][p], x[2][p], x[3][p]};
       dft_small<4, INV>(y);
 #pragma unroll
       for (int q = 0; q < 4; ++q) v[(4 * p + 9 * q) % 12] = y[q];
@@ -176,7 +178,7 @@ BGP_HD void lf_dft(double2* v) {
   } else {
     static_assert(R == 16, "radix 1, 2, 3, 4, 6, 8, 12 or 16");
     // 4 x 4: n = 4 a + b, k = p + 4 q
-    double2 x[4][4];
+    T x[4][4];
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
 #pragma unroll
@@ -194,7 +196,7 @@ BGP_HD void lf_dft(double2* v) {
     x[3][3] = lf_rot<16, 9, INV>(x[3][3]);
 #pragma unroll
     for (int p = 0; p < 4; ++p) {
-      double2 y[4] = {x[0][p], x[1][p], x[2][p], x[3][p]};
+      T y[4] = {x[0][p], x[1][p], x[2][p], x[3][p]};
       dft_small<4, INV>(y);
 #pragma unroll
       for (int q = 0; q < 4; ++q) v[p + 4 * q] = y[q];
@@ -203,10 +205,10 @@ BGP_HD void lf_dft(double2* v) {
 }
 
 // forward transform whose inputs a >= R / 2 are zero (v[0..R/2-1] in, R values out)
-template <int R>
-BGP_HD void lf_dft_half_in(double2* v) {
+template <int R, class T>
+BGP_HD void lf_dft_half_in(T* v) {
   constexpr int H = R / 2;
-  double2 e[H], o[H];
+  T e[H], o[H];
 #pragma unroll
   for (int a = 0; a < H; ++a) { e[a] = v[a]; o[a] = v[a]; }
   lf_rot_all<R, H, false>(o);
@@ -217,10 +219,10 @@ BGP_HD void lf_dft_half_in(double2* v) {
 }
 
 // inverse transform of which only the outputs a < R / 2 are wanted
-template <int R>
-BGP_HD void lf_dft_half_out(double2* v) {
+template <int R, class T>
+BGP_HD void lf_dft_half_out(T* v) {
   constexpr int H = R / 2;
-  double2 e[H], o[H];
+  T e[H], o[H];
 #pragma unroll
   for (int b = 0; b < H; ++b) { e[b] = v[2 * b]; o[b] = v[2 * b + 1]; }
   lf_dft<H, true>(e);
@@ -233,13 +235,13 @@ BGP_HD void lf_dft_half_out(double2* v) {
 // ------------------------------------------------------- one thread's stage work
 // Stage S of thread t on its registers, forward: the sub-transforms and, but for the
 // last stage, the twiddles. HALF: the first stage of a line whose upper half is zero.
-template <int L, int V, int S, bool HALF>
-BGP_HD void lf_stage_fwd(double2 (&v)[lplan(L, V).E], const double2* tab, int t) {
+template <int L, int V, int S, bool HALF, class C>
+BGP_HD void lf_stage_fwd(C (&v)[lplan(L, V).E], const C* tab, int t) {
   constexpr LPlan p = lplan(L, V);
   constexpr int R = p.r[S], NB = p.E / R, T = L / p.E, Lr = lf_Lr(L, V, S), off = lf_tab_off(L, V, S);
 #pragma unroll
   for (int s = 0; s < NB; ++s) {
-    double2 x[R];
+    C x[R];
 #pragma unroll
     for (int a = 0; a < (HALF ? R / 2 : R); ++a) x[a] = v[s + NB * a];
     if constexpr (HALF) lf_dft_half_in<R>(x);
@@ -253,13 +255,13 @@ BGP_HD void lf_stage_fwd(double2 (&v)[lplan(L, V).E], const double2* tab, int t)
     for (int b = 0; b < R; ++b) v[s + NB * b] = x[b];
   }
 }
-template <int L, int V, int S, bool HALF>
-BGP_HD void lf_stage_inv(double2 (&v)[lplan(L, V).E], const double2* tab, int t) {
+template <int L, int V, int S, bool HALF, class C>
+BGP_HD void lf_stage_inv(C (&v)[lplan(L, V).E], const C* tab, int t) {
   constexpr LPlan p = lplan(L, V);
   constexpr int R = p.r[S], NB = p.E / R, T = L / p.E, Lr = lf_Lr(L, V, S), off = lf_tab_off(L, V, S);
 #pragma unroll
   for (int s = 0; s < NB; ++s) {
-    double2 x[R];
+    C x[R];
 #pragma unroll
     for (int b = 0; b < R; ++b) x[b] = v[s + NB * b];
     if constexpr (S + 1 < p.n) {
@@ -349,17 +351,17 @@ inline void lf_fill_table(const double2* w, double2* tab) {
 // The exchange buffer of a tile: slot i of line c at i * LS + c * CS. On a strided
 // axis the lines are interleaved (LS = lines, CS = 1), so 8 neighbouring lines fill
 // one 128-byte wavefront; on the contiguous axis they are CS apart (LS = 1).
-template <int L, int V, int LS, bool WARP>
+template <int L, int V, int LS, bool WARP, class C = double2>
 struct LineFft {
   static constexpr LPlan p = lplan(L, V);
   static constexpr int E = p.E, T = L / E;
-  double2* sm;              // this line's slot 0
-  const double2* __restrict__ tab;
+  C* sm;              // this line's slot 0
+  const C* __restrict__ tab;
   int t;                    // thread of the line
   BGP_D static void sync() { if constexpr (WARP) __syncwarp(); else __syncthreads(); }
 
   template <int X, bool FWD>
-  BGP_D void exchange(double2 (&v)[E]) const {
+  BGP_D void exchange(C (&v)[E]) const {
     constexpr int RB = p.r[X], RA = p.r[X + 1], NBB = E / RB, NBA = E / RA;
     sync();                 // the previous exchange (or use of the buffer) has been read
 #pragma unroll
@@ -375,7 +377,7 @@ struct LineFft {
     }
   }
   template <bool HALF, int S = 0>
-  BGP_D void forward(double2 (&v)[E]) const {
+  BGP_D void forward(C (&v)[E]) const {
     lf_stage_fwd<L, V, S, HALF && S == 0>(v, tab, t);
     if constexpr (S + 1 < p.n) {
       exchange<S, true>(v);
@@ -383,7 +385,7 @@ struct LineFft {
     }
   }
   template <bool HALF, int S = p.n - 1>
-  BGP_D void inverse(double2 (&v)[E]) const {
+  BGP_D void inverse(C (&v)[E]) const {
     lf_stage_inv<L, V, S, HALF && S == 0>(v, tab, t);
     if constexpr (S > 0) {
       exchange<S - 1, false>(v);

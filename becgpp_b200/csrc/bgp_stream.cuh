@@ -91,6 +91,7 @@ struct SKernel {
   void* fn;
   int threads;
   size_t smem;
+  int per_sm;             // CTAs per SM the registers are budgeted for
 };
 
 #if defined(__CUDACC__)
@@ -112,7 +113,8 @@ struct Tile {
     c = CONTIG ? tid / T : tid % CP;
     t = CONTIG ? tid % T : tid / CP;
   }
-  BGP_D double2* line(double2* sm) const { return sm + (CONTIG ? c * lf_slots(L, V) : c); }
+  template <class F = double2>
+  BGP_D F* line(double2* sm) const { return reinterpret_cast<F*>(sm) + (CONTIG ? c * lf_slots(L, V) : c); }
 };
 
 // Sums of NV values over the CTA (W warps) in a fixed order; thread 0 holds the totals.
@@ -338,47 +340,40 @@ __global__ void __launch_bounds__(s_threads(N, C, V), s_min_blocks(N, C, V))
   }
 }
 
-// strided steps: MODE 0: step b (forward); 1: 2D columns and 3D step c (forward, K^,
-// inverse); 2: step d (inverse)
-template <int M, int C, int V, int MODE, int NB>
-__global__ void __launch_bounds__(s_threads(M, C, V), s_min_blocks(M, C, V))
-    k_stream_pad(const __grid_constant__ SLaunchT<NB> SL) {
+// One tile of a strided step: MODE 0: step b (forward); 1: 2D columns and 3D step c
+// (forward, K^, inverse); 2: step d (inverse).
+template <int M, int C, int V, int MODE>
+BGP_D void pad_tile(int tile, int ndim, double2* cb1, double2* cb2, const double* Kq, const double2* tab, double2* sm) {
   using TL = Tile<M, C, V, false>;
   constexpr int E = TL::E, T = TL::T, N = M / 2, Mh = N + 1, Mp = conv_pitch(N), tpl = (Mh + C - 1) / C;
-  extern __shared__ double2 sm[];
-  const int inst = NB == 1 ? 0 : blockIdx.x / SL.tiles, tile = blockIdx.x - inst * SL.tiles;
-  const SInst& I = SL.insts[inst];
   const TL tl;
   const int t = tl.t;
   const int a = tile / tpl, kk = (tile - a * tpl) * C + tl.c;   // a: i (b, d) or jj (c); 0 in 2D
   const bool valid = tl.c < C && kk < Mh;
-  const typename TL::Fft fft{tl.line(sm), I.tabM[V], t};
-  pdl_trigger();
+  const typename TL::Fft fft{tl.line(sm), tab, t};
   const double2* in;
   double2* out;
-  size_t si, so;
+  size_t str;
   if (MODE == 1) {
-    out = I.ndim == 2 ? I.cb1 + kk : I.cb2 + (size_t)a * Mp + kk;
+    out = ndim == 2 ? cb1 + kk : cb2 + (size_t)a * Mp + kk;
     in = out;
-    si = so = I.ndim == 2 ? (size_t)Mp : (size_t)M * Mp;
+    str = ndim == 2 ? (size_t)Mp : (size_t)M * Mp;
   } else {
-    double2* x1 = I.cb1 + (size_t)a * N * Mp + kk;
-    double2* x2 = I.cb2 + (size_t)a * M * Mp + kk;
+    double2* x1 = cb1 + (size_t)a * N * Mp + kk;
+    double2* x2 = cb2 + (size_t)a * M * Mp + kk;
     in = MODE == 0 ? x1 : x2;
     out = MODE == 0 ? x2 : x1;
-    si = so = Mp;
+    str = Mp;
   }
-  pdl_wait();
   double2 v[E];
 #pragma unroll
-  for (int q = 0; q < (MODE == 2 ? E : E / 2); ++q)
-    v[q] = valid ? in[(size_t)(t + T * q) * si] : cmk(0.0, 0.0);
+  for (int q = 0; q < (MODE == 2 ? E : E / 2); ++q) v[q] = valid ? in[(size_t)(t + T * q) * str] : cmk(0.0, 0.0);
   if (MODE != 2) fft.template forward<true>(v);
   if (MODE == 1) {
     // K^ is real and even: K^[min(k, M - k)] of the quadrant's column
     const int bj = a <= N ? a : M - a;
-    const double* __restrict__ K = I.Kq + (I.ndim == 2 ? (size_t)0 : (size_t)bj * Mh) + kk;
-    const size_t sk = I.ndim == 2 ? (size_t)Mh : (size_t)Mh * Mh;
+    const double* __restrict__ K = Kq + (ndim == 2 ? (size_t)0 : (size_t)bj * Mh) + kk;
+    const size_t sk = ndim == 2 ? (size_t)Mh : (size_t)Mh * Mh;
 #pragma unroll
     for (int q = 0; q < E; ++q) {
       const int k = t + T * q;
@@ -389,7 +384,17 @@ __global__ void __launch_bounds__(s_threads(M, C, V), s_min_blocks(M, C, V))
   if (MODE != 0) fft.template inverse<true>(v);
 #pragma unroll
   for (int q = 0; q < (MODE == 0 ? E : E / 2); ++q)
-    if (valid) out[(size_t)(t + T * q) * so] = v[q];
+    if (valid) out[(size_t)(t + T * q) * str] = v[q];
+}
+template <int M, int C, int V, int MODE, int NB>
+__global__ void __launch_bounds__(s_threads(M, C, V), s_min_blocks(M, C, V))
+    k_stream_pad(const __grid_constant__ SLaunchT<NB> SL) {
+  extern __shared__ double2 sm[];
+  const int inst = NB == 1 ? 0 : blockIdx.x / SL.tiles, tile = blockIdx.x - inst * SL.tiles;
+  const SInst& I = SL.insts[inst];
+  pdl_trigger();
+  pdl_wait();
+  pad_tile<M, C, V, MODE>(tile, I.ndim, I.cb1, I.cb2, I.Kq, I.tabM[V], sm);
 }
 
 // ------------------------------------------------------------------ energy sums

@@ -55,7 +55,8 @@ template <int L, int V, bool HALF> void check() {
   printf("%d %d %d %.3Le %.3Le\n", L, V, (int)HALF, sqrtl(e / s), sqrtl(g / h));
 }
 int main() {
-#define CHECK(l) check<l, 0, false>(); check<l, 0, true>(); check<l, 1, false>(); check<l, 1, true>();
+#define CHECK(l) check<l, 0, false>(); check<l, 0, true>(); check<l, 1, false>(); check<l, 1, true>(); \
+  check<l, 2, false>(); check<l, 2, true>();
   LENGTHS
 }
 """
@@ -73,7 +74,7 @@ def test_every_length_and_factorization(tmp_path):
                    capture_output=True)
     rows = [r.split() for r in subprocess.run([str(exe)], check=True, capture_output=True,
                                               text=True).stdout.splitlines()]
-    assert len(rows) == 4 * len(LENGTHS)
+    assert len(rows) == 6 * len(LENGTHS)
     for L, v, half, fwd, pair in rows:
         tol = 2.0 ** -52 * math.log2(int(L))
         assert float(fwd) < tol and float(pair) < 2 * tol, (L, v, half, fwd, pair)
