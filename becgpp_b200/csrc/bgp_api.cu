@@ -51,25 +51,20 @@ bool size_ok(int N, int M) {
   return false;
 }
 
-// kernel entry for a size pair, or for two pairs (mixed: the build with FP32
-// transforms); null if not compiled
-void* kernel_for(int N, int M, int ndim, bool mixed = false) {
-#define X(n, m)                                                                              \
-  if (N == n && M == m) {                                                                    \
-    if (ndim == 3) return mixed ? bgp_kptr_##n##_##m##_d3_mx() : bgp_kptr_##n##_##m##_d3(); \
-    return mixed ? bgp_kptr_##n##_##m##_d2_mx() : bgp_kptr_##n##_##m##_d2();               \
-  }
+// persistent kernel of a size pair, or of two pairs; null if not compiled
+void* kernel_for(int N, int M, int ndim) {
+#define X(n, m) if (N == n && M == m) return ndim == 3 ? bgp_kptr_##n##_##m##_d3() : bgp_kptr_##n##_##m##_d2();
   BGP_FOR_SIZES(X)
 #undef X
   return nullptr;
 }
 // two-size kernels (2D only)
-void* kernel_for2(int N1, int M1, int N2, int M2, int ndim, bool mixed = false) {
+void* kernel_for2(int N1, int M1, int N2, int M2, int ndim) {
   if (ndim != 2) return nullptr;
 #define X(a, b, c, d)                                                                      \
   if ((N1 == a && M1 == b && N2 == c && M2 == d) ||                                      \
       (N1 == c && M1 == d && N2 == a && M2 == b))                                        \
-    return mixed ? bgp_kptr2_##a##_##b##_##c##_##d##_d2_mx() : bgp_kptr2_##a##_##b##_##c##_##d##_d2();
+    return bgp_kptr2_##a##_##b##_##c##_##d##_d2();
   BGP_FOR_COMBOS(X)
 #undef X
   return nullptr;
@@ -81,7 +76,6 @@ void* kernel_for2(int N1, int M1, int N2, int M2, int ndim, bool mixed = false) 
 template <int L>
 struct OpCube {
   static constexpr bool kStore = true;
-  static constexpr bool kMixed = false;
   BGP_NO_OUT(64)
   const Inst& I;
   int ax;
@@ -118,7 +112,6 @@ struct DevCtx {
   int device = -1, sms = 0, max_grid = 0;
   size_t max_smem_optin = 0;
   std::map<int, double2*> tw;   // twiddle tables by length
-  std::map<int, float2*> tw32;  // the same rounded to FP32
   std::map<int, double2*> lf[kLVariants];   // line-transform tables of the stream passes
   std::map<int, float2*> lf32[kLVariants];  // the same rounded to FP32
 };
@@ -162,12 +155,6 @@ int twiddles(DevCtx* d, int L, const double2** out) {
   CK(cudaMalloc(&dp, sizeof(double2) * L));
   CK(cudaMemcpy(dp, h.data(), sizeof(double2) * L, cudaMemcpyHostToDevice));
   d->tw[L] = dp;
-  std::vector<float2> hf(L);
-  for (int t = 0; t < L; ++t) hf[t] = cmake<float2>((float)h[t].x, (float)h[t].y);
-  float2* fp = nullptr;
-  CK(cudaMalloc(&fp, sizeof(float2) * L));
-  CK(cudaMemcpy(fp, hf.data(), sizeof(float2) * L, cudaMemcpyHostToDevice));
-  d->tw32[L] = fp;
   *out = dp;
   return BGP_OK;
 }
@@ -202,14 +189,6 @@ int lf_tables(DevCtx* d, int L) {
 #undef X
     default: return fail(BGP_ERR_UNSUPPORTED, "line length not compiled in");
   }
-}
-
-int twiddles32(DevCtx* d, int L, const float2** out) {
-  const double2* dp = nullptr;
-  int rc = twiddles(d, L, &dp);
-  if (rc) return rc;
-  *out = d->tw32[L];
-  return BGP_OK;
 }
 
 }  // namespace
@@ -359,14 +338,12 @@ int grid_cap_for(bgp_plan* p, void* kern, int* cap) {
 int max_grid(bgp_plan* p) {
   int cap = 1 << 30;
   for (const Inst& I : p->inst) {
-    for (bool mixed : {false, true}) {
-      void* k = kernel_for(I.N, I.M, I.ndim, mixed);
-      if (!k) return fail(BGP_ERR_UNSUPPORTED, "grid size not compiled in");
-      int c = 0;
-      int rc = grid_cap_for(p, k, &c);
-      if (rc) return rc;
-      cap = c < cap ? c : cap;
-    }
+    void* k = kernel_for(I.N, I.M, I.ndim);
+    if (!k) return fail(BGP_ERR_UNSUPPORTED, "grid size not compiled in");
+    int c = 0;
+    int rc = grid_cap_for(p, k, &c);
+    if (rc) return rc;
+    cap = c < cap ? c : cap;
   }
   p->grid_cap = cap;
   return BGP_OK;
@@ -397,20 +374,16 @@ int launch(bgp_plan* p, const std::vector<int>& active, cudaStream_t st) {
     for (auto& q : kinds) seen = seen || q == k;
     if (!seen) kinds.push_back(k);
   }
-  // a mixed-precision solve runs in the kernels built with FP32 transforms while
-  // one of its instances still uses them
-  bool mixed = false;
-  for (int a : active) mixed = mixed || (p->inst[a].prog == kProgSolve && p->inst[a].sp.mixed);
   if (kinds.size() == 1)
-    return launch_group(p, active, kernel_for(kinds[0][1], kinds[0][2], kinds[0][0], mixed), st);
+    return launch_group(p, active, kernel_for(kinds[0][1], kinds[0][2], kinds[0][0]), st);
   if (kinds.size() == 2 && kinds[0][0] == kinds[1][0]) {
-    void* k2 = kernel_for2(kinds[0][1], kinds[0][2], kinds[1][1], kinds[1][2], kinds[0][0], mixed);
+    void* k2 = kernel_for2(kinds[0][1], kinds[0][2], kinds[1][1], kinds[1][2], kinds[0][0]);
     if (k2) return launch_group(p, active, k2, st);
   }
   for (auto& k : kinds) {
     std::vector<int> grp;
     for (int a : active) if (kind_of(a) == k) grp.push_back(a);
-    int rc = launch_group(p, grp, kernel_for(k[1], k[2], k[0], mixed), st);
+    int rc = launch_group(p, grp, kernel_for(k[1], k[2], k[0]), st);
     if (rc) return rc;
   }
   return BGP_OK;
@@ -572,9 +545,7 @@ int bgp_plan_create(const bgp_instance_desc* desc, int n_inst, bgp_plan** plan) 
     const bgp_instance_desc& d = desc[i];
     const size_t n = (size_t)I.n;
     if ((rc = twiddles(dev, I.N, &I.twN))) return bail(rc);
-    if ((rc = twiddles32(dev, I.N, &I.twN32))) return bail(rc);
     if (I.M && (rc = twiddles(dev, I.M, &I.twM))) return bail(rc);
-    if (I.M && (rc = twiddles32(dev, I.M, &I.twM32))) return bail(rc);
     if ((rc = lf_tables(dev, I.N))) return bail(rc);
     if (I.M && (rc = lf_tables(dev, I.M))) return bail(rc);
     if ((rc = palloc_t(p, (size_t)kNB * n, &I.pool))) return bail(rc);
@@ -1814,8 +1785,6 @@ int bgp_solve(bgp_plan* p, const void* const* psi0, void* const* psi_out, const 
       if (outs[a].status == 2) {
         next.push_back(a);
         p->inst[a].resume = 1;
-        // handed over to FP64: later segments run in the smaller FP64-only kernels
-        if (outs[a].fp64_from >= 0) p->inst[a].sp.mixed = 0;
       }
     }
     act.swap(next);

@@ -33,14 +33,13 @@ BGP_D void tile_map(int e, int& r, int& c) {
 // loads of a batch in flight together), then the batch is entered into shared
 // memory; each warp transforms its line; the way out fetches every operand of
 // the thread's elements, then stores.
-template <int L, bool CONTIG, class T, class Op>
-BGP_D void tile_run_t(Op& op, double2* smd, int t) {
+template <int L, bool CONTIG, class Op>
+BGP_D void tile_run(Op& op, double2* sm, int t) {
   constexpr int TOT = kLines * L;
   constexpr int PER = (TOT + kThreads - 1) / kThreads;
   constexpr int LS = line_stride(L);
   constexpr int CH = (Op::kChunk < PER) ? Op::kChunk : PER;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  T* sm = reinterpret_cast<T*>(smd);
 #pragma unroll
   for (int u0 = 0; u0 < PER; u0 += CH) {
     Pre pre[CH];
@@ -59,7 +58,7 @@ BGP_D void tile_run_t(Op& op, double2* smd, int t) {
       if (u0 + q < PER && (TOT % kThreads == 0 || e < TOT)) {
         int r, c;
         tile_map<L, CONTIG>(e, r, c);
-        sm[c * LS + swz(r)] = to_c<T>(op.enter(pre[q], t, r, c));
+        sm[c * LS + swz(r)] = op.enter(pre[q], t, r, c);
       }
     }
   }
@@ -79,7 +78,7 @@ BGP_D void tile_run_t(Op& op, double2* smd, int t) {
           int r, c;
           tile_map<L, CONTIG>(e, r, c);
           pre[q] = op.fetch_out(t, r, c);
-          v[q] = to_d(sm[c * LS + swz(r)]);
+          v[q] = sm[c * LS + swz(r)];
         }
       }
 #pragma unroll
@@ -94,17 +93,6 @@ BGP_D void tile_run_t(Op& op, double2* smd, int t) {
     }
   }
   __syncthreads();
-}
-
-// A tile in the operator's FP64 arithmetic, or with FP32 transforms when
-// `fp32` is set, the operator supports them (Op::kMixed) and this is a
-// mixed-precision build (BGP_MIXED).
-template <int L, bool CONTIG, class Op>
-BGP_D void tile_run(Op& op, double2* sm, int t, int fp32 = 0) {
-  if constexpr (Op::kMixed && BGP_MIXED) {
-    if (fp32) { tile_run_t<L, CONTIG, float2>(op, sm, t); return; }
-  }
-  tile_run_t<L, CONTIG, double2>(op, sm, t);
 }
 
 // Multiply line element r (r = lane, lane + 32, ...) by the real kernel value
@@ -142,10 +130,9 @@ template <int N>
   [[maybe_unused]] double2* H = Q.H; \
   [[maybe_unused]] const double* phi = Q.phi; \
   [[maybe_unused]] const double psc = Q.psc, phisc = Q.phisc; \
-  [[maybe_unused]] const int ax = Q.ax, stage = Q.stage, sp = Q.fp32;
+  [[maybe_unused]] const int ax = Q.ax, stage = Q.stage;
 struct OpH {
   static constexpr bool kStore = true;
-  static constexpr bool kMixed = true;
   static constexpr int kChunk = 64;
   static constexpr int kChunkOut = 4;    // A, psi and phi per element on the way out
   const Inst& I;
@@ -155,16 +142,13 @@ struct OpH {
     OPH_ARGS
     int i, j, k;
     Pre P;
-    P.a = cscale(ldp(psi, nline_elem(g, ax, t, r, c, i, j, k), sp), psc);
+    P.a = cscale(ld2(psi + nline_elem(g, ax, t, r, c, i, j, k)), psc);
     return P;
   }
   BGP_D double2 enter(const Pre& P, int, int, int) { return P.a; }
-  template <class T>
-  BGP_D void line(T* b, int lane, int t, int w) {
+  BGP_D void line(double2* b, int lane, int t, int w) {
     OPH_ARGS
-    using Rt = typename CT<T>::R;
-    const T* twt = twN_of<T>(I);
-    warp_fft<N, false>(b, twt, lane);
+    warp_fft<N, false>(b, tw, lane);
     int i, j, k;
     nline_elem(g, ax, t, 0, w, i, j, k);
     const double wx = (ax == 1) ? -g.Omega * xcoord(g, i) : ((ax == 0) ? g.Omega * xcoord(g, j) : 0.0);
@@ -176,11 +160,11 @@ struct OpH {
       if (N % 32 == 0 || r < N) {
         const double kk = kof(g, r);
         const double m = 0.5 * kk * kk + wx * kk;
-        b[swz(r)] = cscale(b[swz(r)], (Rt)(m * inv));
+        b[swz(r)] = cscale(b[swz(r)], m * inv);
       }
     }
     __syncwarp();
-    warp_fft<N, true>(b, twt, lane);
+    warp_fft<N, true>(b, tw, lane);
   }
   BGP_D Pre fetch_out(int t, int r, int c) {
     OPH_ARGS
@@ -188,9 +172,9 @@ struct OpH {
     if (stage == 0) return P;
     int i, j, k;
     const int f = nline_elem(g, ax, t, r, c, i, j, k);
-    P.b = ldp(A, f, sp);
+    P.b = ld2(A + f);
     if (stage == 2) {
-      P.a = cscale(ldp(psi, f, sp), psc);
+      P.a = cscale(ld2(psi + f), psc);
       P.r = phi ? phisc * ld1(phi + f) : 0.0;
     }
     return P;
@@ -199,13 +183,13 @@ struct OpH {
     OPH_ARGS
     int i, j, k;
     const int f = nline_elem(g, ax, t, r, c, i, j, k);
-    if (stage == 0) { stp(A, f, v, sp); return; }
-    if (stage == 1) { stp(A, f, cadd(P.b, v), sp); return; }
+    if (stage == 0) { st2(A + f, v); return; }
+    if (stage == 1) { st2(A + f, cadd(P.b, v)); return; }
     const double2 p = P.a;
     const double rho = cabs2(p);
     const double pot = potential(g, i, j, k) + g.beta2 * rho + g.beta3 * rho * rho + P.r;
     const double2 h = cadd(cadd(P.b, v), cscale(p, pot));
-    stp(H, f, h, sp);
+    st2(H + f, h);
     acc.s[0] += p.x * h.x + p.y * h.y;
     acc.mx = fmax(acc.mx, rho);
   }
@@ -225,10 +209,9 @@ template <int N>
   [[maybe_unused]] const double2* cin = Q.cin; \
   [[maybe_unused]] double2* W = Q.W; \
   [[maybe_unused]] double2* DIRC = Q.DIRC; \
-  [[maybe_unused]] const int init = Q.init, write_dirc = Q.write_dirc, write_w = Q.write_w, sp = Q.fp32;
+  [[maybe_unused]] const int init = Q.init, write_dirc = Q.write_dirc, write_w = Q.write_w;
 struct OpT {
   static constexpr bool kStore = false;
-  static constexpr bool kMixed = true;
   BGP_NO_OUT(4)                          // three complex operands per element
   const Inst& I;
   const PassArgs& Q;
@@ -239,12 +222,12 @@ struct OpT {
     int i, j, k;
     const int f = nline_elem(g, ax, tt, r, c, i, j, k);
     Pre P;
-    // src: the stored trial state (pool; the caller's state when sp == 0 in mode 2)
-    if (ax != BGP_DIM(g) - 1) { P.a = ldp(src, f, sp); return P; }
+    // src: the stored trial state (pool; the caller's state in mode 2)
+    if (ax != BGP_DIM(g) - 1) { P.a = ld2(src + f); return P; }
     if (init) { P.a = ld2(cin + f); return P; }      // the caller's state: complex128
     if (write_dirc) { dirc_fetch(D, f, P); return P; }
-    P.a = cscale(ldp(D.psi, f, sp), D.psc);
-    P.b = ldp(DIRC, f, sp);
+    P.a = cscale(ld2(D.psi + f), D.psc);
+    P.b = ld2(DIRC + f);
     return P;
   }
   BGP_D double2 enter(const Pre& P, int tt, int r, int c) {
@@ -254,14 +237,14 @@ struct OpT {
     const int f = nline_elem(g, ax, tt, r, c, i, j, k);
     double2 w;
     if (init) {
-      w = rnd_sp(P.a, sp);
+      w = P.a;
     } else {
       double2 d;
-      if (write_dirc) { d = rnd_sp(dirc_of(D, P), sp); stp(DIRC, f, d, sp); }
+      if (write_dirc) { d = dirc_of(D, P); st2(DIRC + f, d); }
       else d = P.b;
-      w = rnd_sp(csub(P.a, cscale(d, D.t)), sp);
+      w = csub(P.a, cscale(d, D.t));
     }
-    if (write_w) stp(W, f, w, sp);
+    if (write_w) st2(W + f, w);
     const double q = cabs2(w);
     const double x = xcoord(g, i), y = xcoord(g, j);
     acc.s[S_N0] += q;
@@ -280,10 +263,9 @@ struct OpT {
     acc.mx = fmax(acc.mx, q);
     return w;
   }
-  template <class T>
-  BGP_D void line(T* b, int lane, int tt, int w) {
+  BGP_D void line(double2* b, int lane, int tt, int w) {
     OPT_ARGS
-    warp_fft<N, false>(b, twN_of<T>(I), lane);
+    warp_fft<N, false>(b, tw, lane);
     int i, j, k;
     nline_elem(g, ax, tt, 0, w, i, j, k);
     double sk = 0.0, sl = 0.0;
@@ -325,10 +307,9 @@ template <int N>
   [[maybe_unused]] unsigned long long* wcand = I.wcand; \
   [[maybe_unused]] const double psc = Q.psc, mu = Q.mu, thr = Q.thr, phisc = Q.phisc; \
   [[maybe_unused]] const unsigned long long win_lo = Q.win_lo, win_hi = Q.win_hi; \
-  [[maybe_unused]] const int keys_on = Q.keys_on, win_on = Q.win_on, sp = Q.fp32;
+  [[maybe_unused]] const int keys_on = Q.keys_on, win_on = Q.win_on;
 struct OpG {
   static constexpr bool kStore = true;
-  static constexpr bool kMixed = true;
   BGP_NO_OUT(4)
   const Inst& I;
   const PassArgs& Q;
@@ -342,8 +323,8 @@ struct OpG {
     int i, j, k;
     const int f = elem(t, r, c, i, j, k);
     Pre P;
-    P.a = cscale(ldp(psi, f, sp), psc);
-    P.b = gin ? ld2(gin + f) : ldp(Hin, f, sp);      // a given gradient is the caller's
+    P.a = cscale(ld2(psi + f), psc);
+    P.b = gin ? ld2(gin + f) : ld2(Hin + f);      // a given gradient is the caller's
     P.r = (keys_on && phi) ? ld1(phi + f) : 0.0;
     return P;
   }
@@ -353,7 +334,7 @@ struct OpG {
     const int f = elem(t, r, c, i, j, k);
     const double2 p = P.a;
     const double2 gr = gin ? P.b : csub(P.b, cscale(p, mu));
-    if (Gout) stp(Gout, f, gr, sp);
+    if (Gout) st2(Gout + f, gr);
     acc.s[0] += cabs2(gr);
     if (keys_on) {
       const double rho = cabs2(p);
@@ -378,12 +359,11 @@ struct OpG {
     }
     return gr;
   }
-  template <class T>
-  BGP_D void line(T* b, int lane, int, int) { warp_fft<N, false>(b, twN_of<T>(I), lane); }
+  BGP_D void line(double2* b, int lane, int, int) { warp_fft<N, false>(b, I.twN, lane); }
   BGP_D void leave(const Pre&, int t, int r, int c, double2 v) {
     OPG_ARGS
     int i, j, k;
-    stp(A, elem(t, r, c, i, j, k), v, sp);
+    st2(A + elem(t, r, c, i, j, k), v);
   }
 };
 
@@ -398,10 +378,9 @@ template <int N>
   [[maybe_unused]] double2* A = Q.A; \
   [[maybe_unused]] double2* Z = Q.Z; \
   [[maybe_unused]] const double psc = Q.psc, sigma = Q.sigma, inv_n = I.inv_n; \
-  [[maybe_unused]] const int ax = Q.ax, mode = Q.mode, sp = Q.fp32;
+  [[maybe_unused]] const int ax = Q.ax, mode = Q.mode;
 struct OpP {
   static constexpr bool kStore = true;
-  static constexpr bool kMixed = true;
   static constexpr int kChunk = 64;
   static constexpr int kChunkOut = 8;
   const Inst& I;
@@ -411,16 +390,13 @@ struct OpP {
     OPP_ARGS
     int i, j, k;
     Pre P;
-    P.a = ldp(A, nline_elem(g, ax, t, r, c, i, j, k), sp);
+    P.a = ld2(A + nline_elem(g, ax, t, r, c, i, j, k));
     return P;
   }
   BGP_D double2 enter(const Pre& P, int, int, int) { return P.a; }
-  template <class T>
-  BGP_D void line(T* b, int lane, int t, int w) {
+  BGP_D void line(double2* b, int lane, int t, int w) {
     OPP_ARGS
-    using Rt = typename CT<T>::R;
-    const T* twt = twN_of<T>(I);
-    if (mode <= 1) warp_fft<N, false>(b, twt, lane);
+    if (mode <= 1) warp_fft<N, false>(b, tw, lane);
     if (mode == 1) {
       int i, j, k;
       nline_elem(g, ax, t, 0, w, i, j, k);
@@ -435,19 +411,19 @@ struct OpP {
           double K2 = kx * kx + ky * ky;
           if (BGP_DIM(g) == 3) K2 = K2 + kz * kz;
           const double rden = 1.0 / (0.5 * K2 + sigma);
-          b[swz(r)] = cscale(b[swz(r)], (Rt)rden);
+          b[swz(r)] = cscale(b[swz(r)], rden);
         }
       }
       __syncwarp();
     }
-    if (mode >= 1) warp_fft<N, true>(b, twt, lane);
+    if (mode >= 1) warp_fft<N, true>(b, tw, lane);
   }
   BGP_D Pre fetch_out(int t, int r, int c) {
     OPP_ARGS
     Pre P{};
     if (mode == 3) {
       int i, j, k;
-      P.a = cscale(ldp(psi, nline_elem(g, ax, t, r, c, i, j, k), sp), psc);
+      P.a = cscale(ld2(psi + nline_elem(g, ax, t, r, c, i, j, k)), psc);
     }
     return P;
   }
@@ -455,9 +431,9 @@ struct OpP {
     OPP_ARGS
     int i, j, k;
     const int f = nline_elem(g, ax, t, r, c, i, j, k);
-    if (mode < 3) { stp(A, f, v, sp); return; }
+    if (mode < 3) { st2(A + f, v); return; }
     const double2 z = cscale(v, inv_n);
-    stp(Z, f, z, sp);
+    st2(Z + f, z);
     const double2 pz = cconjmul(P.a, z);
     acc.s[0] += pz.x;
     acc.s[1] += pz.y;
@@ -482,7 +458,6 @@ template <int M>
   [[maybe_unused]] const RhoArgs R = rho_args(Q, Q.rmode);
 struct OpCa {
   static constexpr bool kStore = true;
-  static constexpr bool kMixed = false;
   BGP_NO_OUT(4)
   const Inst& I;
   const PassArgs& Q;
@@ -513,7 +488,6 @@ template <int M>
   [[maybe_unused]] const double* Kq = Q.Kq;
 struct OpC2b {
   static constexpr bool kStore = true;
-  static constexpr bool kMixed = false;
   BGP_NO_OUT(64)
   const Inst& I;
   const PassArgs& Q;
@@ -558,7 +532,6 @@ template <int M>
   [[maybe_unused]] const int sum_on = Q.sum_on;
 struct OpCinv {
   static constexpr bool kStore = true;
-  static constexpr bool kMixed = false;
   static constexpr int kChunk = 8;
   static constexpr int kChunkOut = 4;
   const Inst& I;
@@ -617,7 +590,6 @@ template <int M>
   [[maybe_unused]] const int inverse = Q.inverse;
 struct OpC3b {
   static constexpr bool kStore = true;
-  static constexpr bool kMixed = false;
   BGP_NO_OUT(64)
   const Inst& I;
   const PassArgs& Q;
@@ -663,7 +635,6 @@ template <int M>
   [[maybe_unused]] const double* Kq = Q.Kq;
 struct OpC3c {
   static constexpr bool kStore = true;
-  static constexpr bool kMixed = false;
   BGP_NO_OUT(64)
   const Inst& I;
   const PassArgs& Q;

@@ -38,7 +38,6 @@ struct Ctl {
   double nkeys;                      // keys written by the last gradient pass
   int med_valid, win_used, fast_hits, slow_runs;
   int yield, it_next;                 // segmented solve
-  int fp32, cg_reset, fp64_from, do_switch;  // mixed form: FP32 on; restart CG; hand-over
   // line search of 3D instances with a kernel: pair sums G_xy = sum Phi_x y of the
   // trial density's parts a = |psi|^2, b = Re(conj(psi) dirc), c = |dirc|^2
   // (aa, ab, ac, bb, bc, cc)
@@ -111,8 +110,7 @@ BGP_D bool phase_end0(Ctx& C) { return phase_sync(C); }
 template <int L1, bool C1, class Op1>
 BGP_D void run_one(Ctx& C, Op1& a, int n1) {
   BGP_PROF_T(ta)
-  const int fp32 = C.Q.fp32;
-  for (int u = C.T.rank; u < n1; u += C.T.size) tile_run<L1, C1>(a, C.sm, u, fp32);
+  for (int u = C.T.rank; u < n1; u += C.T.size) tile_run<L1, C1>(a, C.sm, u);
   BGP_PROF_T(tb)
   BGP_PROF_ADD(C, 18, tb - ta)
 }
@@ -120,10 +118,9 @@ BGP_D void run_one(Ctx& C, Op1& a, int n1) {
 template <int L1, bool C1, class Op1, int L2, bool C2, class Op2>
 BGP_D void run_two(Ctx& C, Op1& a, int n1, Op2& b, int n2) {
   BGP_PROF_T(ta)
-  const int fp32 = C.Q.fp32;
   for (int u = C.T.rank; u < n1 + n2; u += C.T.size) {
-    if (u < n1) tile_run<L1, C1>(a, C.sm, u, fp32);
-    else tile_run<L2, C2>(b, C.sm, u - n1, fp32);
+    if (u < n1) tile_run<L1, C1>(a, C.sm, u);
+    else tile_run<L2, C2>(b, C.sm, u - n1);
   }
   BGP_PROF_T(tb)
   BGP_PROF_ADD(C, 18, tb - ta)
@@ -559,68 +556,6 @@ __device__ __noinline__ bool residual_phases(Ctx& C, Ctl& S) {
   return true;
 }
 
-// Mixed form: consecutive failed line searches in FP32 after which the FP64
-// iterations take over.
-constexpr int kMixedFailSwitch = 3;
-
-// Mixed form: hand over from FP32 to FP64 transforms. The energy, potential,
-// residual and median keys of the current state are evaluated again in FP64,
-// the CG recurrence restarts (beta = 0, no Barzilai-Borwein update) and the
-// energy window and the lowest-residual iterate start afresh.
-template <int N, int M>
-__device__ __noinline__ bool switch_to_fp64(Ctx& C, Ctl& S, int it) {
-  const Inst& I = C.I;
-  PassArgs& Q = C.Q;
-  // every thread has read the control state that led here (S.fp32 among it)
-  // before thread 0 changes it
-  __syncthreads();
-  // the FP32 phase stored the pool fields as complex64: widen the state into a
-  // free pool field (complex128), unscaled; the fields of the earlier iterates are
-  // not read again (the recurrence restarts from the new gradient and z)
-  if (threadIdx.x == 0) {
-    S.f[F_G] = -1; S.f[F_Z] = -1; S.f[F_W] = -1; S.f[F_DIRC] = -1;
-    S.f[F_PSIP] = -1; S.f[F_GP] = -1; S.f[F_ZP] = -1; S.f[F_DIR] = -1; S.f[F_BEST] = -1;
-    S.f[F_H] = pool_alloc(S);
-    S.ok = S.f[F_H] >= 0;
-  }
-  __syncthreads();
-  if (!S.ok) return false;
-  {
-    const double2* src = pool_buf(I, S.f[F_PSI]);
-    double2* dst = pool_buf(I, S.f[F_H]);
-    for (int f = C.T.rank * kThreads + threadIdx.x; f < I.n; f += C.T.size * kThreads)
-      st2(dst + f, ldp(src, f, 1));
-  }
-  if (!phase_end0(C)) return false;
-  if (threadIdx.x == 0) {
-    S.f[F_PSI] = S.f[F_H]; S.f[F_H] = -1;
-    S.f[F_PSIP] = S.f[F_PSI]; S.sc[F_PSIP] = S.sc[F_PSI];
-    S.fp32 = 0; Q.fp32 = 0; S.fp64_from = it;
-    Q.cin = pool_buf(I, S.f[F_PSI]);
-  }
-  __syncthreads();
-  if (!energy_phases<N, M>(C, S, 2, 0, nullptr, nullptr, phi_buf(I, S.phi_cur))) return false;
-  if (threadIdx.x == 0) {
-    // the complex64 state's norm differs from 1 by its rounding: normalize it again
-    const double c = 1.0 / sqrt(S.tsum[S_N0] * I.dv);
-    S.sc[F_PSI] = c; S.sc[F_PSIP] = c;
-    double comp[8];
-    energy_assemble(I, S.tsum, c * c, comp);
-    S.E = comp[0];
-    S.phisc = c * c;
-  }
-  __syncthreads();
-  if (!residual_phases<N, M>(C, S)) return false;
-  if (threadIdx.x == 0) {
-    S.f[F_GP] = S.f[F_G];
-    S.need_pz = 1; S.cg_reset = 1; S.n_fail = 0;
-    S.best_resid = S.resid_rel; S.f[F_BEST] = S.f[F_PSI]; S.sc[F_BEST] = S.sc[F_PSI];
-    S.E_ref = S.E; S.it_ref = it;
-  }
-  __syncthreads();
-  return true;
-}
-
 // ------------------------------------------------------------------ the solver
 template <int N, int M>
 BGP_D void prog_solve(Ctx& C, Ctl& S) {
@@ -634,7 +569,7 @@ BGP_D void prog_solve(Ctx& C, Ctl& S) {
   int it0 = 0;
   if (I.resume) {
     // continue a yielded solve: restore the control state saved by the last launch
-    if (tid == 0) { S = *reinterpret_cast<const Ctl*>(I.save); Q.fp32 = S.fp32; }
+    if (tid == 0) { S = *reinterpret_cast<const Ctl*>(I.save); }
     __syncthreads();
     it0 = S.it_next;
     goto iterate;
@@ -648,8 +583,7 @@ BGP_D void prog_solve(Ctx& C, Ctl& S) {
     S.ntrials = 0; S.ntrace = 0; S.z_proj = 0; S.need_pz = 1; S.accepted = 0; S.ok = 1; S.naccept = 0;
     S.med_valid = 0; S.med_eps = 1e-3; S.win_used = 0; S.fast_hits = 0; S.slow_runs = 0; S.med_prev = 0.0;
     S.alpha = P.alpha0; S.sigma = P.shift_min; S.beta = 0.0; S.done = 0;
-    S.fp32 = BGP_MIXED ? P.mixed : 0; S.cg_reset = 0; S.fp64_from = S.fp32 ? -1 : 0;
-    Q.cin = I.in_psi; Q.fp32 = S.fp32;
+    Q.cin = I.in_psi;
   }
   __syncthreads();
   // ---- initial state: psi = psi0 / ||psi0||, its energy and potential
@@ -698,9 +632,8 @@ iterate:
       if (tid == 0) {
         S.cpsi = cmk(C.tot[0] * dv, C.tot[1] * dv);   // <psi, z_raw> dV
         S.z_proj = 0;
-        // first iteration, and the first after the hand-over to FP64 (whose earlier
-        // z and direction are FP32 fields): start the recurrence from z
-        if (it == 0 || S.cg_reset) { S.f[F_ZP] = S.f[F_Z]; S.f[F_DIR] = S.f[F_Z]; }
+        // first iteration: start the recurrence from z
+        if (it == 0) { S.f[F_ZP] = S.f[F_Z]; S.f[F_DIR] = S.f[F_Z]; }
       }
       __syncthreads();
     }
@@ -720,15 +653,14 @@ iterate:
       const bool proj = !S.z_proj;
       const double2 aproj = S.cpsi;
       const int n = I.n;
-      const int sp = S.fp32;     // pool fields in FP32 while the mixed form runs in FP32
       for (int f = C.T.rank * kThreads + tid; f < n; f += C.T.size * kThreads) {
-        const double2 p = cscale(ldp(ps, f, sp), psc);
-        double2 z = ldp(Z, f, sp);
-        if (proj) { z = csub(z, cmul(aproj, p)); stp(Z, f, z, sp); }
-        const double2 g = ldp(G, f, sp), gp = ldp(GP, f, sp);
-        const double2 zp = zp_alias ? z : ldp(ZP, f, sp);
-        const double2 d = d_alias ? z : ldp(D, f, sp);
-        const double2 q = cscale(ldp(pp, f, sp), ppc);
+        const double2 p = cscale(ld2(ps + f), psc);
+        double2 z = ld2(Z + f);
+        if (proj) { z = csub(z, cmul(aproj, p)); st2(Z + f, z); }
+        const double2 g = ld2(G + f), gp = ld2(GP + f);
+        const double2 zp = zp_alias ? z : ld2(ZP + f);
+        const double2 d = d_alias ? z : ld2(D + f);
+        const double2 q = cscale(ld2(pp + f), ppc);
         const double2 y = csub(g, gp), s = csub(p, q);
         a.s[0] += z.x * y.x + z.y * y.y;
         a.s[1] += zp.x * gp.x + zp.y * gp.y;
@@ -749,7 +681,7 @@ iterate:
         S.z_proj = 1;
         const double* r = C.tot;
         double beta = 0.0;
-        if (!(it == 0 || S.cg_reset || P.cg_beta == 2 || (P.restart > 0 && it % P.restart == 0))) {
+        if (!(it == 0 || P.cg_beta == 2 || (P.restart > 0 && it % P.restart == 0))) {
           if (P.cg_beta == 0) {
             const double den = fmax(r[1] * dv, 1e-300);
             beta = fmax(0.0, (r[0] * dv) / den);
@@ -777,7 +709,7 @@ iterate:
           gd = (r[14] - (pg.x * gpsi.x - pg.y * gpsi.y)) * dv;
         }
         S.gd = gd;
-        if (it > 0 && !S.cg_reset) {
+        if (it > 0) {
           const double sy = r[12] * dv;
           if (sy > 1e-30 && isfinite(sy)) {
             double bb = (r[13] * dv) / sy;
@@ -788,7 +720,6 @@ iterate:
           }
         }
         S.alpha = fmin(fmax(S.alpha, P.alpha_min), P.alpha_max);
-        S.cg_reset = 0;
         S.trial = S.alpha;
         S.accepted = 0;
         S.f[F_DIRC] = pool_alloc(S);
@@ -857,13 +788,7 @@ iterate:
         S.f[F_DIR] = S.f[F_Z];
         S.f[F_DIRC] = -1; S.f[F_W] = -1;
         S.need_pz = 0;
-        S.do_switch = 0;
-        if (S.fp32) {
-          // mixed form: repeated failures mean the energy change has reached the
-          // FP32 floor; the FP64 iterations take over instead of stopping
-          S.done = 0;
-          S.do_switch = (S.n_fail >= kMixedFailSwitch || S.alpha <= P.alpha_min);
-        } else if (S.alpha <= P.alpha_min || S.n_fail >= P.stall_max) {
+        if (S.alpha <= P.alpha_min || S.n_fail >= P.stall_max) {
           S.stop = kStopStalled; S.done = 1;
         } else {
           S.done = 0;
@@ -871,7 +796,6 @@ iterate:
       }
       __syncthreads();
       if (S.done) break;
-      if (S.do_switch && !switch_to_fp64<N, M>(C, S, it)) goto fail;
       continue;
     }
     if (poly) {
@@ -909,9 +833,6 @@ iterate:
     }
     __syncthreads();
     if (!residual_phases<N, M>(C, S)) goto fail;
-    if (S.fp32 && S.resid_rel < P.mixed_tol) {
-      if (!switch_to_fp64<N, M>(C, S, it)) goto fail;
-    }
     if (tid == 0) {
       S.need_pz = 1;
       S.done = 0;
@@ -923,9 +844,7 @@ iterate:
         S.best_resid = S.resid_rel;
         S.f[F_BEST] = S.f[F_PSI]; S.sc[F_BEST] = S.sc[F_PSI];
       }
-      if (S.fp32) {
-        // convergence is declared in FP64 only
-      } else if (S.resid_rel < P.res_tol) { S.converged = 1; S.stop = kStopConverged; S.done = 1; }
+      if (S.resid_rel < P.res_tol) { S.converged = 1; S.stop = kStopConverged; S.done = 1; }
       else if (it - S.it_ref >= P.window) {
         const double dE = fabs(S.E - S.E_ref) / fmax(1.0, fabs(S.E));
         if (dE < P.etol) { S.converged = 1; S.stop = kStopEnergy; S.done = 1; }
@@ -943,23 +862,19 @@ iterate:
         SolveOut o{};
         o.status = 2;
         o.iters = S.n_iter;
-        o.fp64_from = S.fp64_from;   // -1: still in FP32 transforms
         *I.out = o;
       }
       return;
     }
   }
   // ---- result: lowest-residual iterate, then its energy and residual afresh (FP64)
-  if (tid == 0) Q.fp32 = 0;
-  __syncthreads();
   {
     const int use_best = S.best_resid < S.resid_rel;
     const int fb = use_best ? F_BEST : F_PSI;
     const double2* src = pool_buf(I, S.f[fb]);
     const double sc = S.sc[fb];
-    const int sp = S.fp32;     // still FP32 storage if the iterations ended before the hand-over
     for (int f = C.T.rank * kThreads + tid; f < I.n; f += C.T.size * kThreads)
-      st2(I.out_c + f, cscale(ldp(src, f, sp), sc));
+      st2(I.out_c + f, cscale(ld2(src + f), sc));
     if (!phase_end0(C)) goto fail;
     // energy terms of the returned state (and its potential into phi buffer 0)
     if (tid == 0) {
@@ -991,7 +906,7 @@ iterate:
       o.sigma = S.sigma; o.mu = S.mu; o.alpha = S.alpha; o.maxrho = S.maxrho;
       o.E_final = comp[0]; o.mu_final = muf; o.resid_abs_final = raf;
       o.resid_rel_final = raf / fmax(1.0, fabs(muf)); o.mass_final = massf;
-      o.fp64_from = S.fp64_from; o.pad2_ = 0;
+      o.fp64_from = 0; o.pad2_ = 0;
       *I.out = o;
       __threadfence();
       if (I.finished) atomicAdd(I.finished, 1);
@@ -1016,7 +931,7 @@ BGP_D void prog_api(Ctx& C, Ctl& S) {
   double* res = I.res;
   if (tid == 0) {
     Q.psi = I.in_psi; Q.psc = 1.0; Q.cin = I.in_psi;
-    Q.cz = Q.cd = Q.cg = 0.0; Q.use_psi = 0; Q.t = 0.0; Q.fp32 = 0;
+    Q.cz = Q.cd = Q.cg = 0.0; Q.use_psi = 0; Q.t = 0.0;
   }
   __syncthreads();
   if (I.prog == kProgEnergy) {
