@@ -34,9 +34,9 @@ def energy_components(p, G, beta2, beta3, Omega, G_C):
     t = _lib.EnergyTerms()
     _lib.check(_lib.lib().bgp_energy(plan.handle, 0, _lib.ptr(p), _lib.ptr(phi) if kern else None,
                                      ctypes.byref(t), _lib.stream_ptr()), "bgp_energy")
-    names = ("E", "Ekin", "Etrap", "Econtact", "Ethree", "Erot", "Egrav", "Lz")
-    vals = torch.tensor([getattr(t, k) for k in names], dtype=torch.float64).unbind(0)
-    return dict(zip(names, vals), phi=phi)
+    f = lambda v: torch.tensor(v, dtype=torch.float64)
+    return dict(E=f(t.E), Ekin=f(t.Ekin), Etrap=f(t.Etrap), Econtact=f(t.Econtact),
+                Ethree=f(t.Ethree), Erot=f(t.Erot), Egrav=f(t.Egrav), Lz=f(t.Lz), phi=phi)
 
 
 def energy_t(p, G, beta2, beta3, Omega, G_C):
@@ -87,13 +87,16 @@ class HamiltonianBatch:
             self._groups.setdefault(s, []).append(i)
 
     def _outputs(self, psis):
-        """One output per state: the fields of one shape are slices of one allocation."""
+        """One output per state: the fields of one shape are parts of one allocation (64
+        allocations take longer than the device's part of the call). unsafe_split: to
+        autograd each output is a tensor of its own, not a view of the block, so writing
+        one of them in place neither marks the others as written nor ties their gradients."""
         if any(tuple(p.shape) != s for p, s in zip(psis, self._shapes)):
             return [torch.empty_like(p) for p in psis]
         outs = [None] * self.n
         for s, idx in self._groups.items():
-            block = torch.empty((len(idx),) + s, dtype=torch.complex128, device=psis[idx[0]].device)
-            for i, o in zip(idx, block.unbind(0)):
+            block = torch.empty((len(idx) * s[0],) + s[1:], dtype=torch.complex128, device=psis[idx[0]].device)
+            for i, o in zip(idx, torch.unsafe_split(block, s[0], 0)):
                 outs[i] = o
         return outs
 
