@@ -50,15 +50,12 @@ BGP_NS_BEGIN
 
 enum SvState : int { ST_INIT, ST_TRIAL, ST_FINAL, ST_SWITCH, ST_CONV, ST_POLYB, ST_POLYC, ST_H, ST_MED, ST_PRE, ST_DONE };
 enum SvKind : int { KD_ITER, KD_INIT, KD_FINAL, KD_SWITCH };   // what the energy and gradient under way are for
-#ifndef SV_BIG
-#define SV_BIG 512
-#endif
 // Configurations of the solver passes (tile width, factorization), by the size of a group
 // of instances: see sv_step in bgp_api.cu.
 // Resident CTAs per SM their registers are budgeted for: one where a tile has an SM to
 // itself (V = 2), else 384 threads in tiles of 4 lines and 512 in tiles of 8.
 BGP_HD constexpr int sv_blocks(int L, int C, int V) {
-  const int b = (C == 8 ? SV_BIG : 384) / s_threads(L, C, V);
+  const int b = (C == 8 ? 512 : 384) / s_threads(L, C, V);
   return (b < 1 || (V == 2 && C < 8)) ? 1 : (b > 16 ? 16 : b);
 }
 constexpr int kSvSmall = 4;                          // lines per tile on a grid too small to fill the GPU

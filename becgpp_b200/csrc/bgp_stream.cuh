@@ -253,6 +253,17 @@ __global__ void __launch_bounds__(s_threads(N, C, V), s_min_blocks(N, C, V))
 // A real line of M points is one complex transform of N: z_n = x_2n + i x_(2n+1), and
 //   X_k = E_k + w_M^k O_k,  E_k = (Z_k + conj Z_(N-k)) / 2,  O_k = (Z_k - conj Z_(N-k)) / 2i.
 
+// two neighbouring values of a caller's field of doubles: one access where the field
+// starts on 16 bytes (a contiguous slice of a larger array need not)
+BGP_D bool on16(const double* p) { return ((size_t)p & 15) == 0; }
+BGP_D double2 load_pair(const double* p, bool wide) {
+  return wide ? __ldg(reinterpret_cast<const double2*>(p)) : cmk(__ldg(p), __ldg(p + 1));
+}
+BGP_D void store_pair(double* p, double2 v, bool wide) {
+  if (wide) *reinterpret_cast<double2*>(p) = v;
+  else { p[0] = v.x; p[1] = v.y; }
+}
+
 // step a (INV = 0) and the last step (INV = 1)
 template <int N, int C, int V, int INV, int NB>
 __global__ void __launch_bounds__(s_threads(N, C, V), s_min_blocks(N, C, V))
@@ -272,14 +283,14 @@ __global__ void __launch_bounds__(s_threads(N, C, V), s_min_blocks(N, C, V))
   pdl_trigger();
   if (INV == 0) {
     const double2* __restrict__ psi = I.psi + (size_t)line * N;
-    const double2* __restrict__ rho = reinterpret_cast<const double2*>(I.rho + (size_t)line * N);
-    const bool given = I.rho != nullptr;
+    const double* __restrict__ rho = I.rho + (size_t)line * N;
+    const bool given = I.rho != nullptr, wide = on16(I.rho);
 #pragma unroll
     for (int q = 0; q < E / 2; ++q) {
       const int n = t + T * q;
       v[q] = cmk(0.0, 0.0);
       if (valid) {
-        if (given) v[q] = __ldg(rho + n);
+        if (given) v[q] = load_pair(rho + 2 * n, wide);
         else v[q] = cmk(cabs2(__ldg(psi + 2 * n)), cabs2(__ldg(psi + 2 * n + 1)));
       }
     }
@@ -317,13 +328,13 @@ __global__ void __launch_bounds__(s_threads(N, C, V), s_min_blocks(N, C, V))
       v[q] = cmk(e.x - o.y, e.y + o.x);                  // e + i o
     }
     fft.template inverse<true>(v);
-    double2* out = reinterpret_cast<double2*>(I.phi_out + (size_t)line * N);
-    const bool store = valid && I.phi_out != nullptr;
+    double* out = I.phi_out + (size_t)line * N;
+    const bool store = valid && I.phi_out != nullptr, wide = on16(I.phi_out);
     const double sc = I.conv_scale;
 #pragma unroll
     for (int q = 0; q < E / 2; ++q) {
       v[q] = cscale(v[q], sc);
-      if (store) out[t + T * q] = v[q];
+      if (store) store_pair(out + 2 * (t + T * q), v[q], wide);
     }
     if (I.gpart) {
       // the tile's part of sum phi |psi|^2

@@ -36,7 +36,7 @@ struct TfArgs {
   double dx, dv, tc, s, Omega, b2, b3, gc, relax;
   const double* conv;            // dV (K * n) of the current n (mode 1), else null
   double* nf;                    // density: current n in, new n out
-  double* part;                  // 2 x 4 x gridDim.x partial sums
+  double* part;                  // 2 x 8 x gridDim.x partial sums
   unsigned long long* bar;       // team barrier counter
   int* abort_flag;               // status word (4 + gridDim.x ints)
   double* state;                 // out: [0] mu, [1] dn, [2] status, [3] converged, [4] steps taken
