@@ -118,6 +118,60 @@ struct DevCtx {
 std::mutex g_mu;
 std::map<int, DevCtx> g_dev;
 
+// Host memory that the device writes (mapped, pinned): one block of kPinSlots slots per
+// device for the process, because pinning takes 3 ms and creating a small plan 0.07 ms.
+// A plan takes a slot and gives it back when it is destroyed; when all slots are taken,
+// and for more than kPinBytes, the memory is the caller's own.
+constexpr int kPinSlots = 256, kPinBytes = 512;
+struct Pinned {
+  char *host = nullptr, *dev = nullptr;
+  int device = -1, slot = -1;             // slot -1: an allocation of its own
+};
+struct PinBlock {
+  char *host = nullptr, *dev = nullptr;
+  std::vector<int> free;
+};
+std::mutex g_pin_mu;
+std::map<int, PinBlock> g_pin;
+
+bool pin_alloc(size_t bytes, char** host, char** dev) {
+  if (cudaHostAlloc((void**)host, bytes, cudaHostAllocMapped) != cudaSuccess) { *host = nullptr; return false; }
+  if (cudaHostGetDevicePointer((void**)dev, *host, 0) == cudaSuccess) return true;
+  cudaFreeHost(*host);
+  *host = nullptr;
+  return false;
+}
+// memory on the current device `device`
+bool pin_take(int device, size_t bytes, Pinned* P) {
+  if (bytes <= kPinBytes) {
+    std::lock_guard<std::mutex> lk(g_pin_mu);
+    PinBlock& B = g_pin[device];
+    if (!B.host && pin_alloc((size_t)kPinSlots * kPinBytes, &B.host, &B.dev))
+      for (int k = kPinSlots - 1; k >= 0; --k) B.free.push_back(k);
+    if (!B.free.empty()) {
+      P->slot = B.free.back();
+      B.free.pop_back();
+      P->device = device;
+      P->host = B.host + (size_t)P->slot * kPinBytes;
+      P->dev = B.dev + (size_t)P->slot * kPinBytes;
+      return true;
+    }
+  }
+  P->slot = -1;
+  return pin_alloc(bytes, &P->host, &P->dev);
+}
+// once no work that writes it is left
+void pin_give(Pinned* P) {
+  if (!P->host) return;
+  if (P->slot >= 0) {
+    std::lock_guard<std::mutex> lk(g_pin_mu);
+    g_pin[P->device].free.push_back(P->slot);
+  } else {
+    cudaFreeHost(P->host);
+  }
+  *P = Pinned();
+}
+
 int ensure_device(DevCtx** out) {
   int dev = 0;
   CK(cudaGetDevice(&dev));
@@ -218,6 +272,7 @@ struct bgp_plan {
   int* d_act = nullptr;                   // active instances, group by group
   int *h_state = nullptr, *d_state = nullptr; // instances' solver states (mapped host memory)
   std::vector<cudaEvent_t> sv_ev;         // two per size group
+  Pinned pin_sums, pin_state;
   double* h_sums = nullptr;               // totals on the host (mapped: the device writes them)
   double* d_sums = nullptr;               // the same memory as the device sees it
   int max_team = 0;
@@ -592,9 +647,10 @@ int bgp_plan_create(const bgp_instance_desc* desc, int n_inst, bgp_plan** plan) 
     p->part_conv = std::max(p->part_conv, std::max(lines / 2, (size_t)kResidBlocks));
   }
   if ((rc = palloc_t(p, p->part_energy + 2 * p->part_conv, &p->d_part))) return bail(rc);
-  if (cudaHostAlloc((void**)&p->h_sums, sizeof(double) * SumArgs::kMax, cudaHostAllocMapped) != cudaSuccess ||
-      cudaHostGetDevicePointer((void**)&p->d_sums, p->h_sums, 0) != cudaSuccess)
+  if (!pin_take(dev->device, sizeof(double) * SumArgs::kMax, &p->pin_sums))
     return bail(fail(BGP_ERR_OOM, "pinned host memory for the operators' sums"));
+  p->h_sums = (double*)p->pin_sums.host;
+  p->d_sums = (double*)p->pin_sums.dev;
   for (int i = 0; i < n_inst; ++i) {
     p->inst[i].out = p->d_out + i;
     p->inst[i].res = p->d_res + (size_t)i * (kNRec + 1);
@@ -615,8 +671,8 @@ int bgp_plan_destroy(bgp_plan* p) {
   for (cudaEvent_t q : p->ovl_ev) cudaEventDestroy(q);
   for (cudaEvent_t q : p->side_ev) cudaEventDestroy(q);
   for (void* q : p->allocs) cudaFree(q);
-  if (p->h_sums) cudaFreeHost(p->h_sums);
-  if (p->h_state) cudaFreeHost(p->h_state);
+  pin_give(&p->pin_sums);                 // (the frees above have waited for the plan's work)
+  pin_give(&p->pin_state);
   for (cudaEvent_t q : p->sv_ev) cudaEventDestroy(q);
   delete p;
   return BGP_OK;
@@ -1570,8 +1626,7 @@ int sv_step(bgp_plan* p, const SvGroup& g, bool chained, unsigned want = ~0u) {
 }
 
 // the stream solver's state of a plan, allocated by its first mixed solve
-int sv_prepare(bgp_plan* p) {
-  if (p->d_sv) return BGP_OK;
+int sv_alloc(bgp_plan* p) {
   const int n = (int)p->inst.size();
   int rc = BGP_OK;
   if ((rc = palloc_t(p, (size_t)n, &p->d_sv))) return rc;
@@ -1586,10 +1641,25 @@ int sv_prepare(bgp_plan* p) {
     if ((rc = palloc_t(p, (size_t)kDSums * (I.n / I.N / kSvSmall), &q))) return rc;
     p->svpart.push_back(q);
   }
-  if (cudaHostAlloc((void**)&p->h_state, sizeof(int) * n, cudaHostAllocMapped) != cudaSuccess ||
-      cudaHostGetDevicePointer((void**)&p->d_state, p->h_state, 0) != cudaSuccess)
+  if (!pin_take(p->dev->device, sizeof(int) * n, &p->pin_state))
     return fail(BGP_ERR_OOM, "pinned host memory for the solver's flags");
+  p->h_state = (int*)p->pin_state.host;
+  p->d_state = (int*)p->pin_state.dev;
   return BGP_OK;
+}
+int sv_prepare(bgp_plan* p) {
+  if (p->h_state) return BGP_OK;
+  const size_t had = p->allocs.size();
+  const long long bytes = p->bytes;
+  const int rc = sv_alloc(p);
+  if (rc) {                               // all or nothing: the next solve starts over
+    for (size_t k = had; k < p->allocs.size(); ++k) cudaFree(p->allocs[k]);
+    p->allocs.resize(had);
+    p->bytes = bytes;
+    p->svpart.clear();
+    p->d_sv = nullptr;
+  }
+  return rc;
 }
 
 // All instances of the plan in the mixed form: results in p->d_out once the stream's work
