@@ -1020,6 +1020,7 @@ int side_stream(bgp_plan* p, int g, cudaStream_t* out) {
 
 // stream descriptor of an instance (the caller sets psi, H and phi)
 void stream_inst(const bgp_plan* p, const Inst& I, SInst& S) {
+  S = SInst{};                  // no given density, no partial sums (launch blocks start undefined)
   S.ndim = I.ndim; S.N = I.N; S.n = I.n; S.M = I.M; S.Mh = I.Mh; S.i0 = I.i0;
   S.dx = I.dx; S.kfac = I.kfac; S.s = I.s; S.tc = I.tc; S.beta2 = I.beta2; S.beta3 = I.beta3;
   S.Omega = I.Omega; S.dv = I.dv;
