@@ -1456,6 +1456,25 @@ int tf_launch(void* kern, int grid, void** args, bgp_plan* p, const Inst& I, cud
   p->launches++;
   return BGP_OK;
 }
+// CTAs of the cluster that takes a Thomas-Fermi step of n points, 0 for the grid-wide
+// launch. ms of 25 steps with the convolutions, cluster / grid: without a square root in
+// the root (b3 = 0) 64^2 2.7 / 3.9, 128^2 3.4 / 4.3, 192^2 3.9 / 4.5, 256^2 4.6 / 4.7, 64^3
+// 22 / 7.9; with one 64^2 3.6 / 5.9, 128^2 5.2 / 7.6, 256^2 11.4 / 7.7 (16 SMs' FP64 units).
+int tf_cluster(int n, double b3) {
+  if (n > kTfClMax * kTfClThreads * (b3 > 1e-30 ? 2 : kTfClHold)) return 0;
+  return std::min(kTfClMax, (n + kTfClThreads - 1) / kTfClThreads);
+}
+int tf_launch_cluster(int ctas, TfArgs A, bgp_plan* p, cudaStream_t st) {
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = ctas; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
+  cfg.gridDim = dim3(ctas); cfg.blockDim = dim3(kTfClThreads); cfg.stream = st;
+  cfg.attrs = &at; cfg.numAttrs = 1;
+  CK(cudaLaunchKernelEx(&cfg, k_tf_iter_cluster, A));
+  p->launches++;
+  return BGP_OK;
+}
 }  // namespace
 
 int bgp_tf_density(bgp_plan* p, int i, int nonlocal, double Omega, int iters, double relax, double* n_out,
@@ -1476,6 +1495,8 @@ int bgp_tf_density(bgp_plan* p, int i, int nonlocal, double Omega, int iters, do
   // address (256^2, 25 steps: 5.8 ms with 4 points a thread, 6.3 with 2, 8.0 with 1)
   grid = std::min(grid, std::max(1, (I.n + kTfHold * kThreads - 1) / (kTfHold * kThreads)));
   if (grid < 1) return fail(BGP_ERR_CUDA, "Thomas-Fermi kernel does not fit on an SM");
+  const int ctas = tf_cluster(I.n, I.beta3);
+  if (ctas > 8) CK(cudaFuncSetAttribute(k_tf_iter_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   double* state = p->d_res + (size_t)i * (kNRec + 1);
   double* conv = I.phi2 + I.n;   // the plan's second potential field as the convolution output
   TfArgs A;
@@ -1489,15 +1510,19 @@ int bgp_tf_density(bgp_plan* p, int i, int nonlocal, double Omega, int iters, do
   auto read_state = [&]() -> int {
     int ab = 0;
     CK(cudaMemcpyAsync(h, state, sizeof(h), cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(&ab, p->d_abort, sizeof(int), cudaMemcpyDeviceToHost, st));
+    if (!ctas) CK(cudaMemcpyAsync(&ab, p->d_abort, sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     if (ab != 0 || h[2] == (double)kTfBarrier) return fail(BGP_ERR_DEVICE, "Thomas-Fermi kernel: team barrier timeout");
     return BGP_OK;
   };
+  auto step = [&]() -> int {
+    if (ctas) return tf_launch_cluster(ctas, A, p, st);
+    void* args[] = {&A};
+    return tf_launch((void*)k_tf_iter, grid, args, p, I, st);
+  };
   CK(cudaMemcpyAsync(state, h, sizeof(h), cudaMemcpyHostToDevice, st));
   if (!nonlocal) {
-    void* args[] = {&A};
-    if ((rc = tf_launch((void*)k_tf_iter, grid, args, p, I, st))) return rc;
+    if ((rc = step())) return rc;
     if ((rc = read_state())) return rc;
   } else {
     const double sigma = 0.15 * (I.dx * I.N / 2.0);   // 0.15 L
@@ -1510,8 +1535,7 @@ int bgp_tf_density(bgp_plan* p, int i, int nonlocal, double Omega, int iters, do
       SLaunchT<1> SL{};
       op_density(p, I, n_out, conv, 0, SL);
       if ((rc = op_conv(p, SL, sched_rule(I), 0, nullptr, nullptr, st))) return rc;
-      void* args[] = {&A};
-      if ((rc = tf_launch((void*)k_tf_iter, grid, args, p, I, st))) return rc;
+      if ((rc = step())) return rc;
       if ((it + 1) % kTfAhead != 0 && it + 1 < iters) continue;
       if ((rc = read_state())) return rc;
       if (h[2] != (double)kTfOk || h[3] != 0.0) break;

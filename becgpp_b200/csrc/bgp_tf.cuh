@@ -6,23 +6,23 @@
 // reference's relaxed fixed point:
 //   base  = V_eff + phi                      (phi = -G_C dV (K * n), from the plan)
 //   mu    : sum_i rho(mu, base_i) dV = 1, by the reference's bracket expansion and
-//           90 bisection halvings, three to a full-grid reduction: the seven points the
-//           next three halvings can reach are summed together and the decisions follow
-//           as in the one-by-one order, bit for bit (a reduction is a grid barrier
-//           of several us, six more sums of a few points per thread a fraction of one;
-//           25 steps at 256^2, with the convolutions: 14.6 ms with 90 reductions of one
-//           sum over 592 CTAs, 5.8 ms with 30 of seven over 128)
+//           90 bisection halvings, three to a reduction: the seven points the next three
+//           halvings can reach are summed together and the decisions follow in the
+//           one-by-one order. A step is a chain of such reductions, bound by their latency:
+//           25 steps at 256^2, with the convolutions, 14.6 ms with 90 reductions of one sum
+//           over 592 CTAs, 5.8 ms with 30 of seven over 128, 4.7 ms with one division per
+//           sum instead of one per point.
 //   n_new = rho(mu, base) / (sum rho dV)
 //   dn    = sum |n_new - n| dV,  n <- (1 - relax) n + relax n_new,  n <- n / (sum n dV)
 // with rho(mu, b) the upper non-negative root of b3 rho^2 + b2 rho = mu - b.
 // The local references (no long-range term) use the same launch once, in mode 0:
 // n = n_new, no relaxation.
 //
-// Work decomposition: all CTAs of the launch form one team (cooperative launch,
-// bounded team barrier); every full-grid sum is a deterministic grid reduction
-// (thread partials in a fixed grid-stride order, warp butterflies, warp totals
-// in order, CTA partials added in CTA order after the barrier), so every CTA
-// holds the same totals and takes the same bisection decisions without a
+// Work decomposition: the CTAs of the launch form one team, either one thread-block
+// cluster (k_tf_iter_cluster) or all resident CTAs of a cooperative launch with a bounded
+// team barrier (k_tf_iter); every sum is deterministic (thread partials in a fixed
+// stride order, warp butterflies, warp totals and CTA partials in fixed orders), so every
+// CTA holds the same totals and takes the same bisection decisions without a
 // broadcast. The arithmetic of V_eff and rho uses round-to-nearest intrinsics
 // (no contraction into FMAs), the operation order of the reference's tensor
 // expressions.
@@ -60,34 +60,18 @@ BGP_D double tf_veff(const TfArgs& A, int f) {
   return __dsub_rn(V, __dmul_rn(c, rp2));
 }
 
-// a / b with r = 1 / b, both rounded to nearest: the quotient q0 = a r is corrected by its
-// exact remainder (Markstein, IBM J. Res. Dev. 34, 1990), which rounds it correctly; the
-// same quotient as a division instruction's, in three operations that overlap with the
-// other candidates'. (One thread's 28 divisions were half of a reduction of the bisection.)
-BGP_HD double tf_quotient(double a, double b, double r) {
-  const double q = a * r;
-  return fma(fma(-q, b, a), r, q);
-}
-// the density's coefficients and the reciprocals its roots divide by
-struct TfRoot {
-  double b2, b3, r2, r3;       // r2 = 1 / b2, r3 = 1 / (2 b3) where they are used
-};
-BGP_HD TfRoot tf_root(double b2, double b3) {
-  return TfRoot{b2, b3, fabs(b2) > 1e-30 ? 1.0 / b2 : 0.0, b3 > 1e-30 ? 1.0 / (2.0 * b3) : 0.0};
-}
-
 // Upper physical root rho >= 0 of b3 rho^2 + b2 rho = mu - b, zero where there is
 // no real root (becgpp/thomasfermi.py:33-45).
-BGP_D double tf_rho(double mu, double b, const TfRoot& P) {
+BGP_D double tf_rho(double mu, double b, double b2, double b3) {
   const double rhs = __dsub_rn(mu, b);
-  if (P.b3 > 1e-30) {
-    const double disc = __dadd_rn(__dmul_rn(P.b2, P.b2), __dmul_rn(4.0 * P.b3, rhs));
+  if (b3 > 1e-30) {
+    const double disc = __dadd_rn(__dmul_rn(b2, b2), __dmul_rn(4.0 * b3, rhs));
     if (!(disc > 0.0)) return 0.0;
-    const double root = tf_quotient(__dadd_rn(-P.b2, sqrt(disc)), 2.0 * P.b3, P.r3);
+    const double root = __ddiv_rn(__dadd_rn(-b2, sqrt(disc)), 2.0 * b3);
     return root > 0.0 ? root : 0.0;
   }
-  if (fabs(P.b2) > 1e-30) {
-    const double q = tf_quotient(rhs, P.b2, P.r2);
+  if (fabs(b2) > 1e-30) {
+    const double q = __ddiv_rn(rhs, b2);
     return q > 0.0 ? q : 0.0;
   }
   return 0.0;
@@ -96,7 +80,7 @@ BGP_D double tf_rho(double mu, double b, const TfRoot& P) {
 #if defined(__CUDACC__)
 
 constexpr int kTfSums = 7;               // most values of one reduction
-constexpr int kTfHold = 4;               // base values a thread keeps in registers
+constexpr int kTfHold = 4;               // base values a thread keeps in registers (grid)
 
 // Deterministic grid-wide reduction of NV values per thread (op: 0 sum, 1 min,
 // 2 max), identical totals in every CTA. sm: kTfSums * (kWarps + 1) doubles. The
@@ -169,29 +153,121 @@ BGP_D bool grid_reduce(double (&v)[NV], const int (&op)[NV], double* part, int& 
   return true;
 }
 
-// One Thomas-Fermi step (see the file comment). Launched cooperatively with every
-// CTA resident; kThreads threads per CTA.
-__global__ void __launch_bounds__(kThreads) k_tf_iter(TfArgs A) {
-  __shared__ double sm[kTfSums * (kWarps + 1)];
-  Team T{(int)blockIdx.x, (int)gridDim.x, A.bar, A.abort_flag};
-  // a step after the fixed point has converged or failed does nothing (the host enqueues
-  // several steps before it looks)
-  if (ld1(A.state + 2) != (double)kTfOk || ld1(A.state + 3) != 0.0) return;
-  int slot = 0;
-  const int n = A.n;
-  const int first = blockIdx.x * kThreads + threadIdx.x, stride = gridDim.x * kThreads;
+// The team of a cooperative launch: every resident CTA, meeting at a grid barrier.
+struct TfGrid {
+  static constexpr int kHold = kTfHold;
+  Team T;
+  double *part, *sm;
+  int slot;
+  BGP_D int first() const { return blockIdx.x * kThreads + threadIdx.x; }
+  BGP_D int stride() const { return gridDim.x * kThreads; }
+  template <int NV, bool MAX>
+  BGP_D bool reduce(double (&v)[NV]) {
+    int op[NV];
+#pragma unroll
+    for (int q = 0; q < NV; ++q) op[q] = MAX ? 2 : 0;
+    return grid_reduce<NV>(v, op, part, slot, T, sm);
+  }
+};
+
+// The team of one thread-block cluster (up to 16 CTAs of 512 threads): partials go into
+// every CTA's shared memory and the CTAs meet at the cluster's hardware barrier, which
+// costs a fraction of a grid barrier through L2; the price is that 16 SMs do the sums
+// (where that pays: tf_cluster in bgp_api.cu).
+constexpr int kTfClThreads = 512, kTfClWarps = kTfClThreads / 32, kTfClMax = 16, kTfClHold = 8;
+struct TfCluster {
+  static constexpr int kHold = kTfClHold;
+  double *wpart, *buf;           // kTfSums x kTfClWarps; 2 slots x 8 values x kTfClMax CTAs
+  int slot;
+  BGP_D int first() const { return blockIdx.x * kTfClThreads + threadIdx.x; }
+  BGP_D int stride() const { return gridDim.x * kTfClThreads; }
+  static BGP_D void sync() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+  }
+  // Every CTA adds the same partials in the same order. The slots alternate: a CTA writes
+  // a slot again only after the barrier behind which all have read it.
+  template <int NV, bool MAX>
+  BGP_D bool reduce(double (&v)[NV]) {
+    static_assert(NV <= 8 && NV <= kTfClWarps, "more values than a reduction holds");
+    constexpr int P = NV <= 1 ? 1 : (NV <= 2 ? 2 : (NV <= 4 ? 4 : 8));
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, G = gridDim.x;
+    const double none = MAX ? -INFINITY : 0.0;
+    auto comb = [](double a, double b) { return MAX ? fmax(a, b) : a + b; };
+    // warp: halve the values and the lanes that share one together (8 values: 9 exchanges)
+    double x[P];
+#pragma unroll
+    for (int q = 0; q < P; ++q) x[q] = q < NV ? v[q] : none;
+    int q0 = 0, o = 16;
+#pragma unroll
+    for (int half = P / 2; half >= 1; half /= 2) {
+      const bool up = lane & o;
+      if (up) q0 += half;
+#pragma unroll
+      for (int j = 0; j < half; ++j) {
+        const double keep = up ? x[j + half] : x[j], send = up ? x[j] : x[j + half];
+        x[j] = comb(keep, __shfl_xor_sync(0xffffffffu, send, o));
+      }
+      o /= 2;
+    }
+    const int same = 2 * o - 1;                // lane bits that hold the same value
+#pragma unroll
+    for (int k = 16; k > 0; k >>= 1)
+      if (k <= o) x[0] = comb(x[0], __shfl_xor_sync(0xffffffffu, x[0], k));
+    if ((lane & same) == 0 && q0 < NV) wpart[q0 * kTfClWarps + w] = x[0];
+    __syncthreads();
+    // CTA: warp q takes value q and sends it to every CTA
+    if (w < NV) {
+      double y = wpart[w * kTfClWarps + (lane & (kTfClWarps - 1))];
+#pragma unroll
+      for (int k = kTfClWarps / 2; k > 0; k >>= 1) y = comb(y, __shfl_xor_sync(0xffffffffu, y, k));
+      if (lane < G) {
+        const unsigned at = (unsigned)__cvta_generic_to_shared(buf + (slot * 8 + w) * kTfClMax + blockIdx.x);
+        unsigned to;
+        asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(at), "r"(lane));
+        asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(to), "d"(y) : "memory");
+      }
+    }
+    __syncwarp();
+    sync();
+    // every warp adds the CTAs' partials: lane 4 q + j those of CTAs j, j + 4, ...
+    const int q = lane >> 2;
+    double y = none;
+#pragma unroll
+    for (int c = 0; c < kTfClMax / 4; ++c) {
+      const int r = (lane & 3) + 4 * c;
+      if (q < NV && r < G) y = comb(y, buf[(slot * 8 + q) * kTfClMax + r]);
+    }
+    y = comb(y, __shfl_xor_sync(0xffffffffu, y, 1));
+    y = comb(y, __shfl_xor_sync(0xffffffffu, y, 2));
+#pragma unroll
+    for (int u = 0; u < NV; ++u) v[u] = __shfl_sync(0xffffffffu, y, 4 * u);
+    slot ^= 1;
+    return true;
+  }
+};
+
+// One Thomas-Fermi step (see the file comment) by the threads of team R.
+template <class R>
+BGP_D void tf_step(const TfArgs& A, R& team) {
+  constexpr int H = R::kHold;
+  const int n = A.n, first = team.first(), stride = team.stride();
   const double gc = A.gc;
-  const TfRoot root = tf_root(A.b2, A.b3);
+  // rho = d u with d = 2 b3 or |b2| the same for every point, so the masses of the
+  // bisection add u and divide once (a division per point and candidate was half of a
+  // reduction): u = sqrt(b2^2 + 4 b3 (mu - b)) - b2, or sign(b2) (mu - b), where positive
+  const bool quad = A.b3 > 1e-30, lin = !quad && fabs(A.b2) > 1e-30;
+  const double sgn = lin && A.b2 < 0.0 ? -1.0 : 1.0, b22 = A.b2 * A.b2, b34 = 4.0 * A.b3;
+  const double per = quad ? A.dv / (2.0 * A.b3) : (lin ? A.dv / fabs(A.b2) : 0.0);
   auto base = [&](int f) {
     const double v = tf_veff(A, f);
     return A.conv ? __dadd_rn(v, __dmul_rn(-gc, ld1(A.conv + f))) : v;
   };
-  // the thread's base values, kept in registers when they are few
-  const bool held = n <= kTfHold * stride;
-  double hb[kTfHold];
+  // the thread's base values (times sgn), kept in registers when they are few
+  const bool held = n <= H * stride;
+  double hb[H];
   if (held) {
 #pragma unroll
-    for (int u = 0; u < kTfHold; ++u) hb[u] = first + u * stride < n ? base(first + u * stride) : 0.0;
+    for (int u = 0; u < H; ++u) hb[u] = first + u * stride < n ? sgn * base(first + u * stride) : 0.0;
   }
   auto fail = [&](int code) {
     if (blockIdx.x == 0 && threadIdx.x == 0) { A.state[2] = (double)code; A.state[3] = 0.0; A.state[4] += 1.0; }
@@ -199,37 +275,44 @@ __global__ void __launch_bounds__(kThreads) k_tf_iter(TfArgs A) {
   // bracket of mu: [min base, max base + |b2| + |b3| + 1] (becgpp/thomasfermi.py:99-100)
   double lo, hi;
   {
-    double v[2] = {INFINITY, -INFINITY};
-    const int op[2] = {1, 2};
-    for (int f = first; f < n; f += stride) { const double b = base(f); v[0] = fmin(v[0], b); v[1] = fmax(v[1], b); }
-    if (!grid_reduce<2>(v, op, A.part, slot, T, sm)) { fail(kTfBarrier); return; }
-    lo = v[0];
+    double v[2] = {-INFINITY, -INFINITY};        // -min, max
+    for (int f = first; f < n; f += stride) { const double b = base(f); v[0] = fmax(v[0], -b); v[1] = fmax(v[1], b); }
+    if (!team.template reduce<2, true>(v)) { fail(kTfBarrier); return; }
+    lo = -v[0];
     hi = v[1] + fabs(A.b2) + fabs(A.b3) + 1.0;
   }
   // sum rho(mu[q]) dV of NV chemical potentials (q < NV), each summed in point order
   auto masses = [&](auto& mu) {
     constexpr int NV = sizeof(mu) / sizeof(double);
     double v[NV];
-    int op[NV];
 #pragma unroll
-    for (int q = 0; q < NV; ++q) { v[q] = 0.0; op[q] = 0; }
+    for (int q = 0; q < NV; ++q) { v[q] = 0.0; mu[q] *= sgn; }
+    auto add = [&](double b) {                   // b: sgn times the base value
+      if (quad) {
+#pragma unroll
+        for (int q = 0; q < NV; ++q) {
+          const double disc = b22 + b34 * (mu[q] - b);
+          const double u = sqrt(fmax(disc, 0.0)) - A.b2;
+          v[q] += disc > 0.0 && u > 0.0 ? u : 0.0;
+        }
+      } else {
+#pragma unroll
+        for (int q = 0; q < NV; ++q) {
+          const double u = mu[q] - b;
+          if (u > 0.0) v[q] += u;
+        }
+      }
+    };
     if (held) {
 #pragma unroll
-      for (int u = 0; u < kTfHold; ++u)
-        if (first + u * stride < n) {
-#pragma unroll
-          for (int q = 0; q < NV; ++q) v[q] += tf_rho(mu[q], hb[u], root);
-        }
+      for (int u = 0; u < H; ++u)
+        if (first + u * stride < n) add(hb[u]);
     } else {
-      for (int f = first; f < n; f += stride) {
-        const double b = base(f);
-#pragma unroll
-        for (int q = 0; q < NV; ++q) v[q] += tf_rho(mu[q], b, root);
-      }
+      for (int f = first; f < n; f += stride) add(sgn * base(f));
     }
-    if (!grid_reduce<NV>(v, op, A.part, slot, T, sm)) return false;
+    if (!team.template reduce<NV, false>(v)) return false;
 #pragma unroll
-    for (int q = 0; q < NV; ++q) mu[q] = v[q] * A.dv;
+    for (int q = 0; q < NV; ++q) mu[q] = v[q] * per;
     return true;
   };
   auto mass = [&](double mu, double& out) {
@@ -276,21 +359,20 @@ __global__ void __launch_bounds__(kThreads) k_tf_iter(TfArgs A) {
   double dn = 0.0;
   if (A.mode == 0) {
     // local reference: n = rho(mu) / (sum rho dV)
-    for (int f = first; f < n; f += stride) st1(A.nf + f, __ddiv_rn(tf_rho(mu, base(f), root), ssum));
+    for (int f = first; f < n; f += stride) st1(A.nf + f, __ddiv_rn(tf_rho(mu, base(f), A.b2, A.b3), ssum));
   } else {
     // relaxed update and its renormalisation (becgpp/thomasfermi.py:103-110)
     double v[2] = {0.0, 0.0};
-    const int op[2] = {0, 0};
     const double a = 1.0 - A.relax, r = A.relax;
     for (int f = first; f < n; f += stride) {
-      const double nn = __ddiv_rn(tf_rho(mu, base(f), root), ssum);
+      const double nn = __ddiv_rn(tf_rho(mu, base(f), A.b2, A.b3), ssum);
       const double old = ld1(A.nf + f);
       v[0] += fabs(__dsub_rn(nn, old));
       const double upd = __dadd_rn(__dmul_rn(a, old), __dmul_rn(r, nn));
       st1(A.nf + f, upd);
       v[1] += upd;
     }
-    if (!grid_reduce<2>(v, op, A.part, slot, T, sm)) { fail(kTfBarrier); return; }
+    if (!team.template reduce<2, false>(v)) { fail(kTfBarrier); return; }
     dn = v[0] * A.dv;
     const double norm = v[1] * A.dv;
     for (int f = first; f < n; f += stride) st1(A.nf + f, __ddiv_rn(ld1(A.nf + f), norm));
@@ -302,6 +384,26 @@ __global__ void __launch_bounds__(kThreads) k_tf_iter(TfArgs A) {
     A.state[3] = (A.mode == 0 || dn < 1e-9) ? 1.0 : 0.0;
     A.state[4] += 1.0;
   }
+}
+
+// a step after the fixed point has converged or failed does nothing (the host enqueues
+// several steps before it looks)
+BGP_D bool tf_over(const TfArgs& A) { return ld1(A.state + 2) != (double)kTfOk || ld1(A.state + 3) != 0.0; }
+
+// Launched cooperatively with every CTA resident; kThreads threads per CTA.
+__global__ void __launch_bounds__(kThreads) k_tf_iter(TfArgs A) {
+  __shared__ double sm[kTfSums * (kWarps + 1)];
+  if (tf_over(A)) return;
+  TfGrid team{Team{(int)blockIdx.x, (int)gridDim.x, A.bar, A.abort_flag}, A.part, sm, 0};
+  tf_step(A, team);
+}
+// Launched as one cluster of gridDim.x CTAs.
+__global__ void __launch_bounds__(kTfClThreads) k_tf_iter_cluster(TfArgs A) {
+  __shared__ double wpart[kTfSums * kTfClWarps], buf[2 * 8 * kTfClMax];
+  if (tf_over(A)) return;
+  TfCluster team{wpart, buf, 0};
+  TfCluster::sync();             // every CTA has started before the first write to its buf
+  tf_step(A, team);
 }
 
 // Initial density of the fixed point, exp(-r^2 / (2 sigma^2)) with sigma = 0.15 L,
