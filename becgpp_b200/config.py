@@ -8,7 +8,7 @@ becGPP runs here unchanged. Two keys are added for this implementation:
   arithmetic) or ``"mixed"`` (FP32 transforms and bulk with FP64 reductions,
   switching to FP64 iterations once the residual reaches the FP32 floor).
 * ``mixed_switch_res`` -- relative residual below which the mixed form hands
-  over to FP64 transforms (it also hands over at its first failed line search).
+  over to FP64 transforms (it also hands over after three failed line searches).
 * ``batch_team`` -- CTAs per instance in a batched solve; 0 lets the scheduler
   choose.
 """

@@ -3,10 +3,10 @@
 ``ground_state`` keeps the signature and return value of
 becgpp/solvers.py:48-235; the whole iteration (preconditioner with its median
 shift, Polak-Ribiere beta, Barzilai-Borwein step, Armijo search, stop tests,
-lowest-residual iterate) runs in one persistent launch of libbgp with all
-state on the device. ``ground_state_multiseed`` (becgpp/solvers.py:238-263)
+lowest-residual iterate) runs in libbgp with all state on the device: in FP64 as
+one persistent launch, in the mixed form as a chain of short launches. ``ground_state_multiseed`` (becgpp/solvers.py:238-263)
 solves its seeds as one batch; ``BatchSolver`` solves any list of instances
-(grids may differ) in one launch.
+(grids may differ) together.
 """
 import ctypes
 import time
@@ -55,9 +55,8 @@ _c128 = _lib.dev_c128
 
 class BatchSolver:
     """Solve a fixed list of instances together: one plan (scratch and kernel
-    tables built once), one persistent launch sequence per ``solve`` call.
-    With ``autotune`` the first three solves try the relaunch schedules and the
-    later ones use the fastest (``schedule()``).
+    tables built once). With ``autotune`` the first three FP64 solves try the
+    relaunch schedules of the persistent kernel and the later ones use the fastest (``schedule()``).
 
     cfgs: config dicts (physics and grid may differ between instances; the
     solver keys must agree). grids: matching grid dictionaries (default

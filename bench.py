@@ -2,7 +2,7 @@
 
 Workload (default ``c4``): the batched cubic-quintic droplet sweep, 64
 instances (beta2 in linspace(-400,-50,16) x 4 seeds, beta3 = 1e3, L = 20, grids
-128^2 and 256^2) solved together in one persistent launch sequence. A ground
+128^2 and 256^2) solved together in one batched call. A ground
 state counts when the reference's own run of that instance converged
 (resid_rel <= 1e-6) and our returned state's energy agrees with it to
 |dE/E| <= 1e-10; the reference energies are the committed fixture
@@ -33,12 +33,13 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 E_TOL = 1e-10
-# DRAM bytes per algorithmic byte of the solver, per precision, from one ncu capture
-# of `bench.py --case small-solve --instances 8 --maxit 200 [--precision fp64]`
-# (dram__bytes_read.sum + dram__bytes_write.sum of all its solver launches / its
-# algorithmic bytes): the working set lives in L2, so only a fifth to a quarter of
-# the algorithmic bytes reach DRAM.
-TRAFFIC_PER_ALGO_BYTE = {"fp64": 0.239, "mixed": 0.178}
+# DRAM bytes per algorithmic byte of the solver, per precision, from ncu captures of all
+# solver launches of a small solve (dram__bytes_read.sum + dram__bytes_write.sum / its
+# algorithmic bytes): `bench.py --case small-solve --instances 8 --maxit 200 --precision
+# fp64`, and for the mixed form, thousands of short launches, `--maxit 40` with the caches
+# kept between launches. The working set lives in L2, so a small part of the algorithmic
+# bytes reaches DRAM.
+TRAFFIC_PER_ALGO_BYTE = {"fp64": 0.239, "mixed": 0.030}
 ORACLE_RESID_MAX = 1e-6
 METRIC = "ground states/s at |dE/E|<=1e-10 (batched solve)"
 
@@ -856,7 +857,7 @@ def run_ours(a):
         e2e_c += _counts(names, energies.tolist(), ref)[0]
     e2e_value = job_rate(sum(e2e_t), e2e_c, dist, "cuda")[2]
 
-    # roofline of the solver kernel (one persistent launch per step)
+    # roofline of the solver's kernels
     peaks = {}
     try:
         peaks = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json")))

@@ -115,12 +115,12 @@ int bgp_plan_create(const bgp_instance_desc* desc, int n_inst, bgp_plan** plan);
 int bgp_plan_destroy(bgp_plan* plan);
 /* Device bytes held by the plan. */
 long long bgp_plan_bytes(const bgp_plan* plan);
-/* Solver-kernel launches issued through the plan so far (a solve relaunches
- * its unfinished instances with larger teams as others finish). */
+/* Kernel launches of the operators and solves issued through the plan so far. */
 long long bgp_plan_launches(const bgp_plan* plan);
 
 /* Relaunch-schedule autotuner of bgp_solve (no counterpart in the reference).
- * A batched solve is a sequence of persistent launches: a launch yields once a
+ * A batched FP64 solve is a sequence of persistent launches (the mixed form is a chain
+ * of short launches and has no such schedule): a launch yields once a
  * fraction 1/d of its instances has finished and the rest are relaunched with
  * larger teams. With enable = 1 the next three batched solves of the plan try
  * d = 2, 4 and 8 in turn, timed on the device, and later solves use the fastest
@@ -207,7 +207,8 @@ int bgp_precondition(bgp_plan* plan, int inst, const void* grad, const void* psi
                      const double* phi, double shift_min, void* z, double* sigma_out,
                      void* stream);
 
-/* Solve every instance of the plan in one persistent launch. psi0[i] and
+/* Solve every instance of the plan: in FP64 as persistent launches, in the mixed form as
+ * a chain of short launches whose control is on the device. psi0[i] and
  * psi_out[i] are device pointers (may be equal). trace (nullable, host) gets
  * trace_cap x 3 doubles per instance: (iteration, E, resid_rel). */
 int bgp_solve(bgp_plan* plan, const void* const* psi0, void* const* psi_out,
