@@ -1458,8 +1458,9 @@ int tf_launch(void* kern, int grid, void** args, bgp_plan* p, const Inst& I, cud
 }
 // CTAs of the cluster that takes a Thomas-Fermi step of n points, 0 for the grid-wide
 // launch. ms of 25 steps with the convolutions, cluster / grid: without a square root in
-// the root (b3 = 0) 64^2 2.7 / 3.9, 128^2 3.4 / 4.3, 192^2 3.9 / 4.5, 256^2 4.6 / 4.7, 64^3
-// 22 / 7.9; with one 64^2 3.6 / 5.9, 128^2 5.2 / 7.6, 256^2 11.4 / 7.7 (16 SMs' FP64 units).
+// the root (b3 = 0) 64^2 2.3 / 3.5, 128^2 2.8 / 3.5, 192^2 3.1 / 3.8, 256^2 about equal (3.5,
+// on 16 SMs instead of 128), beyond it the grid; with one 64^2 2.9 / 4.7, 128^2 4.0 / 6.5,
+// 256^2 8.3 / 6.1 (the FP64 units of 16 SMs).
 int tf_cluster(int n, double b3) {
   if (n > kTfClMax * kTfClThreads * (b3 > 1e-30 ? 2 : kTfClHold)) return 0;
   return std::min(kTfClMax, (n + kTfClThreads - 1) / kTfClThreads);
