@@ -100,15 +100,27 @@ class HamiltonianBatch:
                 outs[i] = o
         return outs
 
+    def _one_each(self, what, fields):
+        # the library reads n addresses of each list, whatever its length
+        if len(fields) != self.n:
+            raise ValueError(f"{what}: {len(fields)} fields for {self.n} instances")
+
     def apply(self, psis, out=None, phis=None, mu=None):
         """out[i] = H psis[i]. phis: None (potential computed from |psi|^2 where
         the kernel is on) or a list of potentials; mu: optional device float64
-        tensor of n entries receiving Re<psi, H psi> dV."""
+        tensor of n entries receiving Re<psi, H psi> dV. Every list has one
+        entry per instance (ValueError otherwise, before anything is launched)."""
+        psis = list(psis)
+        self._one_each("psis", psis)
         psis = [_dev_c128(p) for p in psis]
         outs = out if out is not None else self._outputs(psis)
         address = lambda ts: array.array("Q", [t.data_ptr() for t in ts])
         a_psi, a_out = address(psis), address(outs)
-        a_phi = address(phis) if phis is not None else None
+        self._one_each("out", a_out)
+        a_phi = None
+        if phis is not None:
+            a_phi = address(phis)
+            self._one_each("phis", a_phi)
         _lib.check(_lib.lib().bgp_apply_H_batch(self.plan.handle, self.n, self._idx, a_psi.buffer_info()[0],
                                                 a_out.buffer_info()[0],
                                                 a_phi.buffer_info()[0] if a_phi is not None else None,
