@@ -81,24 +81,6 @@ class HamiltonianBatch:
         self.plan = Plan([instance_desc(G, c) for G, c in zip(self.grids, self.cfgs)])
         self.n = len(self.cfgs)
         self._idx = (ctypes.c_int * self.n)(*range(self.n))
-        self._shapes = [(int(G["N"]),) * int(G["ndim"]) for G in self.grids]
-        self._groups = {}                 # field shape -> instances
-        for i, s in enumerate(self._shapes):
-            self._groups.setdefault(s, []).append(i)
-
-    def _outputs(self, psis):
-        """One output per state: the fields of one shape are parts of one allocation (64
-        allocations take longer than the device's part of the call). unsafe_split: to
-        autograd each output is a tensor of its own, not a view of the block, so writing
-        one of them in place neither marks the others as written nor ties their gradients."""
-        if any(tuple(p.shape) != s for p, s in zip(psis, self._shapes)):
-            return [torch.empty_like(p) for p in psis]
-        outs = [None] * self.n
-        for s, idx in self._groups.items():
-            block = torch.empty((len(idx) * s[0],) + s[1:], dtype=torch.complex128, device=psis[idx[0]].device)
-            for i, o in zip(idx, torch.unsafe_split(block, s[0], 0)):
-                outs[i] = o
-        return outs
 
     def _one_each(self, what, fields):
         # the library reads n addresses of each list, whatever its length
@@ -113,7 +95,8 @@ class HamiltonianBatch:
         psis = list(psis)
         self._one_each("psis", psis)
         psis = [_dev_c128(p) for p in psis]
-        outs = out if out is not None else self._outputs(psis)
+        # an output each: parts of one allocation would keep one another's memory alive
+        outs = out if out is not None else [torch.empty_like(p) for p in psis]
         address = lambda ts: array.array("Q", [t.data_ptr() for t in ts])
         a_psi, a_out = address(psis), address(outs)
         self._one_each("out", a_out)

@@ -53,3 +53,15 @@ def test_batch_lists_of_the_right_length_reach_the_library(batch):
     out = _fields(3)
     assert hb.apply(iter(_fields(3)), out=out, phis=_fields(3, torch.float64)) is out
     assert [name for name, _ in rec.calls] == ["bgp_apply_H_batch"]
+
+
+def test_batch_outputs_own_their_storage(batch):
+    hb, _ = batch
+    outs = hb.apply(_fields(3))
+    for k, o in enumerate(outs):
+        o.fill_(k + 1.0)
+    assert len({o.untyped_storage().data_ptr() for o in outs}) == 3
+    assert [o.untyped_storage().nbytes() for o in outs] == [16 * 16 * 16] * 3
+    outs[0].resize_(64, 64).fill_(9.0)           # grows its own storage only
+    assert torch.equal(outs[1], torch.full((16, 16), 2.0, dtype=torch.complex128))
+    assert torch.equal(outs[2], torch.full((16, 16), 3.0, dtype=torch.complex128))
