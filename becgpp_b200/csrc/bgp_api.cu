@@ -247,10 +247,19 @@ int lf_tables(DevCtx* d, int L) {
 
 }  // namespace
 
+// An instance's line-transform tables by factorization. The plan holds them from its
+// creation on: the maps of DevCtx are shared by all plans of a device and grow under g_mu
+// while other threads apply and solve.
+struct LineTables {
+  const double2 *N[kLVariants] = {}, *M[kLVariants] = {};   // of its N- and M-lines
+  const float2* F[kLVariants] = {};                         // N in FP32
+};
+
 struct bgp_plan {
   DevCtx* dev = nullptr;
   std::vector<bgp_instance_desc> desc;
   std::vector<Inst> inst;                 // host copies with device pointers
+  std::vector<LineTables> lines;
   std::vector<void*> allocs;
   long long bytes = 0;
   Inst* d_inst = nullptr;
@@ -554,6 +563,7 @@ int bgp_plan_create(const bgp_instance_desc* desc, int n_inst, bgp_plan** plan) 
   p->dev = dev;
   p->desc.assign(desc, desc + n_inst);
   p->inst.resize(n_inst);
+  p->lines.resize(n_inst);
   auto bail = [&](int code) { bgp_plan_destroy(p); return code; };
   // first pass: sizes
   for (int i = 0; i < n_inst; ++i) {
@@ -603,6 +613,11 @@ int bgp_plan_create(const bgp_instance_desc* desc, int n_inst, bgp_plan** plan) 
     if (I.M && (rc = twiddles(dev, I.M, &I.twM))) return bail(rc);
     if ((rc = lf_tables(dev, I.N))) return bail(rc);
     if (I.M && (rc = lf_tables(dev, I.M))) return bail(rc);
+    for (int V = 0; V < kLVariants; ++V) {
+      p->lines[i].N[V] = dev->lf[V][I.N];
+      p->lines[i].F[V] = dev->lf32[V][I.N];
+      if (I.M) p->lines[i].M[V] = dev->lf[V][I.M];
+    }
     if ((rc = palloc_t(p, (size_t)kNB * n, &I.pool))) return bail(rc);
     // potentials: current and trial; 3D with a kernel also the potentials of the
     // density's linear and quadratic parts in the step (the line search's quartic)
@@ -1018,8 +1033,9 @@ int side_stream(bgp_plan* p, int g, cudaStream_t* out) {
   return BGP_OK;
 }
 
-// stream descriptor of an instance (the caller sets psi, H and phi)
-void stream_inst(const bgp_plan* p, const Inst& I, SInst& S) {
+// stream descriptor of instance i (the caller sets psi, H and phi)
+void stream_inst(const bgp_plan* p, int i, SInst& S) {
+  const Inst& I = p->inst[i];
   S = SInst{};                  // no given density, no partial sums (launch blocks start undefined)
   S.ndim = I.ndim; S.N = I.N; S.n = I.n; S.M = I.M; S.Mh = I.Mh; S.i0 = I.i0;
   S.dx = I.dx; S.kfac = I.kfac; S.s = I.s; S.tc = I.tc; S.beta2 = I.beta2; S.beta3 = I.beta3;
@@ -1031,8 +1047,8 @@ void stream_inst(const bgp_plan* p, const Inst& I, SInst& S) {
   S.hscale = 1.0;
   S.twM = I.twM;
   for (int V = 0; V < kLVariants; ++V) {
-    S.tabN[V] = p->dev->lf[V][I.N];
-    S.tabM[V] = I.M ? p->dev->lf[V][I.M] : nullptr;
+    S.tabN[V] = p->lines[i].N[V];
+    S.tabM[V] = p->lines[i].M[V];
   }
 }
 }  // namespace
@@ -1041,15 +1057,16 @@ namespace {
 // ---------------------------------------------- single-instance operators
 // One instance's launch block for the operators: psi as the state (and the density of
 // a convolution).
-void op_init(const bgp_plan* p, const Inst& I, const void* psi, SLaunchT<1>& SL) {
+void op_init(const bgp_plan* p, int i, const void* psi, SLaunchT<1>& SL) {
   SL.ninst = 1;
-  stream_inst(p, I, SL.insts[0]);
+  stream_inst(p, i, SL.insts[0]);
   SL.insts[0].psi = (const double2*)psi;
 }
 
 // The same for the plain convolution out = dV (K * rho) of a given density.
-void op_density(const bgp_plan* p, const Inst& I, const double* rho, double* out, int which_w, SLaunchT<1>& SL) {
-  op_init(p, I, nullptr, SL);
+void op_density(const bgp_plan* p, int i, const double* rho, double* out, int which_w, SLaunchT<1>& SL) {
+  const Inst& I = p->inst[i];
+  op_init(p, i, nullptr, SL);
   SInst& S = SL.insts[0];
   const double Md = (double)I.M;
   S.rho = rho;
@@ -1147,7 +1164,7 @@ int bgp_apply_H(bgp_plan* p, int i, const void* psi, void* hpsi, const double* p
   cudaStream_t st = (cudaStream_t)stream;
   const Sched S = sched_rule(I);
   SLaunchT<1> SL{};
-  op_init(p, I, psi, SL);
+  op_init(p, i, psi, SL);
   if (phi_mode == 2 && has_kernel(I)) {
     if ((rc = op_conv(p, SL, S, 0, nullptr, nullptr, st))) return rc;
     SL.insts[0].phi = I.phi2;
@@ -1172,7 +1189,7 @@ int bgp_energy(bgp_plan* p, int i, const void* psi, double* phi_out, bgp_energy_
   cudaStream_t st = (cudaStream_t)stream;
   const Sched S = sched_rule(I);
   SLaunchT<1> SL{};
-  op_init(p, I, psi, SL);
+  op_init(p, i, psi, SL);
   Sums sums;
   EnergySlots es;
   int grav = -1;
@@ -1198,7 +1215,7 @@ int bgp_energy_grad(bgp_plan* p, int i, const void* psi, bgp_energy_terms* terms
   const Sched S = sched_rule(I);
   const bool kern = has_kernel(I), width = kern && I.kind == kQ2d && I.Wq;
   SLaunchT<1> SL{};
-  op_init(p, I, psi, SL);
+  op_init(p, i, psi, SL);
   Sums sums;
   EnergySlots es;
   int grav = -1, gravW = -1;
@@ -1244,7 +1261,7 @@ int bgp_residual(bgp_plan* p, int i, const void* psi, double* out3, void* stream
   cudaStream_t st = (cudaStream_t)stream;
   const Sched S = sched_rule(I);
   SLaunchT<1> SL{};
-  op_init(p, I, psi, SL);
+  op_init(p, i, psi, SL);
   if (has_kernel(I)) {
     if ((rc = op_conv(p, SL, S, 0, nullptr, nullptr, st))) return rc;
     SL.insts[0].phi = I.phi2;
@@ -1277,7 +1294,7 @@ int bgp_convolve(bgp_plan* p, int i, const double* rho, double* out, int which, 
   if (!rho || !out) return fail(BGP_ERR_ARG, "null pointer");
   cudaStream_t st = (cudaStream_t)stream;
   SLaunchT<1> SL{};
-  op_density(p, I, rho, out, which, SL);
+  op_density(p, i, rho, out, which, SL);
   if ((rc = op_conv(p, SL, sched_rule(I), 0, nullptr, nullptr, st))) return rc;
   CK(cudaStreamSynchronize(st));
   return BGP_OK;
@@ -1358,7 +1375,7 @@ int bgp_apply_H_batch(bgp_plan* p, int n, const int* idx, const void* const* psi
         const int b = grp[g];
         const Inst& I = p->inst[idx[b]];
         SInst& S = SL.insts[g];
-        stream_inst(p, I, S);
+        stream_inst(p, idx[b], S);
         S.psi = (const double2*)psi[b];
         S.H = (double2*)hpsi[b];
         S.phi = conv ? I.phi2 : (phi_mode == 1 ? phi[b] : nullptr);
@@ -1534,7 +1551,7 @@ int bgp_tf_density(bgp_plan* p, int i, int nonlocal, double Omega, int iters, do
     // at once): a wait per step was a tenth of the call, and much more on a busy host
     for (int it = 0; it < iters; ++it) {
       SLaunchT<1> SL{};
-      op_density(p, I, n_out, conv, 0, SL);
+      op_density(p, i, n_out, conv, 0, SL);
       if ((rc = op_conv(p, SL, sched_rule(I), 0, nullptr, nullptr, st))) return rc;
       if ((rc = step())) return rc;
       if ((it + 1) % kTfAhead != 0 && it + 1 < iters) continue;
@@ -1709,9 +1726,9 @@ int sv_solve(bgp_plan* p, const void* const* psi0, void* const* psi_out, const S
     S.beta2 = I.beta2; S.beta3 = I.beta3; S.Omega = I.Omega; S.inv_n = I.inv_n; S.conv_scale = I.conv_scale;
     S.pool = I.pool; S.phi2 = I.phi2; S.cb1 = I.cb1; S.cb2 = I.cb2; S.Kq = I.Kq; S.twM = I.twM;
     for (int V = 0; V < kLVariants; ++V) {
-      S.tabN[V] = p->dev->lf[V][I.N];
-      S.tabF[V] = p->dev->lf32[V][I.N];
-      S.tabM[V] = I.M ? p->dev->lf[V][I.M] : nullptr;
+      S.tabN[V] = p->lines[i].N[V];
+      S.tabF[V] = p->lines[i].F[V];
+      S.tabM[V] = p->lines[i].M[V];
     }
     S.keys = I.keys;
     S.wcand = p->d_svcand + (size_t)i * kSvCap;

@@ -1,0 +1,99 @@
+"""The library's host code (plans, launches, waits, errors) on a machine without a GPU:
+libbgp.so in a process of its own whose CUDA runtime is tests/fake_cudart.cpp, which runs
+no kernel but notes launches, orders the legacy default stream and fails calls on request.
+"""
+import json
+import os
+import re
+import shutil
+import subprocess
+import sys
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+LIB = os.path.join(ROOT, "becgpp_b200", "libbgp.so")
+
+# A process without torch (whose libraries would bring the real runtime): the binding
+# module alone, with a placeholder for torch.
+PRELUDE = r"""
+import ctypes, importlib.util, json, sys, threading, types
+fake = ctypes.CDLL(sys.argv[1])
+fake.fake_count.restype = ctypes.c_longlong
+fake.fake_stream.restype = ctypes.c_void_p
+torch = types.ModuleType("torch"); torch._C = object(); sys.modules["torch"] = torch
+spec = importlib.util.spec_from_file_location("binding", sys.argv[2])
+L = importlib.util.module_from_spec(spec); spec.loader.exec_module(L)
+lib = L.lib()
+count = lambda what: fake.fake_count(what.encode())
+def mallocs():
+    n = fake.fake_mallocs(None, 0)
+    a = (ctypes.c_size_t * n)()
+    fake.fake_mallocs(a, n)
+    return list(a)
+def desc(N=16, ndim=2, kernel="none", beta2=10.0, beta3=0.0):
+    return L.InstanceDesc(ndim, N, 2, L.KERNEL_CODES[kernel], 6.0, 2.0, 0.5, beta2, beta3, 0.0,
+                          5.0 if kernel != "none" else 0.0, 0.0)
+def plan(*descs):
+    h = ctypes.c_void_p()
+    rc = lib.bgp_plan_create((L.InstanceDesc * len(descs))(*descs), len(descs), ctypes.byref(h))
+    return rc, h
+def field(n):
+    return (ctypes.c_double * (2 * n))()
+def solve(h, n, points, stream=None, mixed=1, maxit=1):
+    p = L.SolverParams(maxit, 4, 4, 10, 0, 10, 0, 0, mixed, 1e-8, 1e-12, 0.1, 1.0, 0.1, 1e-3)
+    f = [field(points) for _ in range(n)]
+    P = (ctypes.c_void_p * n)(*[ctypes.addressof(x) for x in f])
+    return lib.bgp_solve(h, P, P, ctypes.byref(p), (L.SolveResult * n)(), None, stream)
+def apply(h, points, stream=None, n=1):
+    f, g = [field(points) for _ in range(n)], [field(points) for _ in range(n)]
+    P = lambda q: (ctypes.c_void_p * n)(*[ctypes.addressof(x) for x in q])
+    return lib.bgp_apply_H_batch(h, n, (ctypes.c_int * n)(*range(n)), P(f), P(g), None, 2, None, stream)
+out = {}
+"""
+
+
+@pytest.fixture(scope="module")
+def run(tmp_path_factory):
+    nvcc = os.environ.get("NVCC", "nvcc")
+    if shutil.which(nvcc) is None or shutil.which("g++") is None:
+        pytest.skip("nvcc or g++ is not on PATH")
+    d = tmp_path_factory.mktemp("fake_runtime")
+    src, obj, so, vmap = os.path.join(ROOT, "tests", "fake_cudart.cpp"), d / "hooks.o", d / "libcudart.so.12", d / "v.map"
+    vmap.write_text("libcudart.so.12 { global: cuda*; __cuda*; fake_*; local: *; };\n")
+    home = os.path.dirname(os.path.dirname(os.path.realpath(shutil.which(nvcc))))
+    subprocess.run([nvcc, "-x", "cu", "-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "-O0", "-w",
+                    "-Xcompiler", "-fPIC", "-I", os.path.join(ROOT, "becgpp_b200", "csrc"), "-c", src, "-o", str(obj)],
+                   check=True)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-w", "-shared", "-fPIC", "-I", os.path.join(home, "include"), src, str(obj),
+                    "-o", str(so), "-Wl,-soname,libcudart.so.12", f"-Wl,--version-script={vmap}"], check=True)
+
+    def go(scenario):
+        r = subprocess.run([sys.executable, "-c", PRELUDE + scenario + "\nprint(json.dumps(out))", str(so),
+                            os.path.join(ROOT, "becgpp_b200", "_lib.py")], capture_output=True, text=True, timeout=300)
+        assert r.returncode == 0, r.stderr
+        return json.loads(r.stdout.splitlines()[-1])
+    return go
+
+
+def test_a_mixed_solve_runs_to_its_end(run):
+    got = run(r"""
+rc, h = plan(desc())
+out["rc"] = rc, solve(h, 1, 256), solve(h, 1, 256, stream=fake.fake_stream())
+out["launches"] = count("k_sv_px")
+lib.bgp_plan_destroy(h)
+""")
+    assert got["rc"] == [0, 0, 0] and got["launches"] > 0
+
+
+def test_only_plan_creation_reads_the_shared_tables():
+    """The maps of a device's tables grow under the creation lock; other threads' calls on
+    other plans hold no lock, so they must not read them."""
+    src = open(os.path.join(ROOT, "becgpp_b200", "csrc", "bgp_api.cu")).read()
+    used, name = set(), None
+    for line in src.splitlines():
+        m = re.match(r"(?:template.*> *)?(?:int|void|bool|const \w+\*|long long|Sched) (\w+)\(", line)
+        name = m.group(1) if m else name
+        if re.search(r"(->|\.)(lf|lf32|tw)\b(\[|\.)", line):
+            used.add(name)
+    assert used == {"twiddles", "lf_table", "bgp_plan_create"}
