@@ -187,6 +187,18 @@ int ensure_device(DevCtx** out) {
   return BGP_OK;
 }
 
+// A table uploaded to device memory of its own.
+template <class T>
+int upload(const std::vector<T>& h, T** out) {
+  T* dp = nullptr;
+  CK(cudaMalloc(&dp, sizeof(T) * h.size()));
+  const cudaError_t e = cudaMemcpy(dp, h.data(), sizeof(T) * h.size(), cudaMemcpyHostToDevice);
+  if (e != cudaSuccess) cudaFree(dp);
+  CK(e);
+  *out = dp;
+  return BGP_OK;
+}
+
 // exp(-2 pi i t / L), t = 0..L-1, from long-double sin/cos of the reduced angle
 int twiddles(DevCtx* d, int L, const double2** out) {
   auto it = d->tw.find(L);
@@ -206,14 +218,15 @@ int twiddles(DevCtx* d, int L, const double2** out) {
     h[t] = cmk((double)c, -(double)s);
   }
   double2* dp = nullptr;
-  CK(cudaMalloc(&dp, sizeof(double2) * L));
-  CK(cudaMemcpy(dp, h.data(), sizeof(double2) * L, cudaMemcpyHostToDevice));
+  int rc = upload(h, &dp);
+  if (rc) return rc;
   d->tw[L] = dp;
   *out = dp;
   return BGP_OK;
 }
 
-// stage twiddles of the stream passes' line transform of length L, variant V
+// stage twiddles of the stream passes' line transform of length L, variant V, in FP64 and
+// rounded to FP32: both or neither
 template <int L, int V>
 int lf_table(DevCtx* d) {
   if (d->lf[V].count(L)) return BGP_OK;
@@ -224,15 +237,13 @@ int lf_table(DevCtx* d) {
   if (rc) return rc;
   CK(cudaMemcpy(w.data(), dw, sizeof(double2) * L, cudaMemcpyDeviceToHost));
   lf_fill_table<L, V>(w.data(), tab.data());
-  double2* dp = nullptr;
-  CK(cudaMalloc(&dp, sizeof(double2) * len));
-  CK(cudaMemcpy(dp, tab.data(), sizeof(double2) * len, cudaMemcpyHostToDevice));
-  d->lf[V][L] = dp;
   std::vector<float2> tf(len);
   for (int q = 0; q < len; ++q) tf[q] = cmake<float2>((float)tab[q].x, (float)tab[q].y);
+  double2* dp = nullptr;
   float2* fp = nullptr;
-  CK(cudaMalloc(&fp, sizeof(float2) * len));
-  CK(cudaMemcpy(fp, tf.data(), sizeof(float2) * len, cudaMemcpyHostToDevice));
+  if ((rc = upload(tab, &dp))) return rc;
+  if ((rc = upload(tf, &fp))) { cudaFree(dp); return rc; }
+  d->lf[V][L] = dp;
   d->lf32[V][L] = fp;
   return BGP_OK;
 }

@@ -97,3 +97,23 @@ def test_only_plan_creation_reads_the_shared_tables():
         if re.search(r"(->|\.)(lf|lf32|tw)\b(\[|\.)", line):
             used.add(name)
     assert used == {"twiddles", "lf_table", "bgp_plan_create"}
+
+
+@pytest.mark.parametrize("N,kernel", [(16, "none"), (24, "log"), (48, "none")])
+def test_tables_of_a_failed_creation_are_complete_or_absent(run, N, kernel):
+    """Whichever allocations of earlier creations failed, a mixed solve finds every line
+    table, the FP32 ones too."""
+    got = run(f"""
+d = desc({N}, kernel="{kernel}")
+rcs = []
+for k in range(1, 40):
+    fake.fake_fail_malloc(k)
+    rc, h = plan(d)
+    rcs.append(rc)
+    if rc == 0: lib.bgp_plan_destroy(h)
+fake.fake_fail_malloc(0)
+rc, h = plan(d)
+out.update(failed=sum(r != 0 for r in rcs), rc=[rc, solve(h, 1, {N * N})], null=count("null_table"), px=count("k_sv_px"))
+""")
+    assert got["failed"] >= 10 and got["rc"] == [0, 0] and got["px"] > 0
+    assert got["null"] == 0
