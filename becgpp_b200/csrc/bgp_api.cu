@@ -336,6 +336,13 @@ int palloc(bgp_plan* p, size_t bytes, void** out) {
   return BGP_OK;
 }
 
+// Waits until what palloc allocated is zero: it is cleared on the default stream, which
+// non-blocking streams do not wait for (a memset does not hold the host).
+int zeroed() {
+  CK(cudaStreamSynchronize(cudaStreamLegacy));
+  return BGP_OK;
+}
+
 template <class T>
 int palloc_t(bgp_plan* p, size_t count, T** out) {
   void* q = nullptr;
@@ -686,6 +693,7 @@ int bgp_plan_create(const bgp_instance_desc* desc, int n_inst, bgp_plan** plan) 
   if ((rc = palloc_t(p, (size_t)n_inst * kProfSlots, &prof))) return bail(rc);
   for (int i = 0; i < n_inst; ++i) p->inst[i].prof = prof + (size_t)i * kProfSlots;
 #endif
+  if ((rc = zeroed())) return bail(rc);
   *plan = p;
   return BGP_OK;
 }
@@ -1697,6 +1705,7 @@ int sv_alloc(bgp_plan* p) {
   }
   if (!pin_take(p->dev->device, sizeof(int) * n, &p->pin_state))
     return fail(BGP_ERR_OOM, "pinned host memory for the solver's flags");
+  if ((rc = zeroed())) return rc;
   p->h_state = (int*)p->pin_state.host;
   p->d_state = (int*)p->pin_state.dev;
   return BGP_OK;
@@ -1712,6 +1721,7 @@ int sv_prepare(bgp_plan* p) {
     p->bytes = bytes;
     p->svpart.clear();
     p->d_sv = nullptr;
+    pin_give(&p->pin_state);
   }
   return rc;
 }

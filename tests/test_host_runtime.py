@@ -117,3 +117,15 @@ out.update(failed=sum(r != 0 for r in rcs), rc=[rc, solve(h, 1, {N * N})], null=
 """)
     assert got["failed"] >= 10 and got["rc"] == [0, 0] and got["px"] > 0
     assert got["null"] == 0
+
+
+def test_memory_is_cleared_before_another_stream_uses_it(run):
+    """The clearing of a plan's memory, and of the mixed solver's (allocated by its first
+    solve), is over before anything runs on a stream the default stream does not order."""
+    got = run(r"""
+st = fake.fake_stream()
+rc, h = plan(desc())
+out["create"] = rc, apply(h, 256, st), count("unordered")
+out["mixed"] = solve(h, 1, 256, st), count("unordered")
+""")
+    assert got == {"create": [0, 0, 0], "mixed": [0, 0]}
