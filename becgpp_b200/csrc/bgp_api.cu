@@ -1483,10 +1483,10 @@ int bgp_plan_stream_set(bgp_plan* p, int N, int lines, int radix_order, int conv
 }
 
 namespace {
-// Cooperative launch of a Thomas-Fermi kernel over `grid` CTAs (one team).
+// Cooperative launch of a Thomas-Fermi kernel over `grid` CTAs (one team). The status word
+// stays as earlier launches left it: the host looks at it only every few steps.
 int tf_launch(void* kern, int grid, void** args, bgp_plan* p, const Inst& I, cudaStream_t st) {
   CK(cudaMemsetAsync(I.bar, 0, sizeof(unsigned long long), st));
-  CK(cudaMemsetAsync(p->d_abort, 0, (4 + (size_t)grid) * sizeof(int), st));
   CK(cudaLaunchCooperativeKernel(kern, dim3(grid), dim3(kThreads), args, 0, st));
   CK(cudaGetLastError());
   p->launches++;
@@ -1547,7 +1547,7 @@ int bgp_tf_density(bgp_plan* p, int i, int nonlocal, double Omega, int iters, do
   auto read_state = [&]() -> int {
     int ab = 0;
     CK(cudaMemcpyAsync(h, state, sizeof(h), cudaMemcpyDeviceToHost, st));
-    if (!ctas) CK(cudaMemcpyAsync(&ab, p->d_abort, sizeof(int), cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(&ab, p->d_abort, sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     if (ab != 0 || h[2] == (double)kTfBarrier) return fail(BGP_ERR_DEVICE, "Thomas-Fermi kernel: team barrier timeout");
     return BGP_OK;
@@ -1558,6 +1558,7 @@ int bgp_tf_density(bgp_plan* p, int i, int nonlocal, double Omega, int iters, do
     return tf_launch((void*)k_tf_iter, grid, args, p, I, st);
   };
   CK(cudaMemcpyAsync(state, h, sizeof(h), cudaMemcpyHostToDevice, st));
+  CK(cudaMemsetAsync(p->d_abort, 0, (4 + (size_t)grid) * sizeof(int), st));
   if (!nonlocal) {
     if ((rc = step())) return rc;
     if ((rc = read_state())) return rc;

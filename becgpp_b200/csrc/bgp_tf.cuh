@@ -39,7 +39,7 @@ struct TfArgs {
   double* nf;                    // density: current n in, new n out
   double* part;                  // 2 x 8 x gridDim.x partial sums
   unsigned long long* bar;       // team barrier counter
-  int* abort_flag;               // status word (4 + gridDim.x ints)
+  int* abort_flag;               // status word (4 + gridDim.x ints), cleared once per density
   double* state;                 // out: [0] mu, [1] dn, [2] status, [3] converged, [4] steps taken
 };
 
@@ -392,8 +392,11 @@ BGP_D void tf_step(const TfArgs& A, R& team) {
 }
 
 // a step after the fixed point has converged or failed does nothing (the host enqueues
-// several steps before it looks)
-BGP_D bool tf_over(const TfArgs& A) { return ld1(A.state + 2) != (double)kTfOk || ld1(A.state + 3) != 0.0; }
+// several steps before it looks). A barrier that timed out in an earlier launch shows in
+// the status word alone when the first CTA got past it.
+BGP_D bool tf_over(const TfArgs& A) {
+  return *(volatile const int*)A.abort_flag != 0 || ld1(A.state + 2) != (double)kTfOk || ld1(A.state + 3) != 0.0;
+}
 
 // Launched cooperatively with every CTA resident; kThreads threads per CTA.
 __global__ void __launch_bounds__(kThreads) k_tf_iter(TfArgs A) {

@@ -129,3 +129,21 @@ out["create"] = rc, apply(h, 256, st), count("unordered")
 out["mixed"] = solve(h, 1, 256, st), count("unordered")
 """)
     assert got == {"create": [0, 0, 0], "mixed": [0, 0]}
+
+
+@pytest.mark.parametrize("N,beta3,step", [(384, 0.0, 1), (384, 0.0, 7), (256, 5.0, 9), (64, 0.0, 3)])
+def test_a_timed_out_thomas_fermi_barrier_is_reported(run, N, beta3, step):
+    """The status word of a step survives the steps enqueued after it, whichever team takes
+    them (a grid at 384^2 and, with beta3 > 0, at 256^2; a cluster at 64^2, which reads the
+    word that the cooperative seed may have set)."""
+    got = run(f"""
+rc, h = plan(desc({N}, kernel="log", beta3={beta3}))
+n, info = (ctypes.c_double * {N * N})(), (ctypes.c_double * 5)()
+tf = lambda: lib.bgp_tf_density(h, 0, 1, 0.0, 12, 0.3, ctypes.addressof(n), info, None)
+out["fine"] = tf(), info[3]
+fake.fake_tf_timeout({step})
+out["timeout"] = tf(), lib.bgp_last_error().decode()
+out["again"] = tf(), info[3]
+""")
+    assert got["fine"] == got["again"] == [0, 12.0]
+    assert got["timeout"][0] == -4 and "timeout" in got["timeout"][1]
