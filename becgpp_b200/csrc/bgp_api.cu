@@ -1893,7 +1893,7 @@ int bgp_solve(bgp_plan* p, const void* const* psi0, void* const* psi_out, const 
   // so the instances that need the most iterations soon get the whole GPU.
   int rc = BGP_OK;
   std::vector<SolveOut> outs(n);
-  const bool tuning = p->tune == 1 && n > 1;
+  const bool tuning = !P.mixed && p->tune == 1 && n > 1;   // the mixed form has no relaunches
   const int ydiv = tuning ? kTuneYield[p->tune_next] : p->yield_div;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   if (tuning) {

@@ -147,3 +147,20 @@ out["again"] = tf(), info[3]
 """)
     assert got["fine"] == got["again"] == [0, 12.0]
     assert got["timeout"][0] == -4 and "timeout" in got["timeout"][1]
+
+
+def test_mixed_solves_do_not_tune_the_relaunch_schedule(run):
+    """Only FP64 solves are launches that yield; the timing of others says nothing about it."""
+    got = run(r"""
+rc, h = plan(desc(), desc(beta2=20.0))
+def schedule():
+    div, tuned, ms = ctypes.c_int(), ctypes.c_int(), (ctypes.c_float * 3)()
+    assert lib.bgp_plan_schedule(h, ctypes.byref(div), ctypes.byref(tuned), ms) == 0
+    return [div.value, tuned.value, list(ms)]
+lib.bgp_plan_autotune(h, 1)
+before = schedule()
+out["mixed"] = [solve(h, 2, 256) for _ in range(4)], schedule() == before
+out["fp64"] = [solve(h, 2, 256, mixed=0) for _ in range(3)], schedule()[1:]
+""")
+    assert got["mixed"] == [[0] * 4, True]
+    assert got["fp64"] == [[0] * 3, [1, [1.0, 1.0, 1.0]]]
