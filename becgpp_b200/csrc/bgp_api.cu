@@ -1501,14 +1501,31 @@ int tf_cluster(int n, double b3) {
   if (n > kTfClMax * kTfClThreads * (b3 > 1e-30 ? 2 : kTfClHold)) return 0;
   return std::min(kTfClMax, (n + kTfClThreads - 1) / kTfClThreads);
 }
-int tf_launch_cluster(int ctas, TfArgs A, bgp_plan* p, cudaStream_t st) {
+// launch configuration of a Thomas-Fermi step by one cluster
+struct TfClusterLaunch {
   cudaLaunchConfig_t cfg{};
-  cudaLaunchAttribute at;
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = ctas; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
-  cfg.gridDim = dim3(ctas); cfg.blockDim = dim3(kTfClThreads); cfg.stream = st;
-  cfg.attrs = &at; cfg.numAttrs = 1;
-  CK(cudaLaunchKernelEx(&cfg, k_tf_iter_cluster, A));
+  cudaLaunchAttribute at{};
+  TfClusterLaunch(int ctas, cudaStream_t st) {
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = ctas; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
+    cfg.gridDim = dim3(ctas); cfg.blockDim = dim3(kTfClThreads); cfg.stream = st;
+    cfg.attrs = &at; cfg.numAttrs = 1;
+  }
+  TfClusterLaunch(const TfClusterLaunch&) = delete;
+};
+// Whether the device can hold such a cluster: more than 8 CTAs are beyond what every
+// device (or partition of one) schedules; the grid-wide launch takes the step where not.
+bool tf_cluster_fits(int ctas) {
+  const TfClusterLaunch L(ctas, nullptr);
+  int n = 0;
+  const bool ok = (ctas <= 8 || cudaFuncSetAttribute(k_tf_iter_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) &&
+                  cudaOccupancyMaxActiveClusters(&n, k_tf_iter_cluster, &L.cfg) == cudaSuccess;
+  if (!ok) cudaGetLastError();
+  return ok && n > 0;
+}
+int tf_launch_cluster(int ctas, TfArgs A, bgp_plan* p, cudaStream_t st) {
+  const TfClusterLaunch L(ctas, st);
+  CK(cudaLaunchKernelEx(&L.cfg, k_tf_iter_cluster, A));
   p->launches++;
   return BGP_OK;
 }
@@ -1532,8 +1549,8 @@ int bgp_tf_density(bgp_plan* p, int i, int nonlocal, double Omega, int iters, do
   // address (256^2, 25 steps: 5.8 ms with 4 points a thread, 6.3 with 2, 8.0 with 1)
   grid = std::min(grid, std::max(1, (I.n + kTfHold * kThreads - 1) / (kTfHold * kThreads)));
   if (grid < 1) return fail(BGP_ERR_CUDA, "Thomas-Fermi kernel does not fit on an SM");
-  const int ctas = tf_cluster(I.n, I.beta3);
-  if (ctas > 8) CK(cudaFuncSetAttribute(k_tf_iter_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  int ctas = tf_cluster(I.n, I.beta3);
+  if (ctas && !tf_cluster_fits(ctas)) ctas = 0;
   double* state = p->d_res + (size_t)i * (kNRec + 1);
   double* conv = I.phi2 + I.n;   // the plan's second potential field as the convolution output
   TfArgs A;

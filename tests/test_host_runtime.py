@@ -164,3 +164,17 @@ out["fp64"] = [solve(h, 2, 256, mixed=0) for _ in range(3)], schedule()[1:]
 """)
     assert got["mixed"] == [[0] * 4, True]
     assert got["fp64"] == [[0] * 3, [1, [1.0, 1.0, 1.0]]]
+
+
+def test_thomas_fermi_without_room_for_a_cluster(run):
+    """A device (or a partition of one) that cannot hold the cluster takes grid-wide steps."""
+    got = run(r"""
+rc, h = plan(desc(64, kernel="log"))
+n, info = (ctypes.c_double * 4096)(), (ctypes.c_double * 5)()
+tf = lambda: lib.bgp_tf_density(h, 0, 1, 0.0, 5, 0.3, ctypes.addressof(n), info, None)
+for clusters in (1, 0):
+    fake.fake_clusters(clusters)
+    a, b = count("k_tf_iter_cluster"), count("k_tf_iter")
+    out[clusters] = tf(), count("k_tf_iter_cluster") - a, count("k_tf_iter") - b
+""")
+    assert got == {"1": [0, 5, 0], "0": [0, 0, 5]}
