@@ -36,12 +36,16 @@ int fail(int code, const std::string& msg) {
   g_err = msg;
   return code;
 }
+// An error that a call returned and that is reported is not left behind as the runtime's
+// last error as well, where the next launch's check (ours or another library's) would find it.
 #define CK(call)                                                                      \
   do {                                                                                \
     cudaError_t e_ = (call);                                                          \
-    if (e_ != cudaSuccess)                                                            \
+    if (e_ != cudaSuccess) {                                                          \
+      cudaGetLastError();                                                             \
       return fail(e_ == cudaErrorMemoryAllocation ? BGP_ERR_OOM : BGP_ERR_CUDA,       \
                   std::string(#call) + ": " + cudaGetErrorString(e_));                \
+    }                                                                                 \
   } while (0)
 
 bool size_ok(int N, int M) {
@@ -135,8 +139,13 @@ std::mutex g_pin_mu;
 std::map<int, PinBlock> g_pin;
 
 bool pin_alloc(size_t bytes, char** host, char** dev) {
-  if (cudaHostAlloc((void**)host, bytes, cudaHostAllocMapped) != cudaSuccess) { *host = nullptr; return false; }
+  if (cudaHostAlloc((void**)host, bytes, cudaHostAllocMapped) != cudaSuccess) {
+    cudaGetLastError();
+    *host = nullptr;
+    return false;
+  }
   if (cudaHostGetDevicePointer((void**)dev, *host, 0) == cudaSuccess) return true;
+  cudaGetLastError();
   cudaFreeHost(*host);
   *host = nullptr;
   return false;
@@ -328,7 +337,10 @@ int palloc(bgp_plan* p, size_t bytes, void** out) {
   void* q = nullptr;
   if (bytes == 0) { *out = nullptr; return BGP_OK; }
   cudaError_t e = cudaMalloc(&q, bytes);
-  if (e != cudaSuccess) return fail(BGP_ERR_OOM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return fail(BGP_ERR_OOM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+  }
   p->allocs.push_back(q);
   p->bytes += (long long)bytes;
   CK(cudaMemset(q, 0, bytes));

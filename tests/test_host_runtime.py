@@ -178,3 +178,22 @@ for clusters in (1, 0):
     out[clusters] = tf(), count("k_tf_iter_cluster") - a, count("k_tf_iter") - b
 """)
     assert got == {"1": [0, 5, 0], "0": [0, 0, 5]}
+
+
+def test_a_failed_allocation_is_reported_once(run):
+    """After a mixed solve, a plan or pinned memory that found no memory, other calls work."""
+    got = run(r"""
+rc, h = plan(desc())
+fake.fake_fail_malloc(3)
+out["solve"] = solve(h, 1, 256), apply(h, 256), solve(h, 1, 256), apply(h, 256)
+fake.fake_fail_malloc(2)
+out["plan"] = plan(desc(24))[0], apply(h, 256)
+""")
+    assert got["solve"] == [-3, 0, 0, 0]
+    assert got["plan"] == [-3, 0]
+    got = run(r"""
+fake.fake_fail_host_alloc(1)                     # the device's block: the plan takes memory of its own
+rc, h = plan(desc())
+out["pinned"] = rc, apply(h, 256), lib.bgp_plan_destroy(h), count("live") >= 0
+""")
+    assert got["pinned"] == [0, 0, 0, True]
