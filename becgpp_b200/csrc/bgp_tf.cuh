@@ -292,8 +292,10 @@ BGP_D void tf_step(const TfArgs& A, R& team) {
       if (quad) {
 #pragma unroll
         for (int q = 0; q < NV; ++q) {
-          const double disc = b22 + b34 * (mu[q] - b);
-          const double u = sqrt(fmax(disc, 0.0)) - A.b2;
+          // the roundings of tf_rho: where b3 is small against b2^2 the roots differ from
+          // rounding to rounding, and the density is tf_rho over the sum of these
+          const double disc = __dadd_rn(b22, __dmul_rn(b34, __dsub_rn(mu[q], b)));
+          const double u = __dadd_rn(-A.b2, sqrt(fmax(disc, 0.0)));
           v[q] += disc > 0.0 && u > 0.0 ? u : 0.0;
         }
       } else {
