@@ -7,6 +7,7 @@
 
 #include <algorithm>
 #include <array>
+#include <atomic>
 #include <map>
 #include <mutex>
 #include <string>
@@ -118,6 +119,7 @@ struct DevCtx {
   std::map<int, double2*> tw;   // twiddle tables by length
   std::map<int, double2*> lf[kLVariants];   // line-transform tables of the stream passes
   std::map<int, float2*> lf32[kLVariants];  // the same rounded to FP32
+  std::atomic<signed char> tf_fits[kTfClMax + 1] = {};   // clusters by size: 0 not asked, 1 fits, -1 does not
 };
 std::mutex g_mu;
 std::map<int, DevCtx> g_dev;
@@ -284,7 +286,8 @@ struct bgp_plan {
   long long bytes = 0;
   Inst* d_inst = nullptr;
   int* d_cta_inst = nullptr;
-  int* d_abort = nullptr;
+  double* d_tf = nullptr;                  // Thomas-Fermi state (kTfState values), then
+  int* d_abort = nullptr;                  // the status words: one copy brings both to the host
   int* d_finished = nullptr;               // finished-instance counter of a solve launch
   long long launches = 0;                  // kernel launches issued by this plan
   SolveOut* d_out = nullptr;
@@ -681,7 +684,8 @@ int bgp_plan_create(const bgp_instance_desc* desc, int n_inst, bgp_plan** plan) 
   }
   if ((rc = palloc_t(p, (size_t)n_inst, &p->d_inst))) return bail(rc);
   if ((rc = palloc_t(p, (size_t)p->grid_cap, &p->d_cta_inst))) return bail(rc);
-  if ((rc = palloc_t(p, (size_t)4 + p->grid_cap, &p->d_abort))) return bail(rc);
+  if ((rc = palloc(p, sizeof(double) * kTfState + sizeof(int) * ((size_t)4 + p->grid_cap), (void**)&p->d_tf))) return bail(rc);
+  p->d_abort = (int*)(p->d_tf + kTfState);
   if ((rc = palloc_t(p, (size_t)1, &p->d_finished))) return bail(rc);
   if ((rc = palloc_t(p, (size_t)n_inst, &p->d_out))) return bail(rc);
   if ((rc = palloc_t(p, (size_t)n_inst * (kNRec + 1), &p->d_res))) return bail(rc);
@@ -1527,13 +1531,19 @@ struct TfClusterLaunch {
 };
 // Whether the device can hold such a cluster: more than 8 CTAs are beyond what every
 // device (or partition of one) schedules; the grid-wide launch takes the step where not.
-bool tf_cluster_fits(int ctas) {
-  const TfClusterLaunch L(ctas, nullptr);
-  int n = 0;
-  const bool ok = (ctas <= 8 || cudaFuncSetAttribute(k_tf_iter_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) &&
-                  cudaOccupancyMaxActiveClusters(&n, k_tf_iter_cluster, &L.cfg) == cudaSuccess;
-  if (!ok) cudaGetLastError();
-  return ok && n > 0;
+// Asked once per device and size: the query takes longer than a launch.
+bool tf_cluster_fits(DevCtx* d, int ctas) {
+  signed char known = d->tf_fits[ctas].load(std::memory_order_relaxed);
+  if (known == 0) {
+    const TfClusterLaunch L(ctas, nullptr);
+    int n = 0;
+    const bool ok = (ctas <= 8 || cudaFuncSetAttribute(k_tf_iter_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) &&
+                    cudaOccupancyMaxActiveClusters(&n, k_tf_iter_cluster, &L.cfg) == cudaSuccess;
+    if (!ok) cudaGetLastError();
+    known = ok && n > 0 ? 1 : -1;
+    d->tf_fits[ctas].store(known, std::memory_order_relaxed);
+  }
+  return known > 0;
 }
 int tf_launch_cluster(int ctas, TfArgs A, bgp_plan* p, cudaStream_t st) {
   const TfClusterLaunch L(ctas, st);
@@ -1562,8 +1572,7 @@ int bgp_tf_density(bgp_plan* p, int i, int nonlocal, double Omega, int iters, do
   grid = std::min(grid, std::max(1, (I.n + kTfHold * kThreads - 1) / (kTfHold * kThreads)));
   if (grid < 1) return fail(BGP_ERR_CUDA, "Thomas-Fermi kernel does not fit on an SM");
   int ctas = tf_cluster(I.n, I.beta3);
-  if (ctas && !tf_cluster_fits(ctas)) ctas = 0;
-  double* state = p->d_res + (size_t)i * (kNRec + 1);
+  if (ctas && !tf_cluster_fits(p->dev, ctas)) ctas = 0;
   double* conv = I.phi2 + I.n;   // the plan's second potential field as the convolution output
   TfArgs A;
   memset(&A, 0, sizeof(A));
@@ -1571,13 +1580,14 @@ int bgp_tf_density(bgp_plan* p, int i, int nonlocal, double Omega, int iters, do
   A.dx = I.dx; A.dv = I.dv; A.tc = I.tc; A.s = I.s; A.Omega = Omega;
   A.b2 = I.beta2; A.b3 = I.beta3; A.gc = I.G_C; A.relax = relax;
   A.conv = nonlocal ? conv : nullptr;
-  A.nf = n_out; A.part = I.part; A.bar = I.bar; A.abort_flag = p->d_abort; A.state = state;
-  double h[5] = {NAN, INFINITY, 0.0, 0.0, 0.0};
+  A.nf = n_out; A.part = I.part; A.bar = I.bar; A.abort_flag = p->d_abort; A.state = p->d_tf;
+  // state and, in the last place, the first status word (a copy to pageable memory takes 9 us)
+  double h[kTfState + 1] = {NAN, INFINITY, 0.0, 0.0, 0.0};
   auto read_state = [&]() -> int {
     int ab = 0;
-    CK(cudaMemcpyAsync(h, state, sizeof(h), cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(&ab, p->d_abort, sizeof(int), cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(h, p->d_tf, sizeof(double) * kTfState + sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
+    memcpy(&ab, h + kTfState, sizeof(int));
     if (ab != 0 || h[2] == (double)kTfBarrier) return fail(BGP_ERR_DEVICE, "Thomas-Fermi kernel: team barrier timeout");
     return BGP_OK;
   };
@@ -1586,7 +1596,7 @@ int bgp_tf_density(bgp_plan* p, int i, int nonlocal, double Omega, int iters, do
     void* args[] = {&A};
     return tf_launch((void*)k_tf_iter, grid, args, p, I, st);
   };
-  CK(cudaMemcpyAsync(state, h, sizeof(h), cudaMemcpyHostToDevice, st));
+  CK(cudaMemcpyAsync(p->d_tf, h, sizeof(double) * kTfState, cudaMemcpyHostToDevice, st));
   CK(cudaMemsetAsync(p->d_abort, 0, (4 + (size_t)grid) * sizeof(int), st));
   if (!nonlocal) {
     if ((rc = step())) return rc;

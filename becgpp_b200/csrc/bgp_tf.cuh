@@ -43,6 +43,7 @@ struct TfArgs {
   double* state;                 // out: [0] mu, [1] dn, [2] status, [3] converged, [4] steps taken
 };
 
+constexpr int kTfState = 5;      // values of TfArgs::state
 enum TfStatus : int { kTfOk = 0, kTfNoBracket = 1, kTfEmpty = 2, kTfBarrier = 3 };
 
 // V_eff at flat index f (becgpp/thomasfermi.py:21-30 with becgpp/grid.py:86-91).
@@ -394,20 +395,24 @@ BGP_D void tf_step(const TfArgs& A, R& team) {
 }
 
 // a step after the fixed point has converged or failed does nothing (the host enqueues
-// several steps before it looks). A barrier that timed out in an earlier launch shows in
-// the status word alone when the first CTA got past it.
+// several steps before it looks)
 BGP_D bool tf_over(const TfArgs& A) {
-  return *(volatile const int*)A.abort_flag != 0 || ld1(A.state + 2) != (double)kTfOk || ld1(A.state + 3) != 0.0;
+  const double status = ld1(A.state + 2), done = ld1(A.state + 3);
+  return status != (double)kTfOk || done != 0.0;
 }
 
 // Launched cooperatively with every CTA resident; kThreads threads per CTA.
 __global__ void __launch_bounds__(kThreads) k_tf_iter(TfArgs A) {
   __shared__ double sm[kTfSums * (kWarps + 1)];
-  if (tf_over(A)) return;
+  // (a barrier that timed out in an earlier launch shows in the status word alone when the
+  // first CTA got past it)
+  const int gave_up = __ldcg(A.abort_flag);
+  if (tf_over(A) || gave_up != 0) return;
   TfGrid team{Team{(int)blockIdx.x, (int)gridDim.x, A.bar, A.abort_flag}, A.part, sm, 0};
   tf_step(A, team);
 }
-// Launched as one cluster of gridDim.x CTAs.
+// Launched as one cluster of gridDim.x CTAs. (Its barrier has no time-out; the seed's is
+// reported by the host.)
 __global__ void __launch_bounds__(kTfClThreads) k_tf_iter_cluster(TfArgs A) {
   __shared__ double wpart[kTfSums * kTfClWarps], buf[2 * 8 * kTfClMax];
   if (tf_over(A)) return;
