@@ -1903,7 +1903,9 @@ int bgp_solve(bgp_plan* p, const void* const* psi0, void* const* psi_out, const 
   P.res_tol = sp->res_tol; P.etol = sp->energy_tol; P.alpha0 = sp->step; P.alpha_min = 1e-8;
   P.alpha_max = sp->step_max; P.shift_min = sp->precond_shift_min; P.c1 = 1e-4; P.shrink = 0.5;
   P.growth = 1.1; P.bb_min = 0.05; P.bb_max = sp->step_max; P.bb_mix = 0.5;
-  P.mixed = sp->mixed ? 1 : 0; P.mixed_tol = sp->mixed_switch_res;
+  // a line search of no trials never leaves the initial state: there is nothing for the
+  // mixed form's launches (a trial each) to do
+  P.mixed = sp->mixed && sp->linesearch_max > 0 ? 1 : 0; P.mixed_tol = sp->mixed_switch_res;
   if (P.cg_beta < 0 || P.cg_beta > 2) return fail(BGP_ERR_ARG, "cg_beta must be 0, 1 or 2");
   if (P.maxit < 0) return fail(BGP_ERR_ARG, "maxit must be >= 0");
   double* d_trace = nullptr;

@@ -40,8 +40,8 @@ def plan(*descs):
     return rc, h
 def field(n):
     return (ctypes.c_double * (2 * n))()
-def solve(h, n, points, stream=None, mixed=1, maxit=1):
-    p = L.SolverParams(maxit, 4, 4, 10, 0, 10, 0, 0, mixed, 1e-8, 1e-12, 0.1, 1.0, 0.1, 1e-3)
+def solve(h, n, points, stream=None, mixed=1, maxit=1, trials=4):
+    p = L.SolverParams(maxit, trials, 4, 10, 0, 10, 0, 0, mixed, 1e-8, 1e-12, 0.1, 1.0, 0.1, 1e-3)
     f = [field(points) for _ in range(n)]
     P = (ctypes.c_void_p * n)(*[ctypes.addressof(x) for x in f])
     return lib.bgp_solve(h, P, P, ctypes.byref(p), (L.SolveResult * n)(), None, stream)
@@ -197,3 +197,14 @@ rc, h = plan(desc())
 out["pinned"] = rc, apply(h, 256), lib.bgp_plan_destroy(h), count("live") >= 0
 """)
     assert got["pinned"] == [0, 0, 0, True]
+
+
+def test_a_line_search_of_no_trials_has_none_in_the_mixed_form(run):
+    """linesearch_max = 0 stalls at the initial state: the FP64 solver's answer, not a solve
+    whose launches each hold a trial."""
+    got = run(r"""
+rc, h = plan(desc())
+out["rc"] = rc, solve(h, 1, 256, trials=0), solve(h, 1, 256, trials=-1), count("k_sv_trial")
+out["one"] = solve(h, 1, 256, trials=1), count("k_sv_trial") > 0
+""")
+    assert got == {"rc": [0, 0, 0, 0], "one": [0, True]}
