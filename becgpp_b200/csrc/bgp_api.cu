@@ -881,13 +881,15 @@ Sched sched_of(const bgp_plan::StreamSched& sc) {
 // points or more fills the GPU with 8-line tiles (128-byte rows) and takes the
 // factorization with the fewest exchanges; a smaller one is a few microseconds of
 // latency: narrower tiles spread it over more SMs, and lengths 2^a take the
-// factorization with more threads per line. The autotuner picks the same on 128^3
-// (8 lines; 4 lines 3 % slower), on 192^3 (padded lines of 384: the second factorization
-// 716 us, the first 772) and 256^2 (H psi 4 or 8 lines within 2 %; the quasi-2D
-// convolution 2 and 4 lines 17.5 us, 8 and 8 lines 19 us).
+// factorization with more threads per line. 128^3: 8 lines, 4 lines 3 % slower; 256^2: H psi
+// 4 or 8 lines within 2 %, the quasi-2D convolution 2 and 4 lines 17.5 us, 8 and 8 lines
+// 19 us. Padded lines of 384 and 768 have three stages in the second factorization and
+// four in the first (us of a volume's apply with its potential, second / first: 192^3
+// 704 / 764, 384^3 7240 / 7398); lines of 192 have three in either (96^3 95 / 93), and of
+// 2^a points no fewer in the second (128^3 211 / 178, 256^3 1819 / 1561).
 Sched sched_rule(const Inst& I) {
   const int v = (I.N & (I.N - 1)) == 0;
-  if (I.n >= (1 << 19)) return Sched{8, 0, 8, 8, I.ndim == 3 && !v};
+  if (I.n >= (1 << 19)) return Sched{8, 0, 8, 8, I.ndim == 3 && !v && I.M >= 384};
   return Sched{4, v, 2, 4, v};
 }
 
