@@ -1074,7 +1074,7 @@ int side_stream(bgp_plan* p, int g, cudaStream_t* out) {
 void stream_inst(const bgp_plan* p, int i, SInst& S) {
   const Inst& I = p->inst[i];
   S = SInst{};                  // no given density, no partial sums (launch blocks start undefined)
-  S.ndim = I.ndim; S.N = I.N; S.n = I.n; S.M = I.M; S.Mh = I.Mh; S.i0 = I.i0;
+  S.ndim = I.ndim; S.N = I.N; S.n = I.n; S.M = I.M;
   S.dx = I.dx; S.kfac = I.kfac; S.s = I.s; S.tc = I.tc; S.beta2 = I.beta2; S.beta3 = I.beta3;
   S.Omega = I.Omega; S.dv = I.dv;
   S.A = I.pool;                 // pool field 0 of the instance as the accumulator
@@ -1783,7 +1783,7 @@ int sv_solve(bgp_plan* p, const void* const* psi0, void* const* psi_out, const S
     const Inst& I = p->inst[i];
     SvInst& S = hi[i];
     memset(&S, 0, sizeof(S));
-    S.ndim = I.ndim; S.N = I.N; S.n = I.n; S.M = I.M; S.Mh = I.Mh;
+    S.ndim = I.ndim; S.N = I.N; S.n = I.n; S.M = I.M;
     S.kern = has_kernel(I); S.poly = S.kern && I.ndim == 3;
     S.dx = I.dx; S.dv = I.dv; S.kfac = I.kfac; S.s = I.s; S.tc = I.tc;
     S.beta2 = I.beta2; S.beta3 = I.beta3; S.Omega = I.Omega; S.inv_n = I.inv_n; S.conv_scale = I.conv_scale;

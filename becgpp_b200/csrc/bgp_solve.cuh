@@ -102,7 +102,7 @@ struct alignas(128) SvSync {
 
 // Everything a pass needs about its instance (device memory, written once per solve).
 struct SvInst {
-  int ndim, N, n, M, Mh, kern, poly;
+  int ndim, N, n, M, kern, poly;
   double dx, dv, kfac, s, tc, beta2, beta3, Omega, inv_n, conv_scale;
   double2* pool;
   double* phi2;

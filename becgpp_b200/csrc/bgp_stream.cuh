@@ -36,7 +36,7 @@ BGP_NS_BEGIN
 
 // One instance of a stream batch (device copy).
 struct SInst {
-  int ndim, N, n, M, Mh, i0;
+  int ndim, N, n, M;
   double dx, kfac, s, tc, beta2, beta3, Omega, dv;
   const double2* psi;     // input state
   double2* A;             // per-axis accumulator (scratch, n)

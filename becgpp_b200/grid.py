@@ -183,10 +183,6 @@ def instance_desc(G, cfg):
     return d
 
 
-def desc_key(d):
-    return tuple(getattr(d, f) for f, _ in InstanceDesc._fields_)
-
-
 class Plan:
     """A libbgp plan for a list of instance descriptors (device scratch and tables)."""
 
