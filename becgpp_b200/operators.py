@@ -95,7 +95,8 @@ class HamiltonianBatch:
         psis = list(psis)
         self._one_each("psis", psis)
         psis = [_dev_c128(p) for p in psis]
-        # an output each: parts of one allocation would keep one another's memory alive
+        # an output each: parts of one allocation (113 us a call of 64 instead of 152) would
+        # keep one another's memory alive, and resizing one would write over the next
         outs = out if out is not None else [torch.empty_like(p) for p in psis]
         address = lambda ts: array.array("Q", [t.data_ptr() for t in ts])
         a_psi, a_out = address(psis), address(outs)

@@ -83,7 +83,8 @@ typedef struct {
                   inner products, Armijo test and long-range potential stay FP64;
                   hands over to FP64 storage and transforms at mixed_switch_res or
                   after three consecutive failed line searches; convergence is only
-                  declared in FP64 */
+                  declared in FP64. With linesearch_max < 1 (no trials, no step) the
+                  solve takes the FP64 form */
   double res_tol, energy_tol, step, step_max, precond_shift_min;
   double mixed_switch_res;
 } bgp_solver_params;
