@@ -12,7 +12,6 @@ import sys
 import pytest
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-LIB = os.path.join(ROOT, "becgpp_b200", "libbgp.so")
 
 # A process without torch (whose libraries would bring the real runtime): the binding
 # module alone, with a placeholder for torch.
